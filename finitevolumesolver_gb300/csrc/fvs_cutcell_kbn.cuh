@@ -35,7 +35,7 @@ namespace fvs {
 namespace cc {
 
 // Arithmetic of the physics below: IEEE quotients and square roots (CcIeee:
-// the exact flavour, and FP32 for the mixed one) or the fast FP64 flavour's
+// the exact flavour, on the integer pipes; and FP32 for the mixed one) or the fast FP64 flavour's
 // (CcFast: quotients as products with a reciprocal refined from the
 // rcp.approx seed, square roots as a times its refined reciprocal square
 // root; each within 2 ulp; the square root of a non-positive number is 0).
@@ -44,8 +44,10 @@ namespace cc {
 // different translation units, never share a symbol.
 struct CcIeee {
   static constexpr bool kFast = false;
-  template <class T> static __device__ __forceinline__ T Div(T a, T b) { return a / b; }
-  template <class T> static __device__ __forceinline__ T Sqrt(T a) { return sqrt(a); }
+  static __device__ __forceinline__ double Div(double a, double b) { return ieee64::Div(a, b); }
+  static __device__ __forceinline__ double Sqrt(double a) { return ieee64::Sqrt(a); }
+  static __device__ __forceinline__ float Div(float a, float b) { return a / b; }
+  static __device__ __forceinline__ float Sqrt(float a) { return sqrtf(a); }
 };
 struct CcFast {
   static constexpr bool kFast = true;
@@ -119,10 +121,10 @@ __device__ __forceinline__ void CompleteT(const GasT<T, M>& eq, C2T<T>& q, const
     q.p = (q.E - e_kin) * eq.gm1;
     q.c = M::Sqrt(eq.gamma * q.p * ir);
   } else {
-    const T e_kin = T(0.5) * (q.m[0] * q.m[0] + q.m[1] * q.m[1]) / q.rho;
+    const T e_kin = M::Div(T(0.5) * (q.m[0] * q.m[0] + q.m[1] * q.m[1]), q.rho);
     const T e_int = q.E - e_kin;
-    q.p = e_int / eq.gamma_minus_1_inv;
-    q.c = sqrt(eq.gamma * q.p / q.rho);
+    q.p = M::Div(e_int, eq.gamma_minus_1_inv);
+    q.c = M::Sqrt(M::Div(eq.gamma * q.p, q.rho));
   }
 }
 
@@ -203,12 +205,12 @@ __device__ __forceinline__ void EinfeldtMasked(const GasT<T, M>& eq, const C2T<T
     hL = (L.E + L.p) * irL;
     hR = (R.E + R.p) * irR;
   } else {
-    uL = Sel(L.m, dir) / rhoL;
-    uR = Sel(R.m, dir) / rhoR;
-    wL = sqRhoL / sqRho;
-    wR = sqRhoR / sqRho;
-    hL = (L.E + L.p) / rhoL;
-    hR = (R.E + R.p) / rhoR;
+    uL = M::Div(Sel(L.m, dir), rhoL);
+    uR = M::Div(Sel(R.m, dir), rhoR);
+    wL = M::Div(sqRhoL, sqRho);
+    wR = M::Div(sqRhoR, sqRho);
+    hL = M::Div(L.E + L.p, rhoL);
+    hR = M::Div(R.E + R.p, rhoR);
   }
   const T roeU = uL * wL + uR * wR;
   const T roeH = hL * wL + hR * wR;
@@ -281,7 +283,7 @@ __device__ __forceinline__ void HllMasked(const GasT<T, M>& eq, T* nf, const C2T
     for (int k = 0; k < 4; ++k) nf[k] = (sR * fL[k] - sL * fR[k] + sLsR * (qR[k] - qL[k])) * ids;
   } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) nf[k] = (sR * fL[k] - sL * fR[k] + sLsR * (qR[k] - qL[k])) / ds;
+    for (int k = 0; k < 4; ++k) nf[k] = M::Div(sR * fL[k] - sL * fR[k] + sLsR * (qR[k] - qL[k]), ds);
   }
 }
 

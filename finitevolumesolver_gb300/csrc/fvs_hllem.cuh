@@ -25,16 +25,17 @@ __device__ __forceinline__ void HllemFlux(const Gas& eq, double* nf, const Compl
                                           const Complete<D>& right, int ix) {
   constexpr int K = D + 2;
   const double Msq = 1.0;
-  const double Minv = 1.0 / sqrt(Msq);
+  const double Minv = 1.0;
   Complete<D> L = left, R = right;
   const double rhoL = L.rho, rhoR = R.rho;
+  const ieee64::Divisor dL = MakeDivisor(rhoL), dR = MakeDivisor(rhoR);
   double vL_[D], vR_[D];
   double eKinRL = 0.0, eKinRR = 0.0;
 #pragma unroll
   for (int i = 0; i < D; ++i) {
     const int mask = i == ix;
-    vL_[i] = L.m[i] / rhoL;
-    vR_[i] = R.m[i] / rhoR;
+    vL_[i] = Div(L.m[i], dL);
+    vR_[i] = Div(R.m[i], dR);
     eKinRL += (1 - mask) * vL_[i] * vL_[i];
     eKinRR += (1 - mask) * vR_[i] * vR_[i];
     L.m[i] *= mask;
@@ -50,18 +51,19 @@ __device__ __forceinline__ void HllemFlux(const Gas& eq, double* nf, const Compl
   const double aL = L.c, aR = R.c;
   const double rhoEL = L.E, rhoER = R.E;
   const double pL = L.p, pR = R.p;
-  const double hL = (rhoEL + pL) / rhoL;
-  const double hR = (rhoER + pR) / rhoR;
-  const double sqRhoL = sqrt(rhoL);
-  const double sqRhoR = sqrt(rhoR);
+  const double hL = Div(rhoEL + pL, dL);
+  const double hR = Div(rhoER + pR, dR);
+  const double sqRhoL = Sqrt(rhoL);
+  const double sqRhoR = Sqrt(rhoR);
   const double sqRhoSum = sqRhoL + sqRhoR;
-  const double wL = sqRhoL / sqRhoSum;
-  const double wR = sqRhoR / sqRhoSum;
+  const ieee64::Divisor dsq = MakeDivisor(sqRhoSum);
+  const double wL = Div(sqRhoL, dsq);
+  const double wR = Div(sqRhoR, dsq);
   double uL[D], uR[D], roeU[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) {
-    uL[i] = L.m[i] / rhoL;
-    uR[i] = R.m[i] / rhoR;
+    uL[i] = Div(L.m[i], dL);
+    uR[i] = Div(R.m[i], dR);
     roeU[i] = wL * uL[i] + wR * uR[i];
   }
   const double roeH = wL * hL + wR * hR;
@@ -70,10 +72,10 @@ __device__ __forceinline__ void HllemFlux(const Gas& eq, double* nf, const Compl
   for (int i = 0; i < D; ++i) sqN += roeU[i] * roeU[i];
   sqN *= Msq;
   const double sqN_half = 0.5 * sqN;
-  const double roeGamma = (sqRhoL * eq.gamma + sqRhoR * eq.gamma) / sqRhoSum;
+  const double roeGamma = Div(sqRhoL * eq.gamma + sqRhoR * eq.gamma, dsq);
   const double gm1 = roeGamma - 1.0;
   const double roeA2 = gm1 * (roeH - sqN_half);
-  const double roeA = sqrt(roeA2);
+  const double roeA = Sqrt(roeA2);
   const double maxA = PMax(aL, aR);
   const double sL1 = uL[ix] - maxA * Minv;
   const double sL2 = roeU[ix] - roeA * Minv;
@@ -81,26 +83,27 @@ __device__ __forceinline__ void HllemFlux(const Gas& eq, double* nf, const Compl
   const double sR2 = uR[ix] + maxA * Minv;
   const double sL = PMin(sL1, sL2);
   const double sR = PMax(sR1, sR2);
-  const double bL = PMin(sL, 0.0);
-  const double bR = PMax(sR, 0.0);
+  const double bL = PMin0(sL);
+  const double bR = PMax0(sR);
   const double bLbR = bL * bR;
   const double db = bR - bL;
-  const double dbp = (db > 0.0) ? db : 1.0;
+  const double dbp = ieee64::Positive(db) ? db : 1.0;
+  const ieee64::Divisor ddb = MakeDivisor(dbp);
   double qL[K], qR[K], hlle[K];
   AsCons<D>(qL, L);
   AsCons<D>(qR, R);
 #pragma unroll
   for (int k = 0; k < K; ++k)
-    hlle[k] = (bR * fL[k] - bL * fR[k] + bLbR * (qR[k] - qL[k])) / dbp;
+    hlle[k] = Div(bR * fL[k] - bL * fR[k] + bLbR * (qR[k] - qL[k]), ddb);
   const double u_bar = 0.5 * (sR + sL);
-  const double delta = roeA / (roeA + fabs(u_bar));
-  const double b = bLbR / dbp;
+  const double delta = Div(roeA, roeA + fabs(u_bar));
+  const double b = Div(bLbR, ddb);
   const double dRho = rhoR - rhoL;
   double dRhoU[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) dRhoU[i] = R.m[i] - L.m[i];
   const double dRhoE = rhoER - rhoEL;
-  const double g = gm1 / roeA2;
+  const double g = Div(gm1, roeA2);
   if constexpr (D == 1) {
     const double l21 = g * (roeH - sqN);
     const double l22 = g * Msq * roeU[0];
@@ -121,7 +124,7 @@ __device__ __forceinline__ void HllemFlux(const Gas& eq, double* nf, const Compl
     const double bda2 = bd * alpha_2;
     nf[0] = hlle[0] - bda2;
     nf[1 + ix] = hlle[1 + ix] - bda2 * roeU[ix];
-    const bool upwind = nf[0] > 0.0;
+    const bool upwind = ieee64::Positive(nf[0]);
     nf[1 + iy] = nf[0] * (upwind ? vL_[iy] : vR_[iy]);
     nf[3] = hlle[3] - bda2 * sqN_half + nf[0] * (upwind ? eKinRL : eKinRR);
   } else {
@@ -138,7 +141,7 @@ __device__ __forceinline__ void HllemFlux(const Gas& eq, double* nf, const Compl
     const double bda2 = bd * alpha_2;
     nf[0] = hlle[0] - bda2;
     nf[1 + ix] = hlle[1 + ix] - bda2 * roeU[iy];
-    const bool upwind = nf[0] > 0.0;
+    const bool upwind = ieee64::Positive(nf[0]);
     nf[1 + iy] = nf[0] * (upwind ? vL_[iy] : vR_[iy]);
     nf[1 + iz] = nf[0] * (upwind ? vL_[iz] : vR_[iz]);
     nf[4] = hlle[4] - bda2 * sqN_half + nf[0] * (upwind ? eKinRL : eKinRR);
@@ -152,20 +155,22 @@ __device__ __forceinline__ double HllemMaxSpeed(const Gas& eq, const Complete<D>
                                                 const Complete<D>& R, int ix) {
   const double gm1 = eq.gamma - 1.0;
   const double Msq = 1.0;
-  const double Minv = 1.0 / sqrt(Msq);
+  const double Minv = 1.0;
   const double rhoL = L.rho, rhoR = R.rho;
-  const double hL = (L.E + L.p) / rhoL;
-  const double hR = (R.E + R.p) / rhoR;
-  const double sqRhoL = sqrt(rhoL);
-  const double sqRhoR = sqrt(rhoR);
+  const ieee64::Divisor dL = MakeDivisor(rhoL), dR = MakeDivisor(rhoR);
+  const double hL = Div(L.E + L.p, dL);
+  const double hR = Div(R.E + R.p, dR);
+  const double sqRhoL = Sqrt(rhoL);
+  const double sqRhoR = Sqrt(rhoR);
   const double sqRhoSum = sqRhoL + sqRhoR;
-  const double wL = sqRhoL / sqRhoSum;
-  const double wR = sqRhoR / sqRhoSum;
+  const ieee64::Divisor dsq = MakeDivisor(sqRhoSum);
+  const double wL = Div(sqRhoL, dsq);
+  const double wR = Div(sqRhoR, dsq);
   double uL[D], uR[D], roeU[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) {
-    uL[i] = L.m[i] / rhoL;
-    uR[i] = R.m[i] / rhoR;
+    uL[i] = Div(L.m[i], dL);
+    uR[i] = Div(R.m[i], dR);
     roeU[i] = wL * uL[i] + wR * uR[i];
   }
   const double roeH = wL * hL + wR * hR;
@@ -174,7 +179,7 @@ __device__ __forceinline__ double HllemMaxSpeed(const Gas& eq, const Complete<D>
   for (int i = 0; i < D; ++i) sqN += roeU[i] * roeU[i];
   sqN *= Msq;
   const double roeA2 = gm1 * (roeH - 0.5 * sqN);
-  const double roeA = sqrt(roeA2);
+  const double roeA = Sqrt(roeA2);
   const double maxA = PMax(L.c, R.c);
   const double sL = PMin(uL[ix] - maxA * Minv, roeU[ix] - roeA * Minv);
   const double sR = PMax(roeU[ix] + roeA * Minv, uR[ix] + maxA * Minv);

@@ -173,13 +173,14 @@ __global__ void __launch_bounds__(256) StableDtKernel(StableDtArgs a) {
     for (int c = 0; c < K; ++c) u[c] = __ldg(a.in + c * cs + cell);
     exact::Complete<D> q;
     exact::CompleteFromCons<D>(eq, q, u);
-    const double sq = sqrt(q.rho);
-    const double h = (q.E + q.p) / q.rho;
+    const ieee64::Divisor rho = exact::MakeDivisor(q.rho);
+    const double sq = exact::Sqrt(q.rho);
+    const double h = exact::Div(q.E + q.p, rho);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       exact::CellWave w;
       w.sq = sq;
-      w.u = q.m[d] / q.rho;
+      w.u = exact::Div(q.m[d], rho);
       w.h = h;
       w.a = q.c;
       const int nd = a.n[d];

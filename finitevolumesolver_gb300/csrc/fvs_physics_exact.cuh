@@ -6,6 +6,13 @@
 // sqrt are the IEEE correctly rounded ones, so the results are bit-identical
 // to the reference's x86-64 SSE2 build (no FMA contraction).
 //
+// The kernels of this flavour are bound by the FP64 pipe, so whatever has the
+// same bits elsewhere is taken off it: quotients and square roots run on the
+// integer pipes (fvs_ieee64.cuh: 137 and 143 clocks of the FP64 pipe per warp
+// become about 25 of the integer pipes), comparisons of signs and magnitudes
+// are integer ones, and products with 0.5 and 2 are left out or folded into
+// an FMA whose product they make exact.
+//
 // Reference functions restated here (maikel/FiniteVolumeSolver):
 //   PerfectGas<D>::CompleteFromCons, Flux   src/equations/PerfectGas.cpp:25-124
 //   EinfeldtSignalVelocities<PerfectGas<D>> src/equations/perfect_gas/EinfeldtSignalVelocities.hpp:64-97
@@ -16,8 +23,14 @@
 
 #include <cstdint>
 
+#include "fvs_ieee64.cuh"
+
 namespace fvs {
 namespace exact {
+
+using ieee64::Div;
+using ieee64::MakeDivisor;
+using ieee64::Sqrt;
 
 struct Gas {
   double gamma;
@@ -44,8 +57,11 @@ template <int D> __device__ __forceinline__ double SquaredNorm(const double* m) 
   }
 }
 
-__device__ __forceinline__ double PMin(double a, double b) { return a < b ? a : b; }
-__device__ __forceinline__ double PMax(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ double PMin(double a, double b) { return ieee64::Less(a, b) ? a : b; }
+__device__ __forceinline__ double PMax(double a, double b) { return ieee64::Less(b, a) ? a : b; }
+// PMin(a, 0) and PMax(a, 0)
+__device__ __forceinline__ double PMin0(double a) { return ieee64::Negative(a) ? a : 0.0; }
+__device__ __forceinline__ double PMax0(double a) { return ieee64::Positive(a) ? a : 0.0; }
 
 // CompleteFromCons: e_kin = 0.5*|m|^2/rho, p = (E - e_kin) / gamma_minus_1_inv,
 // c = sqrt(gamma*p/rho).
@@ -56,15 +72,16 @@ __device__ __forceinline__ void CompleteFromCons(const Gas& eq, Complete<D>& q,
 #pragma unroll
   for (int d = 0; d < D; ++d) q.m[d] = u[1 + d];
   q.E = u[1 + D];
-  const double e_kin = 0.5 * SquaredNorm<D>(q.m) / q.rho;
+  const ieee64::Divisor rho = MakeDivisor(q.rho);
+  const double e_kin = Div<true>(SquaredNorm<D>(q.m), rho);
   const double e_int = q.E - e_kin;
-  q.p = e_int / eq.gamma_minus_1_inv;
-  q.c = sqrt(eq.gamma * q.p / q.rho);
+  q.p = Div(e_int, eq.gamma_minus_1_inv);
+  q.c = Sqrt(Div(eq.gamma * q.p, rho));
 }
 
 template <int D>
 __device__ __forceinline__ void Flux(double* f, const Complete<D>& q, int dir) {
-  const double velocity = q.m[dir] / q.rho;
+  const double velocity = Div(q.m[dir], q.rho);
   f[0] = q.m[dir];
 #pragma unroll
   for (int d = 0; d < D; ++d) f[1 + d] = velocity * q.m[d];
@@ -80,23 +97,27 @@ __device__ __forceinline__ void AsCons(double* u, const Complete<D>& q) {
   u[1 + D] = q.E;
 }
 
+// (gamma - 1) (roeH - 0.5 roeU roeU), the half folded into an FMA
+__device__ __forceinline__ double RoeA2(const Gas& eq, double roeU, double roeH) {
+  return (eq.gamma - 1.0) * __fma_rn(-0.5, roeU * roeU, roeH);
+}
+
 template <int D>
 __device__ __forceinline__ void Einfeldt(const Gas& eq, const Complete<D>& L,
                                          const Complete<D>& R, int dir,
                                          double& sL, double& sR) {
   const double rhoL = L.rho;
   const double rhoR = R.rho;
-  const double sqRhoL = sqrt(rhoL);
-  const double sqRhoR = sqrt(rhoR);
-  const double oosqRhoSum = 1.0 / (sqRhoL + sqRhoR);
-  const double uL = L.m[dir] / rhoL;
-  const double uR = R.m[dir] / rhoR;
+  const double sqRhoL = Sqrt(rhoL);
+  const double sqRhoR = Sqrt(rhoR);
+  const double oosqRhoSum = Div(1.0, sqRhoL + sqRhoR);
+  const double uL = Div(L.m[dir], rhoL);
+  const double uR = Div(R.m[dir], rhoR);
   const double roeU = (uL * sqRhoL + uR * sqRhoR) * oosqRhoSum;
-  const double hL = (L.E + L.p) / rhoL;
-  const double hR = (R.E + R.p) / rhoR;
+  const double hL = Div(L.E + L.p, rhoL);
+  const double hR = Div(R.E + R.p, rhoR);
   const double roeH = (hL * sqRhoL + hR * sqRhoR) * oosqRhoSum;
-  const double roeA2 = (eq.gamma - 1.0) * (roeH - 0.5 * roeU * roeU);
-  const double roeA = sqrt(roeA2);
+  const double roeA = Sqrt(RoeA2(eq, roeU, roeH));
   sL = PMin(uL - L.c, roeU - roeA);
   sR = PMax(roeU + roeA, uR + R.c);
 }
@@ -113,14 +134,15 @@ __device__ __forceinline__ void HllFlux(const Gas& eq, double* nf,
   Flux<D>(fR, R, dir);
   AsCons<D>(qL, L);
   AsCons<D>(qR, R);
-  const double sL = PMin(s0, 0.0);
-  const double sR = PMax(s1, 0.0);
+  const double sL = PMin0(s0);
+  const double sR = PMax0(s1);
   const double sLsR = sL * sR;
   double ds = sR - sL;
-  ds = (ds > 0.0) ? ds : 1.0;
+  ds = ieee64::Positive(ds) ? ds : 1.0;
+  const ieee64::Divisor dds = MakeDivisor(ds);
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    nf[k] = (sR * fL[k] - sL * fR[k] + sLsR * (qR[k] - qL[k])) / ds;
+    nf[k] = Div(sR * fL[k] - sL * fR[k] + sLsR * (qR[k] - qL[k]), dds);
   }
 }
 
@@ -139,9 +161,10 @@ __device__ __forceinline__ CellWave MakeCellWave(const Gas& eq, const double* u,
   Complete<D> q;
   CompleteFromCons<D>(eq, q, u);
   CellWave w;
-  w.sq = sqrt(q.rho);
-  w.u = q.m[dir] / q.rho;
-  w.h = (q.E + q.p) / q.rho;
+  const ieee64::Divisor rho = MakeDivisor(q.rho);
+  w.sq = Sqrt(q.rho);
+  w.u = Div(q.m[dir], rho);
+  w.h = Div(q.E + q.p, rho);
   w.a = q.c;
   return w;
 }
@@ -150,11 +173,10 @@ __device__ __forceinline__ CellWave MakeCellWave(const Gas& eq, const double* u,
 // is dx divided by it (Hll::ComputeStableDt, HllMethod.hpp:337-347).
 __device__ __forceinline__ double FaceMaxSpeed(const Gas& eq, const CellWave& L,
                                                const CellWave& R) {
-  const double oosqRhoSum = 1.0 / (L.sq + R.sq);
+  const double oosqRhoSum = Div(1.0, L.sq + R.sq);
   const double roeU = (L.u * L.sq + R.u * R.sq) * oosqRhoSum;
   const double roeH = (L.h * L.sq + R.h * R.sq) * oosqRhoSum;
-  const double roeA2 = (eq.gamma - 1.0) * (roeH - 0.5 * roeU * roeU);
-  const double roeA = sqrt(roeA2);
+  const double roeA = Sqrt(RoeA2(eq, roeU, roeH));
   const double sL = PMin(L.u - L.a, roeU - roeA);
   const double sR = PMax(roeU + roeA, R.u + R.a);
   return PMax(PMax(0.0, fabs(sL)), fabs(sR));
@@ -164,18 +186,27 @@ __device__ __forceinline__ double FaceMaxSpeed(const Gas& eq, const CellWave& L,
 // (slope 0) -- include/fub/flux_method/MusclHancockMethod.hpp:31-187.
 enum Limiter : int { kVanLeer = 0, kMinMod = 1, kNoLimiter = 2, kNoGradient = 3 };
 
-__device__ __forceinline__ double LimitedSlope(int limiter, double qL, double qM,
-                                               double qR) {
+// Half the limited slope, what the predictor adds and subtracts.  Van Leer:
+// 0.5 ((2 sL sR) / (sL + sR)) has the bits of (sL sR) / (sL + sR) unless
+// sL sR leaves the range of ieee64's quotients.
+__device__ __forceinline__ double HalfSlope(int limiter, double qL, double qM, double qR) {
   const double sL = qM - qL;
   const double sR = qR - qM;
   if (limiter == kVanLeer) {
-    const double c = 2.0 * sL * sR;
-    return (c > 0.0) ? c / (sL + sR) : 0.0;
+    const double c = sL * sR;
+    const bool pos = ieee64::Positive(c);
+    double hs = Div(c, pos ? sL + sR : 1.0);
+    hs = pos ? hs : 0.0;
+    if (ieee64::Span(ieee64::Hi(c)) >= ieee64::kSpan && !ieee64::IsZero(sL) && !ieee64::IsZero(sR)) {
+      const double c2 = 2.0 * sL * sR;
+      hs = 0.5 * ((c2 > 0.0) ? c2 / (sL + sR) : 0.0);
+    }
+    return hs;
   }
   if (limiter == kMinMod) {
-    return (sR > 0) ? PMax(0.0, PMin(sL, sR)) : PMin(0.0, PMax(sL, sR));
+    return 0.5 * ((sR > 0) ? PMax(0.0, PMin(sL, sR)) : PMin(0.0, PMax(sL, sR)));
   }
-  if (limiter == kNoLimiter) return 0.5 * (sL + sR);
+  if (limiter == kNoLimiter) return 0.5 * (0.5 * (sL + sR));
   return 0.0;
 }
 
@@ -195,9 +226,9 @@ __device__ __forceinline__ void MusclPredictBoth(const Gas& eq, Complete<D>& rec
   double uL[K], uR[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const double slope = LimitedSlope(limiter, q0[k], q1[k], q2[k]);
-    uL[k] = q1[k] - 0.5 * slope;
-    uR[k] = q1[k] + 0.5 * slope;
+    const double hs = HalfSlope(limiter, q0[k], q1[k], q2[k]);
+    uL[k] = q1[k] - hs;
+    uR[k] = q1[k] + hs;
   }
   Complete<D> qL, qR;
   CompleteFromCons<D>(eq, qL, uL);

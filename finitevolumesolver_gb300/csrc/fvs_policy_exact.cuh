@@ -59,12 +59,13 @@ template <int D> struct ExactPolicy {
   static __device__ __forceinline__ void MakeWaves(const Gas& eq, const double* u, Wave* w) {
     exact::Complete<D> q;
     exact::CompleteFromCons<D>(eq, q, u);
-    const double sq = sqrt(q.rho);
-    const double h = (q.E + q.p) / q.rho;
+    const ieee64::Divisor rho = exact::MakeDivisor(q.rho);
+    const double sq = exact::Sqrt(q.rho);
+    const double h = exact::Div(q.E + q.p, rho);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       w[d].sq = sq;
-      w[d].u = q.m[d] / q.rho;
+      w[d].u = exact::Div(q.m[d], rho);
       w[d].h = h;
       w[d].a = q.c;
     }

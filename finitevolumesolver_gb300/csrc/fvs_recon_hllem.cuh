@@ -21,7 +21,9 @@ namespace exact {
 // of the same sign, else 0.
 __device__ __forceinline__ double VanLeerOf(double sL, double sR) {
   const double r = 2.0 * sL * sR;
-  return (r > 0.0) ? r / (sL + sR) : 0.0;
+  const bool pos = ieee64::Positive(r);
+  const double v = Div(r, pos ? sL + sR : 1.0);
+  return pos ? v : 0.0;
 }
 
 // MusclHancockCharacteristic<Rank>, array path
@@ -44,16 +46,16 @@ __device__ __forceinline__ void CharPredictBoth(const Gas& eq, Complete<D>& recL
   const int iy = (ix + 1) % 3;
   const int iz = (iy + 1) % 3;
   const double rho = s1.rho;
-  const double u = s1.m[ix] / rho;
+  const double u = Div(s1.m[ix], rho);
   const double c = s1.c;
   const double rhoc = rho * c;
-  const double ooc2 = 1.0 / (c * c);
+  const double ooc2 = Div(1.0, c * c);
   double v0[3], v1[3], v2[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    v0[d] = d < D ? s0.m[d] / s0.rho : 0.0;
-    v1[d] = d < D ? s1.m[d] / s1.rho : 0.0;
-    v2[d] = d < D ? s2.m[d] / s2.rho : 0.0;
+    v0[d] = d < D ? Div(s0.m[d], s0.rho) : 0.0;
+    v1[d] = d < D ? Div(s1.m[d], s1.rho) : 0.0;
+    v2[d] = d < D ? Div(s2.m[d], s2.rho) : 0.0;
   }
   double slope[5];
   {
@@ -68,7 +70,7 @@ __device__ __forceinline__ void CharPredictBoth(const Gas& eq, Complete<D>& recL
   }
   double um[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) um[d] = d < D ? s1.m[d] / s1.rho : 0.0;
+  for (int d = 0; d < 3; ++d) um[d] = d < D ? Div(s1.m[d], s1.rho) : 0.0;
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     const double sign = side == 0 ? 1.0 : -1.0;
@@ -80,7 +82,7 @@ __device__ __forceinline__ void CharPredictBoth(const Gas& eq, Complete<D>& recL
     const double dpres = 0.5 * (minus + plus);
     const double drho = ooc2 * dpres + zero;
     double dvel[3];
-    dvel[ix] = 0.5 * (plus - minus) / rhoc;
+    dvel[ix] = Div<true>(plus - minus, MakeDivisor(rhoc));
     dvel[iy] = dv;
     dvel[iz] = dw;
     const double w_rho = drho + rho;
@@ -90,9 +92,9 @@ __device__ __forceinline__ void CharPredictBoth(const Gas& eq, Complete<D>& recL
 #pragma unroll
     for (int d = 0; d < D; ++d) rec.m[d] = w_rho * (dvel[d] + um[d]);
     rec.p = w_p;
-    const double e_kin = 0.5 * SquaredNorm<D>(rec.m) / w_rho;
+    const double e_kin = Div<true>(SquaredNorm<D>(rec.m), MakeDivisor(w_rho));
     rec.E = e_kin + w_p * eq.gamma_minus_1_inv;
-    rec.c = sqrt(eq.gamma * w_p / w_rho);
+    rec.c = Sqrt(Div(eq.gamma * w_p, w_rho));
   }
 }
 
@@ -104,11 +106,11 @@ __device__ __forceinline__ double PrimLimiter(double qL, double qM, double qR) {
   const double delta_q = 0.5 * (qR - qL);
   const bool is_relevant = fabs(delta_q) > 1e-12;
   const double dq = is_relevant ? delta_q : 1.0;
-  const double rL = is_relevant ? (qM - qL) / dq : 0.0;
-  const double rR = is_relevant ? (qR - qM) / dq : 0.0;
+  const double rL = is_relevant ? Div(qM - qL, dq) : 0.0;
+  const double rR = is_relevant ? Div(qR - qM, dq) : 0.0;
   const bool is_positive = rL > 0.0 && rR > 0.0;
   const double r = is_positive ? PMin(rL, rR) : 0.0;
-  const double r_1 = 2.0 * r / (1.0 + r);
+  const double r_1 = Div(2.0 * r, 1.0 + r);
   const double r_2 = 0.5 * (r + 1.0);
   const double sigma = r < 1.0 ? r_1 : r_2;
   return sigma * delta_q;
@@ -127,9 +129,9 @@ __device__ __forceinline__ void PrimPredictBoth(const Gas& eq, Complete<D>& recL
   double u0[D], u1[D], u2[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) {
-    u0[i] = s0.m[i] / s0.rho;
-    u1[i] = s1.m[i] / s1.rho;
-    u2[i] = s2.m[i] / s2.rho;
+    u0[i] = Div(s0.m[i], s0.rho);
+    u1[i] = Div(s1.m[i], s1.rho);
+    u2[i] = Div(s2.m[i], s2.rho);
   }
   const double rho = s1.rho, p = s1.p, a = s1.c;
   const double drho = PrimLimiter(s0.rho, rho, s2.rho);
@@ -140,7 +142,7 @@ __device__ __forceinline__ void PrimPredictBoth(const Gas& eq, Complete<D>& recL
   const double ud = u1[d], dud = du[d];
   const double tr = lambda * (ud * drho + rho * dud);
   const double tp = lambda * (rho * a * a * dud + ud * dp);
-  const double ucorr = 0.5 * lambda * dp / rho;
+  const double ucorr = Div(0.5 * lambda * dp, rho);
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     double rec_rho, rec_p, rec_u[D];
@@ -161,7 +163,7 @@ __device__ __forceinline__ void PrimPredictBoth(const Gas& eq, Complete<D>& recL
 #pragma unroll
     for (int i = 0; i < D; ++i) rec.m[i] = rec_rho * rec_u[i];
     rec.p = rec_p;
-    rec.c = sqrt(eq.gamma * rec_p / rec_rho);
+    rec.c = Sqrt(Div(eq.gamma * rec_p, rec_rho));
     rec.E = 0.5 * rec_rho * SquaredNorm<D>(rec_u) + rec_p * eq.gamma_minus_1_inv;
   }
 }
