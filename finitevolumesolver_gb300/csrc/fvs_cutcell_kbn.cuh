@@ -36,9 +36,8 @@ namespace cc {
 
 // Arithmetic of the physics below: IEEE quotients and square roots (CcIeee:
 // the exact flavour, on the integer pipes; and FP32 for the mixed one) or the fast FP64 flavour's
-// (CcFast: quotients as products with a reciprocal refined from the
-// rcp.approx seed, square roots as a times its refined reciprocal square
-// root; each within 2 ulp; the square root of a non-positive number is 0).
+// (CcFast: nearly rounded ones on the integer pipes, within 0.57 and 0.75
+// ulp; the square root of a non-positive number is 0).
 // The policy is a template argument of every kernel and launcher, so the
 // exact and the fast FP64 instantiations, compiled with different flags in
 // different translation units, never share a symbol.
@@ -50,11 +49,10 @@ struct CcIeee {
   static __device__ __forceinline__ float Sqrt(float a) { return sqrtf(a); }
 };
 struct CcFast {
-  static constexpr bool kFast = true;
+  static constexpr bool kFast = false;  // divides: a reciprocal's product costs the FP64 pipe more
   static __device__ __forceinline__ double Div(double a, double b) {
     return fast::Math<double>::Div(a, b);
   }
-  static __device__ __forceinline__ double Rcp(double a) { return fast::Math<double>::Rcp(a); }
   static __device__ __forceinline__ double Sqrt(double a) { return fast::Math<double>::Sqrt(a); }
 };
 

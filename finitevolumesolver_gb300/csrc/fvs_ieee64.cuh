@@ -173,8 +173,21 @@ __host__ __device__ __forceinline__ Divisor MakeDivisor(double b) {
   return d;
 }
 
-// a / d.b, or with kHalf (0.5 a) / d.b
-template <bool kHalf = false>
+// The correctly rounded 53-bit mantissa of ma / mb from Q' (al: ma's low word).
+__host__ __device__ __forceinline__ uint64_t RoundedQuotient(uint64_t q, bool ge1, uint32_t al,
+                                                             const Divisor& d) {
+  const uint64_t f1 = (q >> (ge1 ? 6 : 5)) + 1;  // the floor F, or F + 1
+  const uint32_t f1l = static_cast<uint32_t>(f1), f1h = static_cast<uint32_t>(f1 >> 32);
+  const uint64_t p = uint64_t(f1l) * d.lo + (uint64_t(f1l * d.hi + f1h * d.lo) << 32);
+  const uint64_t rem = (uint64_t(al << (ge1 ? 21 : 22)) << 32) - p;  // 2^53|54 ma - f1 mb
+  // F = f1 - (rem < 0); the rounded mantissa (F + 1) >> 1
+  return (f1 + 1 + static_cast<uint64_t>(static_cast<int64_t>(rem) >> 63)) >> 1;
+}
+
+// a / d.b, or with kHalf (0.5 a) / d.b.  kNear: without the remainder that
+// decides the rounding; Q' plus its mean error rounded at the mantissa's last
+// bit, within 0.57 ulp (exact quotients stay exact).
+template <bool kHalf = false, bool kNear = false>
 __host__ __device__ __forceinline__ double Div(double a, const Divisor& d) {
   const uint32_t ah = Hi(a), al = Lo(a);
   const uint32_t mh = (ah & 0x000FFFFFu) | 0x00100000u;
@@ -185,12 +198,12 @@ __host__ __device__ __forceinline__ double Div(double a, const Divisor& d) {
                      (uint64_t(q1) * d.lo + (uint64_t(q1 * d.hi) << 32));
   const uint64_t q = uint64_t(q1) * (1u << 28) + MulHi(static_cast<uint32_t>(r >> 24), d.y);
   const bool ge1 = (q >> 59) != 0;  // quotient of the mantissas >= 1
-  const uint64_t f1 = (q >> (ge1 ? 6 : 5)) + 1;  // the floor F, or F + 1
-  const uint32_t f1l = static_cast<uint32_t>(f1), f1h = static_cast<uint32_t>(f1 >> 32);
-  const uint64_t p = uint64_t(f1l) * d.lo + (uint64_t(f1l * d.hi + f1h * d.lo) << 32);
-  const uint64_t rem = (uint64_t(al << (ge1 ? 21 : 22)) << 32) - p;  // 2^53|54 ma - f1 mb
-  // F = f1 - (rem < 0); the rounded mantissa (F + 1) >> 1
-  const uint64_t n = (f1 + 1 + static_cast<uint64_t>(static_cast<int64_t>(rem) >> 63)) >> 1;
+  uint64_t n;
+  if constexpr (kNear) {
+    n = (q + (ge1 ? 64u + 4u : 32u + 4u)) >> (ge1 ? 7 : 6);
+  } else {
+    n = RoundedQuotient(q, ge1, al, d);
+  }
   const uint32_t ea = (ah & 0x7FF00000u) + d.exp - (ge1 ? 0u : 1u << 20) -
                       (kHalf ? 1u << 20 : 0u);
   const uint32_t sign = (ah ^ Hi(d.b)) & 0x80000000u;
@@ -202,12 +215,12 @@ __host__ __device__ __forceinline__ double Div(double a, const Divisor& d) {
   if (d.span >= kSpan || !(Span(ah) < kSpan || zero)) return (kHalf ? 0.5 * a : a) / d.b;
   return Make(hi, lo);
 }
-
 __host__ __device__ __forceinline__ double Div(double a, double b) { return Div(a, MakeDivisor(b)); }
 
 inline double HostSqrt(double a) { return __builtin_sqrt(a); }
 
-__host__ __device__ __forceinline__ double Sqrt(double a) {
+// kNear: without the deciding remainder, within 0.75 ulp.
+template <bool kNear = false> __host__ __device__ __forceinline__ double Sqrt(double a) {
   const uint32_t h = Hi(a), l = Lo(a);
   const uint32_t odd = (~h >> 20) & 1u;  // odd exponent: m = 2 * 1.f in [2, 4)
   const uint32_t mh = (h & 0x000FFFFFu) | 0x00100000u;
@@ -223,11 +236,16 @@ __host__ __device__ __forceinline__ double Sqrt(double a) {
   const uint32_t s1 = static_cast<uint32_t>((uint64_t(xh) * y) >> 31);
   const uint64_t r = ((uint64_t(xh) << 32) | xl) - uint64_t(s1) * s1;
   const uint64_t s = uint64_t(s1) * (1u << 26) + MulHi(static_cast<uint32_t>(r >> 6), y);
-  const uint64_t f1 = (s >> 4) + 1;  // floor(2^53 sqrt(m)) or one more
-  const uint32_t f1l = static_cast<uint32_t>(f1), f1h = static_cast<uint32_t>(f1 >> 32);
-  const uint64_t p = uint64_t(f1l) * f1l + (uint64_t(f1l * (f1h * 2u)) << 32);
-  const uint64_t rem = (uint64_t(l << (22 + static_cast<int>(odd))) << 32) - p;
-  const uint64_t n = (f1 + 1 + static_cast<uint64_t>(static_cast<int64_t>(rem) >> 63)) >> 1;
+  uint64_t n;
+  if constexpr (kNear) {
+    n = (s + 16u + 5u) >> 5;  // s is low by 5 of 2^-57 on average
+  } else {
+    const uint64_t f1 = (s >> 4) + 1;  // floor(2^53 sqrt(m)) or one more
+    const uint32_t f1l = static_cast<uint32_t>(f1), f1h = static_cast<uint32_t>(f1 >> 32);
+    const uint64_t p = uint64_t(f1l) * f1l + (uint64_t(f1l * (f1h * 2u)) << 32);
+    const uint64_t rem = (uint64_t(l << (22 + static_cast<int>(odd))) << 32) - p;
+    n = (f1 + 1 + static_cast<uint64_t>(static_cast<int64_t>(rem) >> 63)) >> 1;
+  }
   const uint32_t er = ((h + (1021u << 20)) >> 1) & 0x7FF00000u;  // floor((e + 1021) / 2)
   if (h - 0x00100000u >= 0x7FE00000u) {  // zero, subnormal, negative, infinite, NaN
 #ifdef __CUDA_ARCH__

@@ -17,18 +17,20 @@
 // the exact flavour per call); T = float gives the mixed flavour's FP32
 // reconstruction and flux.
 //
-// Reciprocal and reciprocal square root in FP64 start from the PTX
-// rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64 estimates (measured on GB300: at
-// most 2^-20 relative error) and refine them with one third-order step from
-// the series of the exact value in the residual r of the estimate y0:
-//   1/a       = y0 / (1 - r),        r = 1 - a y0:   y0 (1 + r + r^2 + ...)
-//   1/sqrt(a) = y0 (1 - r)^(-1/2),   r = 1 - a y0^2: y0 (1 + r/2 + 3 r^2/8 + ...)
-// truncated after the r^2 term, so the refined value is off by ~r^3 < 2^-60
-// (a few ulp after rounding).  a/b = a * (1/b) and sqrt(a) = a * (1/sqrt(a))
-// then carry about one more ulp.
+// In FP64 the quotients and square roots run on the integer pipes
+// (fvs_ieee64.cuh, nearly rounded: within 0.57 and 0.75 ulp) and so do
+// comparisons, because the FP64 pipe (2 lanes per SM and clock) bounds these
+// kernels; a quotient there costs the FP64 pipe nothing, where a product with
+// a refined reciprocal took 3 to 6 of its operations.  So the FP64 forms below
+// divide where the FP32 ones multiply by a shared reciprocal, and are written
+// for few FP64 additions, multiplications and FMAs: about 130 per 3-D
+// cell-update (250 with reciprocals).
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
+
+#include "fvs_ieee64.cuh"
 
 namespace fvs {
 namespace fast {
@@ -36,34 +38,21 @@ namespace fast {
 template <typename T> struct Math;
 
 template <> struct Math<double> {
-  static __device__ __forceinline__ double RcpSeed(double a) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    return y;
+  static __device__ __forceinline__ double Div(double a, const ieee64::Divisor& b) {
+    return ieee64::Div<false, true>(a, b);
   }
-  static __device__ __forceinline__ double RsqrtSeed(double a) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    return y;
+  static __device__ __forceinline__ double Div(double a, double b) {
+    return Div(a, ieee64::MakeDivisor(b));
   }
-  // 1/a: y0 (1 + r + r^2), r = 1 - a y0.
-  static __device__ __forceinline__ double Rcp(double a) {
-    const double y = RcpSeed(a);
-    const double r = fma(-a, y, 1.0);
-    return fma(y, fma(r, r, r), y);
+  // (a / 2) / b
+  static __device__ __forceinline__ double HalfDiv(double a, const ieee64::Divisor& b) {
+    return ieee64::Div<true, true>(a, b);
   }
-  // a/b as a times the refined reciprocal.
-  static __device__ __forceinline__ double Div(double a, double b) { return a * Rcp(b); }
-  // 1/sqrt(a), a > 0: y0 (1 + r (1/2 + 3 r/8)), r = 1 - a y0^2.
-  static __device__ __forceinline__ double Rsqrt(double a) {
-    const double y = RsqrtSeed(a);
-    const double r = fma(-a, y * y, 1.0);
-    return fma(y * r, fma(0.375, r, 0.5), y);
-  }
-  // sqrt(a) for a >= 0 (0 for a <= 0).
+  static __device__ __forceinline__ double Rcp(double a) { return Div(1.0, a); }
+  // sqrt(a) for a >= 0 (0 for a <= 0 and NaN).
   static __device__ __forceinline__ double Sqrt(double a) {
-    if (!(a > 0.0)) return 0.0;
-    return a * Rsqrt(a);
+    const double s = ieee64::Sqrt<true>(a);
+    return ieee64::Positive(a) ? s : 0.0;
   }
 };
 
@@ -73,6 +62,8 @@ template <> struct Math<float> {
   static __device__ __forceinline__ float Rsqrt(float a) { return rsqrtf(a); }
   static __device__ __forceinline__ float Sqrt(float a) { return a > 0.0f ? a * rsqrtf(a) : 0.0f; }
 };
+
+template <typename T> constexpr bool kIsF64 = std::is_same_v<T, double>;
 
 template <typename T> struct Gas {
   T gamma;
@@ -111,6 +102,15 @@ __device__ __forceinline__ void Prepare(const Gas<T>& eq, State<D, T>& s, const 
 #pragma unroll
   for (int d = 0; d < D; ++d) s.m[d] = u[1 + d];
   s.E = u[1 + D];
+  if constexpr (kIsF64<T>) {
+    const ieee64::Divisor rho = ieee64::MakeDivisor(s.rho);
+    s.sq = M::Sqrt(s.rho);
+    s.p = (s.E - M::HalfDiv(SquaredNorm<D, T>(s.m), rho)) * eq.gm1;
+    s.u = M::Div(s.m[dir], rho);
+    s.h = M::Div(s.E + s.p, rho);
+    s.a = M::Sqrt(M::Div(eq.gamma * s.p, rho));
+    return;
+  } else {
   const T rs = M::Rsqrt(s.rho);
   const T ir = rs * rs;
   s.sq = s.rho * rs;
@@ -119,12 +119,23 @@ __device__ __forceinline__ void Prepare(const Gas<T>& eq, State<D, T>& s, const 
   s.u = s.m[dir] * ir;
   s.h = (s.E + s.p) * ir;
   s.a = M::Sqrt(eq.gamma * s.p * ir);
+  }
 }
 
 // Physical flux of a conservative state (PerfectGas::Flux), no sound speed.
 template <int D, typename T>
 __device__ __forceinline__ void FluxOfCons(const Gas<T>& eq, T* f, const T* u, int dir) {
   using M = Math<T>;
+  if constexpr (kIsF64<T>) {
+    const ieee64::Divisor rho = ieee64::MakeDivisor(u[0]);
+    const T p = (u[1 + D] - M::HalfDiv(SquaredNorm<D, T>(u + 1), rho)) * eq.gm1;
+    const T v = M::Div(u[1 + dir], rho);
+    f[0] = u[1 + dir];
+#pragma unroll
+    for (int d = 0; d < D; ++d) f[1 + d] = d == dir ? fma(v, u[1 + d], p) : v * u[1 + d];
+    f[1 + D] = v * (u[1 + D] + p);
+    return;
+  } else {
   const T ir = M::Rcp(u[0]);
   const T ke = T(0.5) * SquaredNorm<D, T>(u + 1) * ir;
   const T p = (u[1 + D] - ke) * eq.gm1;
@@ -134,15 +145,22 @@ __device__ __forceinline__ void FluxOfCons(const Gas<T>& eq, T* f, const T* u, i
   for (int d = 0; d < D; ++d) f[1 + d] = v * u[1 + d];
   f[1 + dir] += p;
   f[1 + D] = v * (u[1 + D] + p);
+  }
 }
 
 template <int D, typename T>
 __device__ __forceinline__ void FluxOfState(T* f, const State<D, T>& s, int dir) {
   f[0] = s.m[dir];
+  if constexpr (kIsF64<T>) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) f[1 + d] = d == dir ? fma(s.u, s.m[d], s.p) : s.u * s.m[d];
+    f[1 + D] = s.m[dir] * s.h;
+  } else {
 #pragma unroll
   for (int d = 0; d < D; ++d) f[1 + d] = s.u * s.m[d];
   f[1 + dir] += s.p;
   f[1 + D] = s.u * (s.E + s.p);
+  }
 }
 
 template <int D, typename T>
@@ -153,17 +171,35 @@ __device__ __forceinline__ void ConsOf(T* q, const State<D, T>& s) {
   q[1 + D] = s.E;
 }
 
-template <typename T> __device__ __forceinline__ T Min(T a, T b) { return a < b ? a : b; }
-template <typename T> __device__ __forceinline__ T Max(T a, T b) { return a > b ? a : b; }
+template <typename T> __device__ __forceinline__ T Min(T a, T b) {
+  if constexpr (kIsF64<T>) return ieee64::Less(a, b) ? a : b;
+  else return a < b ? a : b;
+}
+template <typename T> __device__ __forceinline__ T Max(T a, T b) {
+  if constexpr (kIsF64<T>) return ieee64::Less(b, a) ? a : b;
+  else return a > b ? a : b;
+}
+template <typename T> __device__ __forceinline__ bool Positive(T a) {
+  if constexpr (kIsF64<T>) return ieee64::Positive(a);
+  else return a > T(0);
+}
 
 // Einfeldt speeds from the states' precomputed sqrt(rho), u, h, a.
 template <typename T, class S>
 __device__ __forceinline__ void Einfeldt(const T gm1, const S& L, const S& R, T& sL, T& sR) {
   using M = Math<T>;
-  const T oo = M::Rcp(L.sq + R.sq);
-  const T roeU = fma(L.u, L.sq, R.u * R.sq) * oo;
-  const T roeH = fma(L.h, L.sq, R.h * R.sq) * oo;
-  const T roeA = M::Sqrt(gm1 * fma(T(-0.5) * roeU, roeU, roeH));
+  T roeU, roeH, roeA;
+  if constexpr (kIsF64<T>) {
+    const ieee64::Divisor sum = ieee64::MakeDivisor(L.sq + R.sq);
+    roeU = M::Div(fma(L.u, L.sq, R.u * R.sq), sum);
+    roeH = M::Div(fma(L.h, L.sq, R.h * R.sq), sum);
+    roeA = M::Sqrt(gm1 * fma(-0.5, roeU * roeU, roeH));
+  } else {
+    const T oo = M::Rcp(L.sq + R.sq);
+    roeU = fma(L.u, L.sq, R.u * R.sq) * oo;
+    roeH = fma(L.h, L.sq, R.h * R.sq) * oo;
+    roeA = M::Sqrt(gm1 * fma(T(-0.5) * roeU, roeU, roeH));
+  }
   sL = Min(L.u - L.a, roeU - roeA);
   sR = Max(roeU + roeA, R.u + R.a);
 }
@@ -178,6 +214,25 @@ __device__ __forceinline__ void HllFlux(const Gas<T>& eq, T* nf, const State<D, 
   T fL[K], fR[K];
   FluxOfState<D, T>(fL, L, dir);
   FluxOfState<D, T>(fR, R, dir);
+  if constexpr (kIsF64<T>) {
+    // the flux of the upwind state (the side of the slower wave) and a
+    // difference that vanishes for equal states: F_L + (sL / ds) (F_L - F_R +
+    // sR (q_R - q_L)) = F_R + (sR / ds) (F_L - F_R + sL (q_R - q_L)), 4 FP64
+    // operations per component and exactly F_L or F_R in supersonic flow
+    const T sL = ieee64::Negative(s0) ? s0 : 0.0;
+    const T sR = ieee64::Positive(s1) ? s1 : 0.0;
+    const T ds = sR - sL;
+    const bool right = ieee64::Hi(sR) < (ieee64::Hi(sL) & 0x7FFFFFFFu);  // sR < -sL or near it
+    const T w = Math<T>::Div(right ? sR : sL, ieee64::Positive(ds) ? ds : 1.0);
+    const T so = right ? sL : sR;
+    T qL[K], qR[K];
+    ConsOf<D, T>(qL, L);
+    ConsOf<D, T>(qR, R);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      nf[k] = fma(w, fma(so, qR[k] - qL[k], fL[k] - fR[k]), right ? fR[k] : fL[k]);
+    return;
+  } else {
   const T sL = Min(s0, T(0));
   const T sR = Max(s1, T(0));
   const T sLsR = sL * sR;
@@ -191,6 +246,7 @@ __device__ __forceinline__ void HllFlux(const Gas<T>& eq, T* nf, const State<D, 
   ConsOf<D, T>(qR, R);
 #pragma unroll
   for (int k = 0; k < K; ++k) nf[k] = fma(wL, fL[k], fma(-wR, fR[k], wq * (qR[k] - qL[k])));
+  }
 }
 
 // Half the limited slope (what the predictor adds and subtracts).  Van Leer:
@@ -202,7 +258,13 @@ __device__ __forceinline__ T HalfSlope(int limiter, T qL, T qM, T qR) {
   const T sR = qR - qM;
   if (limiter == 0) {  // van Leer
     const T c = sL * sR;
-    return (c > T(0)) ? Math<T>::Div(c, sL + sR) : T(0);
+    if constexpr (kIsF64<T>) {
+      const bool pos = ieee64::Positive(c);
+      const T h = Math<T>::Div(c, pos ? sL + sR : 1.0);
+      return pos ? h : 0.0;
+    } else {
+      return (c > T(0)) ? Math<T>::Div(c, sL + sR) : T(0);
+    }
   }
   if (limiter == 1) {  // MinMod
     return T(0.5) * ((sR > T(0)) ? Max(T(0), Min(sL, sR)) : Min(T(0), Max(sL, sR)));
@@ -260,6 +322,16 @@ __device__ __forceinline__ Wave<T> MakeWave(const Gas<T>& eq, const T* u, int di
 template <int D, typename T>
 __device__ __forceinline__ void MakeWaves(const Gas<T>& eq, const T* u, Wave<T>* w) {
   using M = Math<T>;
+  if constexpr (kIsF64<T>) {
+    const ieee64::Divisor rho = ieee64::MakeDivisor(u[0]);
+    const T sq = M::Sqrt(u[0]);
+    const T p = (u[1 + D] - M::HalfDiv(SquaredNorm<D, T>(u + 1), rho)) * eq.gm1;
+    const T h = M::Div(u[1 + D] + p, rho);
+    const T a = M::Sqrt(M::Div(eq.gamma * p, rho));
+#pragma unroll
+    for (int d = 0; d < D; ++d) w[d] = Wave<T>{sq, M::Div(u[1 + d], rho), h, a};
+    return;
+  } else {
   const T rho = u[0];
   const T rs = M::Rsqrt(rho);
   const T ir = rs * rs;
@@ -270,6 +342,7 @@ __device__ __forceinline__ void MakeWaves(const Gas<T>& eq, const T* u, Wave<T>*
   const T a = M::Sqrt(eq.gamma * p * ir);
 #pragma unroll
   for (int d = 0; d < D; ++d) w[d] = Wave<T>{sq, u[1 + d] * ir, h, a};
+  }
 }
 
 template <typename T>

@@ -12,7 +12,7 @@
 // with the reference's operation order (the including translation unit is
 // compiled with -fmad=false).  The powers of pressure ratios are n-th roots
 // (Powers) or CUDA's pow(), and the quotients and square roots of variable
-// operands refined reciprocal seeds (Div, Sqrt), so results agree with the
+// operands nearly rounded (Div, Sqrt), so results agree with the
 // CPU oracle to ~1e-15 relative rather than bit for bit.
 //
 // Differences by design:
@@ -28,7 +28,6 @@
 
 #include "fvs_mlp.cuh"
 #include "fvs_physics_exact.cuh"
-#include "fvs_physics_fast.cuh"
 #include "fvs_roots.cuh"
 
 namespace fvs {
@@ -44,23 +43,14 @@ struct Options {
   int root_n;        // RootOrder(gamma): 0, or n with n-th roots in place of pow()
 };
 
-// Quotients and square roots of the solver's variable operands: a reciprocal
-// (reciprocal square root) seed refined by one third-order step, the fast
-// flavour's fast::Math<double> (within ~2 ulp of IEEE), in place of IEEE
-// division and sqrt, which cost the FP64 pipe several times as much.
-// Operands that are zero, negative, not finite or within 2^2 of the FP64
-// range's ends take IEEE division and sqrt, so vacuum and failed states keep
+// Quotients and square roots of the solver's variable operands on the integer
+// pipes (fvs_ieee64.cuh, nearly rounded: within 0.57 and 0.75 ulp), since the
+// FP64 pipe bounds the solver; zero, negative and non-finite operands keep
 // IEEE semantics (inf, NaN).
-__device__ __forceinline__ bool InRange(double b) {
-  const unsigned e = static_cast<unsigned>(__double2hiint(b)) & 0x7FFFFFFFu;
-  return e >= 0x00200000u && e < 0x7FD00000u;
-}
 __device__ __forceinline__ double Div(double a, double b) {
-  return InRange(b) ? a * fast::Math<double>::Rcp(b) : a / b;
+  return ieee64::Div<false, true>(a, ieee64::MakeDivisor(b));
 }
-__device__ __forceinline__ double Sqrt(double a) {
-  return (a > 0.0 && InRange(a)) ? a * fast::Math<double>::Rsqrt(a) : sqrt(a);
-}
+__device__ __forceinline__ double Sqrt(double a) { return ieee64::Sqrt<true>(a); }
 
 // PerfectGas::CompleteFromCons and Flux (src/equations/PerfectGas.cpp:52-124)
 // with the quotients and square root above: the Godunov sweeps' cell states
