@@ -323,17 +323,35 @@ const void* TmaMapOf(const fvs_solver* s, const double* in, int dir) {
   return nullptr;
 }
 
+// Slots of the one-cell-per-lane sweep (a segment length of 1).
+int64_t LaneSlots(const fvs_solver* s, int dir) {
+  return s->cells / s->g.n[dir] * (int64_t(s->g.n[dir]) + 2);
+}
+
 int SegLen(const fvs_solver* s, int dir) {
   if (s->seg_len > 0) return s->seg_len;
   if (s->seg_tuned[dir] > 0) return s->seg_tuned[dir];
   const int nd = s->g.n[dir];
   int64_t ntrans = s->cells / nd;
+  const bool mixed = s->m.precision == FVS_MIXED;
+  // Small grids: one cell per lane (SweepLanesKernel) instead of marching
+  // segments, whose serial chains leave the chip idle.  Measured per sweep
+  // against the best marching segment (16 cells, the shortest default, in
+  // brackets): exact FP64 64^3 0.13 / 0.18 ms (0.26), 128^3 0.99 / 1.03 ms,
+  // 192^3 3.25 / 2.95 ms; double-float 128^3 0.44 / 0.46 ms; mixed, where
+  // lanes along y or z load a sector per value: 64^2 25 / 31 us (38), 32^3
+  // equal, 64^3 20 / 11 us.
+  if (!s->cc && (mixed ? s->g.rank == 1 || s->cells <= (int64_t(1) << 14)
+                       : s->cells <= (int64_t(1) << 22)) &&
+      LaneSlots(s, dir) < (int64_t(1) << 31))
+    return 1;
   // Enough threads for several waves of resident blocks on 152 SMs
   // (~60K threads per wave at 150 registers per thread); never shorter than
-  // 16 cells (the 2-cell halo of a segment is recomputed).
+  // 16 cells, mixed 8 (the 2-cell halo of a segment is recomputed).
   const int64_t target = 262144;
+  const int shortest = mixed && !s->cc ? 8 : 16;
   int seg = nd;
-  while (seg > 16 && ntrans * ((nd + seg - 1) / seg) < target) seg = (seg + 1) / 2;
+  while (seg > shortest && ntrans * ((nd + seg - 1) / seg) < target) seg = (seg + 1) / 2;
   return seg;
 }
 
@@ -422,6 +440,7 @@ cudaError_t LaunchSweep(const fvs_solver* s, const double* in, double* out,
   a.mlp = s->m.mlp_params;
   a.stats_out = ctrl ? ctrl->newton : s->newton_words;
   a.skip_cfl = skip_cfl ? 1 : 0;
+  a.lanes = a.seg_len == 1 && a.occupancy < 20 && LaneSlots(s, dir) < (int64_t(1) << 31) ? 1 : 0;
   a.tmap = a.occupancy >= 20 ? TmaMapOf(s, in, dir) : nullptr;
   a.t_lo = t_lo;
   a.t_hi = t_hi;
@@ -1046,7 +1065,7 @@ int fvs_solver_autotune(fvs_solver* s, int* seg_out) {
   // register/occupancy variants of the same kernel), timed on the current
   // state with a small dt (output goes to a spare buffer; the state is not
   // changed).
-  const int cands[] = {8, 16, 32, 64, 128, 256, 512};
+  const int cands[] = {1, 8, 16, 32, 64, 128, 256, 512};  // 1: one cell per lane
   const bool plain_hlle = s->m.flux_method <= FVS_HLLE && !s->cc;
   const bool mixed = s->m.precision == FVS_MIXED && plain_hlle;
   const bool df = s->m.precision == FVS_FP64_DF && plain_hlle;
@@ -1088,9 +1107,11 @@ int fvs_solver_autotune(fvs_solver* s, int* seg_out) {
       // the lanes-along-x kernel has no segment length: one candidate
       const bool warp_x = mixed && d == 0 && occs[oi] < 10;
       for (int c : cands) {
-        if (c > 2 * nd && c != cands[0]) break;
+        if (c > 2 * nd && c > 8) break;
+        // one cell per lane: one candidate, under the first variant
+        if (c == 1 && (s->cc || oi > 0)) continue;
         // the tile kernels (mixed cut cells, variant 0) have no segment length
-        if ((warp_x || (cc_cell && occs[oi] == 0)) && c != cands[0]) break;
+        if ((warp_x || (cc_cell && occs[oi] == 0)) && c > 8) break;
         s->seg_len = c;
         float ms_sum = 0.f;
         for (int rep = 0; rep < 3; ++rep) {

@@ -94,6 +94,7 @@ struct SweepArgs {
                         // variant is compiled for (mixed: 4, 5; double-float: 3);
                         // mixed x sweeps: + 10 for the marching kernel in x;
                         // mixed y/z sweeps: + 20 for the TMA-staged kernel
+  int lanes;            // 1: the one-cell-per-lane sweep (ntrans (n + 2) < 2^31 slots)
   const void* tmap;     // host: CUtensorMap of `in` for the TMA-staged kernel, or NULL
   // grid lines [t_lo, t_hi) only (t: the line index of the marching and
   // lanes-along-x kernels); t_hi == 0: every line

@@ -16,6 +16,7 @@ template <int D> struct Df64Policy : FastBase<D, df64> {};
 // spilled); the autotuner picks between the two
 template <int D> struct Df64PolicyOcc3 : FastBase<D, df64> {
   static constexpr int kMinBlocks = 3;
+  static constexpr int kLaneBlocks = 0;
 };
 
 template <template <int> class PT> cudaError_t LaunchSweepDf64T(const SweepArgs& a, cudaStream_t s) {
@@ -30,7 +31,7 @@ template <template <int> class PT> cudaError_t LaunchSweepDf64T(const SweepArgs&
 }
 
 cudaError_t LaunchSweepDf64(const SweepArgs& a, cudaStream_t s) {
-  return a.occupancy == 3 ? LaunchSweepDf64T<Df64PolicyOcc3>(a, s)
+  return a.occupancy == 3 && !a.lanes ? LaunchSweepDf64T<Df64PolicyOcc3>(a, s)
                           : LaunchSweepDf64T<Df64Policy>(a, s);
 }
 

@@ -39,6 +39,7 @@ template <template <int> class PT> cudaError_t LaunchSweepMixedT(const SweepArgs
 // occupancy: 0, 4, 5 = register/occupancy variant (x sweeps with lanes along
 // x); 10, 14, 15 = the same variants with the marching kernel in x.
 cudaError_t LaunchSweepMixed(const SweepArgs& a, cudaStream_t s) {
+  if (a.lanes) return LaunchSweepMixedT<Mixed32Policy>(a, s);
   // reflective rows: the marching kernel (its loads reflect ghost states)
   if (a.dir == 0 && (a.occupancy >= 10 || a.bc == 2)) {
     switch (a.occupancy) {

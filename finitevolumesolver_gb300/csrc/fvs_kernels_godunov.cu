@@ -39,6 +39,7 @@ template <int D, bool kMuscl> struct GodunovPolicyT {
   using Real = double;
   static constexpr bool kWarpX = false;
   static constexpr int kMinBlocks = 1;
+  static constexpr int kLaneBlocks = 4;
   using Gas = GodunovGas;
   using Rec = exact::Complete<D>;
   using Wave = exact::Complete<D>;

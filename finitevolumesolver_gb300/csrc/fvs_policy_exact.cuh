@@ -14,6 +14,7 @@ template <int D> struct ExactPolicy {
   using Real = double;
   static constexpr bool kWarpX = false;
   static constexpr int kMinBlocks = 3;  // at most 168 registers
+  static constexpr int kLaneBlocks = 4;
   static constexpr bool kEinfeldtCfl = true;  // CFL speeds screened in FP32
   using Gas = exact::Gas;
   using Wave = exact::CellWave;

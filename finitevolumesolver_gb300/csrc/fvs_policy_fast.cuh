@@ -23,6 +23,7 @@ template <int D, typename T> struct FastBase {
   // the mixed flavour is memory-bound: its x sweep uses lanes along x
   static constexpr bool kWarpX = sizeof(T) == 4;
   static constexpr int kMinBlocks = 1;
+  static constexpr int kLaneBlocks = 4;
   // FP64 and double-float: the sweep screens the Einfeldt CFL speeds in FP32
   static constexpr bool kEinfeldtCfl = sizeof(T) != 4;
   using Gas = fast::Gas<T>;
@@ -109,21 +110,26 @@ template <int D> struct Mixed32Policy : FastBase<D, float> {};
 // The same arithmetic compiled for more resident blocks per SM (fewer
 // registers per thread, more warps to hide latency); the autotuner picks.
 template <int D> struct Mixed32PolicyOcc4 : FastBase<D, float> {
+  static constexpr int kLaneBlocks = 0;
   static constexpr int kMinBlocks = 4;
 };
 template <int D> struct Mixed32PolicyOcc5 : FastBase<D, float> {
+  static constexpr int kLaneBlocks = 0;
   static constexpr int kMinBlocks = 5;
 };
 // The mixed flavour with the marching kernel in x as well (a thread walks a
 // row; each row's loads are reused from L1 instead of exchanged by shuffles).
 template <int D> struct Mixed32PolicyMarchX : FastBase<D, float> {
+  static constexpr int kLaneBlocks = 0;
   static constexpr bool kWarpX = false;
 };
 template <int D> struct Mixed32PolicyMarchXOcc4 : FastBase<D, float> {
+  static constexpr int kLaneBlocks = 0;
   static constexpr bool kWarpX = false;
   static constexpr int kMinBlocks = 4;
 };
 template <int D> struct Mixed32PolicyMarchXOcc5 : FastBase<D, float> {
+  static constexpr int kLaneBlocks = 0;
   static constexpr bool kWarpX = false;
   static constexpr int kMinBlocks = 5;
 };

@@ -967,6 +967,163 @@ __global__ void __launch_bounds__(128, PT<D>::kMinBlocks) SweepXWarpKernel(Sweep
   if (status && a.ctrl) atomicOr(&a.ctrl->step_status, status);
 }
 
+// Policies that have the one-cell-per-lane sweep (kLaneBlocks: the resident
+// blocks per SM it is compiled for).
+template <class P, class = void> struct HasLanes : std::false_type {};
+template <class P>
+struct HasLanes<P, std::enable_if_t<(P::kLaneBlocks > 0)>> : std::true_type {};
+
+// One cell per lane: the grid's lines along the sweep direction are laid end
+// to end as slots, n + 2 per line (cells -1..n); warp w takes the slots
+// 30 w .. 30 w + 31.  A lane evaluates its cell's predictor and the face on
+// the cell's left with what its left neighbour's lane hands it by shuffles,
+// and the lanes 1..30 own their slots (CFL speed of the face, update of the
+// cell with the right neighbour's face).  Where a line ends or the warp does,
+// a lane loads the missing neighbour cell itself.  Every face and cell takes
+// the marching sweep's arithmetic, so the results are the same bits.
+//
+// It is the sweep of grids whose lines are too few to fill the chip by
+// marching: a marching thread's segment is a serial chain over its cells (16
+// cells of ~160 FP64 operations, 64 clocks each in one of an SM's four FP64
+// units, which one warp saturates), while here a grid of 20 thousand cells
+// already gives every FP64 unit a warp.  The cost is 32 predictors for 30
+// cells and, in y and z, loads of one sector per lane, which the FP64
+// flavours hide behind their arithmetic.
+constexpr int kLaneStep = 30;
+
+template <int D, int DIR, template <int> class PT>
+__global__ void __launch_bounds__(128, PT<D>::kLaneBlocks) SweepLanesKernel(SweepArgs a) {
+  using P = PT<D>;
+  using R = typename P::Real;
+  constexpr int K = D + 2;
+  using Cell = CellArr<R, K>;
+  using FluxT = typename FluxOf<P>::type;
+  using Flx = CellArr<FluxT, K>;
+  const int nx = a.n[0], ny = a.n[1], nz = a.n[2];
+  const double split_dt = a.dt_ptr ? a.dt_scale * (*a.dt_ptr) : a.dt_value;
+  if (!BlockAll(SweepGate(a, split_dt))) return;
+  const int nd = a.n[DIR];
+  const int64_t ntrans = DIR == 0 ? int64_t(ny) * nz : DIR == 1 ? int64_t(nx) * nz : int64_t(nx) * ny;
+  const int64_t t_end = a.t_hi > 0 ? a.t_hi : ntrans;
+  const uint32_t per = uint32_t(nd) + 2;
+  const uint32_t total = uint32_t(t_end - a.t_lo) * per;  // < 2^31: the launcher checks
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // slots past the end take the last one again and own nothing
+  const uint32_t want = warp * kLaneStep + lane;
+  const uint32_t slot = want < total ? want : total - 1;
+  const uint32_t lrel = slot / per;
+  const int j = static_cast<int>(slot - lrel * per) - 1;
+  const int64_t t = a.t_lo + lrel;
+
+  GlobalLine<K, DIR> line;
+  line.in = a.in;
+  line.cs = int64_t(nx) * ny * nz;
+  line.nd = nd;
+  line.bc = a.bc;
+  if (DIR == 0) {
+    line.base = t * nx;
+    line.stride = 1;
+  } else if (DIR == 1) {
+    const int64_t i = t % nx, k = t / nx;
+    line.base = k * int64_t(nx) * ny + i;
+    line.stride = nx;
+  } else {
+    line.base = t;
+    line.stride = int64_t(nx) * ny;
+  }
+  const typename P::Gas eq = P::MakeGasFor(a);
+  const double lambda_half = 0.5 * split_dt / a.dx;
+  const double dt_dx = split_dt / a.dx;
+  const bool skip_cfl = HasFluxOnly<P>::value && a.skip_cfl != 0;
+  constexpr bool kFilter = FilteredCfl<P>::value && HasFluxOnly<P>::value;
+
+  double u[K], ue[K];
+  Cell C, Cm, Cp;
+  bool flip = line.Load(u, j);
+  const bool left = j == -1 || lane == 0, right = j == nd || lane == 31;
+  bool flip_e = false;
+  if (left || right) flip_e = line.Load(ue, left ? j - 1 : j + 1);
+  P::ToCell(C.v, u);
+  if (flip) C.v[1 + DIR] = -C.v[1 + DIR];
+  Cm = ShflUp(C, 1);
+  Cp = ShflDown(C, 1);
+  if (left || right) {
+    Cell E;
+    P::ToCell(E.v, ue);
+    if (flip_e) E.v[1 + DIR] = -E.v[1 + DIR];
+    if (left) Cm = E;
+    else Cp = E;
+    // both ends (a line of one cell at the warp's edge): the right one too
+    if (left && right) {
+      flip_e = line.Load(ue, j + 1);
+      P::ToCell(E.v, ue);
+      if (flip_e) E.v[1 + DIR] = -E.v[1 + DIR];
+      Cp = E;
+    }
+  }
+  const bool own = want < total && lane >= 1 && lane <= kLaneStep && j >= 0;
+  R smax = R(0);
+  int status = 0;
+  typename P::Stats stats, other;
+  if constexpr (kFilter) {
+    // the FP32 screen of the marching sweep, the threshold read once: the
+    // warp evaluates its faces' exact speeds if any of them can hold the
+    // sweep's maximum
+    if (!skip_cfl) {
+      fast::Gas<float> g32;
+      g32.gamma = static_cast<float>(a.gamma);
+      g32.gm1 = static_cast<float>(a.gamma - 1.0);
+      using S = CflScreen<P, D>;
+      float thr = 0.0f;
+      if (a.smax_out)
+        thr = CflFloatBelow(BitsToDouble(*reinterpret_cast<volatile unsigned long long*>(a.smax_out)));
+      float c32[K];
+#pragma unroll
+      for (int c = 0; c < K; ++c) c32[c] = CflToF32(C.v[c]);
+      const typename S::V v = S::Wave(g32, c32, DIR);
+      const bool ok = a.gamma > 1.0 && a.gamma <= 2.0 && CflInRange<D>(c32) && v.a > 0.0f;
+      const typename S::V vm = ShflUp(v, 1);
+      const bool okm = __shfl_up_sync(0xffffffffu, ok ? 1 : 0, 1) != 0;
+      const float s32 = S::Speed(g32, vm, v, DIR);
+      const float sh = fast::Math<float>::Sqrt(fmaxf(vm.h, v.h));
+      const float bound = fmaf(s32, kCflRel, fmaf(kCflScale, sh, kCflAbs));
+      if (__any_sync(0xffffffffu, own && !(ok && okm && bound < thr))) {
+        const typename P::Wave w = P::MakeWave(eq, C.v, DIR);
+        const typename P::Wave wm = ShflUp(w, 1);
+        const R s = P::FaceMaxSpeed(eq, wm, w);
+        if (own) smax = s > smax ? s : smax;
+      }
+    }
+  }
+  typename P::Rec recL, recR;
+  P::Predict(eq, recL, recR, Cm.v, C.v, Cp.v, a.limiter, lambda_half, DIR);
+  const typename P::Rec recRm = ShflUp(recR, 1);
+  Flx F;
+  if constexpr (kFilter) {
+    SweepFluxOnly<P>(eq, F.v, recRm, recL, DIR);
+  } else {
+    const typename P::Wave w = P::MakeWave(eq, C.v, DIR);
+    const typename P::Wave wm = ShflUp(w, 1);
+    const R s = SweepFace<P>(eq, F.v, recRm, recL, wm, w, DIR, own ? stats : other);
+    if (own) smax = s > smax ? s : smax;
+  }
+  const Flx Fr = ShflDown(F, 1);  // face j + 1
+  if (own && j < nd) {
+    const int64_t off = line.base + int64_t(j) * line.Stride();
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      const double v = u[c] + dt_dx * FluxDiff(F.v[c], Fr.v[c]);
+      a.out[c * line.cs + off] = v;
+      if (c == 0 && __double_as_longlong(v) <= 0) status |= kStatusNonPositiveDensity;
+    }
+  }
+  stats.Flush(a.stats_out);
+  const double smax_d = static_cast<double>(smax);
+  BlockMaxAtomic<1>(a.smax_out, &smax_d);
+  if (status && a.ctrl) atomicOr(&a.ctrl->step_status, status);
+}
+
 // The TMA-staged y/z sweep (a.tmap: the host's tensor map of a.in), built
 // for the mixed flavour's policies with lanes-along-x x sweeps.
 template <class P, class = void> struct TmaStaged : std::false_type {};
@@ -1005,6 +1162,18 @@ cudaError_t LaunchSweepT(const SweepArgs& a, cudaStream_t s) {
   const int seg = a.seg_len > 0 ? a.seg_len : nd;
   SweepArgs b = a;
   b.seg_len = seg;
+  if constexpr (HasLanes<P<D>>::value) {
+    if (a.lanes) {
+      const int64_t warps = (ntrans * (int64_t(nd) + 2) - 1 + kLaneStep - 1) / kLaneStep;
+      const unsigned lgrid = static_cast<unsigned>((warps * 32 + block - 1) / block);
+      if (a.dir == 0) SweepLanesKernel<D, 0, P><<<lgrid, block, 0, s>>>(b);
+      if constexpr (D >= 2)
+        if (a.dir == 1) SweepLanesKernel<D, 1, P><<<lgrid, block, 0, s>>>(b);
+      if constexpr (D >= 3)
+        if (a.dir == 2) SweepLanesKernel<D, 2, P><<<lgrid, block, 0, s>>>(b);
+      return cudaGetLastError();
+    }
+  }
   dim3 grid(static_cast<unsigned>((ntrans + block - 1) / block),
             static_cast<unsigned>((nd + seg - 1) / seg));
   switch (a.dir) {
