@@ -24,6 +24,7 @@
 // (subnormal, infinite and NaN among them) take the IEEE operation.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -120,6 +121,12 @@ __host__ __device__ __forceinline__ uint32_t ToUint(float x) {
 #endif
 }
 
+// The IEEE operations, out of line: operands outside the range below are rare,
+// and inlined they would double the kernels' code (instruction fetch bounds a
+// lone warp).
+static __host__ __device__ __noinline__ double IeeeDiv(double a, double b) { return a / b; }
+static __host__ __device__ __noinline__ double IeeeSqrt(double a) { return sqrt(a); }
+
 // Unsigned distance of a high word's exponent into [2^-510, 2^511): below
 // kSpan inside, at or above it outside (the sign bit drops out).
 constexpr uint32_t kSpan = 1021u << 21;
@@ -212,12 +219,10 @@ __host__ __device__ __forceinline__ double Div(double a, const Divisor& d) {
   const bool zero = ((ah * 2u) | al) == 0u;
   hi = zero ? sign : hi;
   lo = zero ? 0u : lo;
-  if (d.span >= kSpan || !(Span(ah) < kSpan || zero)) return (kHalf ? 0.5 * a : a) / d.b;
+  if (d.span >= kSpan || !(Span(ah) < kSpan || zero)) return IeeeDiv(kHalf ? 0.5 * a : a, d.b);
   return Make(hi, lo);
 }
 __host__ __device__ __forceinline__ double Div(double a, double b) { return Div(a, MakeDivisor(b)); }
-
-inline double HostSqrt(double a) { return __builtin_sqrt(a); }
 
 // kNear: without the deciding remainder, within 0.75 ulp.
 template <bool kNear = false> __host__ __device__ __forceinline__ double Sqrt(double a) {
@@ -248,11 +253,7 @@ template <bool kNear = false> __host__ __device__ __forceinline__ double Sqrt(do
   }
   const uint32_t er = ((h + (1021u << 20)) >> 1) & 0x7FF00000u;  // floor((e + 1021) / 2)
   if (h - 0x00100000u >= 0x7FE00000u) {  // zero, subnormal, negative, infinite, NaN
-#ifdef __CUDA_ARCH__
-    return sqrt(a);
-#else
-    return HostSqrt(a);
-#endif
+    return IeeeSqrt(a);
   }
   return Make(static_cast<uint32_t>(n >> 32) + er, static_cast<uint32_t>(n));
 }

@@ -19,7 +19,7 @@ __device__ __forceinline__ GodunovGas MakeGodunovGas(double gamma, int guess, in
                                                      double tol, const float* mlp) {
   GodunovGas g;
   g.eq.gamma = gamma;
-  g.eq.gamma_minus_1_inv = 1.0 / (gamma - 1.0);
+  g.eq.gamma_minus_1_inv = ieee64::Div(1.0, gamma - 1.0);
   g.opt.guess = guess;
   g.opt.max_iterations = max_it;
   g.opt.tol = tol;

@@ -199,7 +199,7 @@ __device__ __forceinline__ double HalfSlope(int limiter, double qL, double qM, d
     hs = pos ? hs : 0.0;
     if (ieee64::Span(ieee64::Hi(c)) >= ieee64::kSpan && !ieee64::IsZero(sL) && !ieee64::IsZero(sR)) {
       const double c2 = 2.0 * sL * sR;
-      hs = 0.5 * ((c2 > 0.0) ? c2 / (sL + sR) : 0.0);
+      hs = 0.5 * ((c2 > 0.0) ? ieee64::IeeeDiv(c2, sL + sR) : 0.0);
     }
     return hs;
   }

@@ -22,7 +22,7 @@ template <int D> struct ExactPolicy {
   static __device__ __forceinline__ Gas MakeGas(double gamma) {
     Gas g;
     g.gamma = gamma;
-    g.gamma_minus_1_inv = 1.0 / (gamma - 1.0);
+    g.gamma_minus_1_inv = ieee64::Div(1.0, gamma - 1.0);
     return g;
   }
   static __device__ __forceinline__ Gas MakeGasFor(const SweepArgs& a) {

@@ -133,8 +133,8 @@ __device__ __forceinline__ bool SweepGate(const SweepArgs& a, double split_dt) {
     if (a.ctrl->abort || a.ctrl->done) return false;
     if (a.prev_check >= 0) {
       const double smax = BitsToDouble(a.ctrl->smax_check[a.prev_check]);
-      const double level_dt = a.prev_dx / smax;
-      if (level_dt < split_dt) return false;
+      const double level_dt = ieee64::Div(a.prev_dx, smax);
+      if (ieee64::Less(level_dt, split_dt)) return false;
     }
   }
   return true;
@@ -406,8 +406,8 @@ __device__ __forceinline__ void MarchSegment(const SweepArgs& a, Line& line, int
   // the FP32 screen's error bound is stated for 1 < gamma <= 2
   const bool screen = kFilter && !skip_cfl && a.gamma > 1.0 && a.gamma <= 2.0;
   const typename P::Gas eq = P::MakeGasFor(a);
-  const double lambda_half = 0.5 * split_dt / a.dx;
-  const double dt_dx = split_dt / a.dx;
+  const double lambda_half = ieee64::Div(0.5 * split_dt, a.dx);
+  const double dt_dx = ieee64::Div(split_dt, a.dx);
   using R = typename P::Real;
   double* __restrict__ out = a.out;
   const int64_t cs = line.cs;
@@ -800,8 +800,8 @@ __device__ __forceinline__ void XWarpRow(const SweepArgs& a, int64_t row, double
   const int64_t base = row * nx;
   const bool periodic = (a.bc == 0);
   const typename P::Gas eq = P::MakeGasFor(a);
-  const double lambda_half = 0.5 * split_dt / a.dx;
-  const double dt_dx = split_dt / a.dx;
+  const double lambda_half = ieee64::Div(0.5 * split_dt, a.dx);
+  const double dt_dx = ieee64::Div(split_dt, a.dx);
   const double* __restrict__ in = a.in;
   double* __restrict__ out = a.out;
   auto load = [&](Dbl& u, int x) {
@@ -1033,8 +1033,8 @@ __global__ void __launch_bounds__(128, PT<D>::kLaneBlocks) SweepLanesKernel(Swee
     line.stride = int64_t(nx) * ny;
   }
   const typename P::Gas eq = P::MakeGasFor(a);
-  const double lambda_half = 0.5 * split_dt / a.dx;
-  const double dt_dx = split_dt / a.dx;
+  const double lambda_half = ieee64::Div(0.5 * split_dt, a.dx);
+  const double dt_dx = ieee64::Div(split_dt, a.dx);
   const bool skip_cfl = HasFluxOnly<P>::value && a.skip_cfl != 0;
   constexpr bool kFilter = FilteredCfl<P>::value && HasFluxOnly<P>::value;
 
