@@ -57,11 +57,14 @@ struct LevelHost {
   int32_t nrows[2] = {0, 0};
   Seg* segs[2][kSplits] = {};
   int32_t nsegs[2][kSplits] = {};
-  int split[2] = {0, 0};  // index into kSplitOf; kSplits: x rows with lanes along x
-  // slots of the x sweep with lanes along x (PatchSweepArgs::slot_row)
-  int32_t* slot_row = nullptr;
-  int32_t* row_slot0 = nullptr;
-  int64_t nslots = 0;
+  int split[2] = {0, 0};  // index into kSplitOf; kSplits: the lanes of a warp along the rows
+  // slots of the sweeps with lanes along the rows (PatchSweepArgs::slot_row)
+  int32_t* slot_row[2] = {nullptr, nullptr};
+  int32_t* row_slot0[2] = {nullptr, nullptr};
+  int64_t nslots[2] = {0, 0};
+  int64_t RowWarps(int d) const {
+    return std::max<int64_t>(1, (nslots[d] - 1 + kRowWarpStep - 1) / kRowWarpStep);
+  }
   Cap* caps[2] = {nullptr, nullptr};
   RefluxCell* reflux = nullptr;
   int32_t nreflux = 0;
@@ -421,16 +424,16 @@ int Build(fvs_amr* a) {
         Lv.nsegs[d][si] = int32_t(segs.size());
         AMR_CUDA(a->Upload(&Lv.segs[d][si], segs));
       }
-      if (d == 0) {
-        // x rows end to end as slots, cells -1..n of each
+      {
+        // rows end to end as slots, cells -1..n of each
         std::vector<int32_t> slot_row, row_slot0(R.size());
         for (size_t r = 0; r < R.size(); ++r) {
           row_slot0[r] = int32_t(slot_row.size());
           slot_row.insert(slot_row.end(), size_t(R[r].n) + 2, int32_t(r));
         }
-        Lv.nslots = int64_t(slot_row.size());
-        AMR_CUDA(a->Upload(&Lv.slot_row, slot_row));
-        AMR_CUDA(a->Upload(&Lv.row_slot0, row_slot0));
+        Lv.nslots[d] = int64_t(slot_row.size());
+        AMR_CUDA(a->Upload(&Lv.slot_row[d], slot_row));
+        AMR_CUDA(a->Upload(&Lv.row_slot0[d], row_slot0));
       }
     }
     AMR_CUDA(a->Upload(&Lv.reflux, reflux_h[size_t(l)]));
@@ -443,8 +446,15 @@ int Build(fvs_amr* a) {
     for (auto& kv : h)
       Lv.hist += std::to_string(kv.first.first) + "x" + std::to_string(kv.first.second) + ":" +
                  std::to_string(kv.second) + ",";
-    for (int d = 0; d < 2; ++d)
+    for (int d = 0; d < 2; ++d) {
       Lv.grid[d] = std::max(1, std::min((Lv.nsegs[d][0] + 127) / 128, a->sms * 4));
+      // FP64 levels start with the lanes along the rows (a 65 k-cell level's
+      // sweep: 0.58 ms marching one thread per row, 20 us so)
+      if (a->m.precision != FVS_MIXED) {
+        Lv.split[d] = kSplits;
+        Lv.grid[d] = static_cast<int>(std::min<int64_t>((Lv.RowWarps(d) + 3) / 4, a->sms * 64));
+      }
+    }
   }
   AMR_CUDA(a->Alloc(&a->reg, size_t(std::max(a->nslots, 1)) * 3 * kComp));
   AMR_CUDA(a->Upload(&a->signs, signs_h));
@@ -482,12 +492,12 @@ cudaError_t LaunchSweep(fvs_amr* a, int l, int d, const double* in, double* out,
     s.coarse = a->L[size_t(l - 1)].A;
     s.coarse_ncells = int32_t(a->L[size_t(l - 1)].ncells);
   }
-  if (split == kSplits) {  // x rows with the lanes of a warp along x
+  if (split == kSplits) {  // the lanes of a warp along the rows
     s.segs = Lv.segs[d][0];
     s.nsegs = Lv.nsegs[d][0];
-    s.slot_row = Lv.slot_row;
-    s.row_slot0 = Lv.row_slot0;
-    s.nslots = Lv.nslots;
+    s.slot_row = Lv.slot_row[d];
+    s.row_slot0 = Lv.row_slot0[d];
+    s.nslots = Lv.nslots[d];
     occ += 10;
   } else {
     s.segs = Lv.segs[d][split];
@@ -526,8 +536,17 @@ cudaError_t LaunchMaxSpeed(fvs_amr* a, int l, int d) {
   s.gamma = a->m.gamma;
   s.smax_out = &a->ctrl->smax_stable[l][d];
   const int block = 128;
+  int64_t threads = s.nsegs;
+  if (a->m.precision != FVS_MIXED) {  // one face per lane
+    s.segs = Lv.segs[d][0];
+    s.nsegs = Lv.nsegs[d][0];
+    s.slot_row = Lv.slot_row[d];
+    s.row_slot0 = Lv.row_slot0[d];
+    s.nslots = Lv.nslots[d];
+    threads = (s.nslots - 1 + kLaneFaces - 1) / kLaneFaces * 32;
+  }
   const int grid = static_cast<int>(std::max<int64_t>(
-      1, std::min<int64_t>((int64_t(s.nsegs) + block - 1) / block, int64_t(a->sms) * 16)));
+      1, std::min<int64_t>((threads + block - 1) / block, int64_t(a->sms) * 16)));
   switch (a->m.precision) {
   case FVS_FP64_EXACT:
     return LaunchPatchMaxSpeedExact(d, s, grid, block, a->stream);
@@ -961,16 +980,14 @@ int fvs_amr_autotune(fvs_amr* a, int32_t* configs) {
       float best = 1e30f;
       Tuned bt{128, Lv.grid[d], 0, 0};
       const bool mixed = a->m.precision == FVS_MIXED;
-      // splits of the marching kernel, and (mixed x sweeps) the kernel with
-      // the lanes of a warp along x
+      // splits of the marching kernel, and (mixed: x sweeps) the kernel with
+      // the lanes of a warp along the rows
       for (int si = 0; si <= kSplits; ++si) {
-        if (si == kSplits && !(mixed && d == 0)) continue;
+        if (si == kSplits && mixed && d != 0) continue;
         if (si > 0 && si < kSplits && Lv.nsegs[d][si] == Lv.nsegs[d][si - 1])
           continue;  // rows too short
         const int64_t threads =
-            si == kSplits
-                ? 32 * std::max<int64_t>(1, (Lv.nslots - 1 + kRowWarpStep - 1) / kRowWarpStep)
-                : int64_t(Lv.nsegs[d][si]);
+            si == kSplits ? 32 * Lv.RowWarps(d) : int64_t(Lv.nsegs[d][si]);
         for (int occ : {0, 5}) {
           if (occ && !mixed) continue;
           for (int block : {64, 128}) {

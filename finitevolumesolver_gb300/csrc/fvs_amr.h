@@ -119,7 +119,7 @@ struct PatchSweepArgs {
   double dt_scale;       // split dt = dt_scale * (*dt_ptr)
   unsigned long long* smax_out;  // this sweep's max signal speed (bits)
   AmrControl* ctrl;
-  // x sweeps with the lanes of a warp along x (PatchRowWarpKernel): the
+  // sweeps with the lanes of a warp along the rows (PatchRowWarpKernel): the
   // level's rows (segs, one segment per row) laid end to end as slots,
   // n + 2 per row (cells -1..n); slot_row[s] is slot s's row, row_slot0[r]
   // row r's first slot
@@ -131,6 +131,8 @@ struct PatchSweepArgs {
 // Slots of a row-warp sweep: warp w takes slots kRowWarpStep * w ..
 // kRowWarpStep * w + 31 and owns (updates, captures, CFL) the middle 30.
 constexpr int kRowWarpStep = 30;
+// Slots (faces on their cells' left) a warp of the max-speed pass owns.
+constexpr int kLaneFaces = 31;
 
 struct MaxSpeedArgs {
   const double* in;
@@ -141,11 +143,16 @@ struct MaxSpeedArgs {
   int32_t nsegs;
   double gamma;
   unsigned long long* smax_out;
+  // nslots > 0: one face per lane over the rows' slots (segs: whole rows)
+  const int32_t* slot_row;
+  const int32_t* row_slot0;
+  int64_t nslots;
 };
 
 // Launchers (fvs_amr_exact.cu: exact FP64 and the table kernels, compiled
 // with -fmad=false; fvs_amr_fast.cu: fast FP64 and mixed).  `grid` is the
 // number of persistent blocks.
+// a.nslots > 0: with the lanes of a warp along the rows
 cudaError_t LaunchPatchSweepExact(int dir, const PatchSweepArgs& a, int grid, int block,
                                   cudaStream_t s);
 cudaError_t LaunchPatchSweepFast(int dir, const PatchSweepArgs& a, int grid, int block,

@@ -12,11 +12,13 @@ namespace amr {
 
 cudaError_t LaunchPatchSweepExact(int dir, const PatchSweepArgs& a, int grid, int block,
                                   cudaStream_t s) {
+  if (a.nslots > 0) return LaunchPatchRowWarpT<ExactPolicy>(dir, a, grid, block, s);
   return LaunchPatchSweepT<ExactPolicy>(dir, a, grid, block, s);
 }
 
 cudaError_t LaunchPatchMaxSpeedExact(int dir, const MaxSpeedArgs& a, int grid, int block,
                                      cudaStream_t s) {
+  if (a.nslots > 0) return LaunchPatchMaxSpeedLanesT<ExactPolicy>(dir, a, grid, block, s);
   return LaunchPatchMaxSpeedT<ExactPolicy>(dir, a, grid, block, s);
 }
 

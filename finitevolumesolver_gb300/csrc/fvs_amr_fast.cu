@@ -9,6 +9,7 @@ namespace amr {
 
 cudaError_t LaunchPatchSweepFast(int dir, const PatchSweepArgs& a, int grid, int block,
                                  cudaStream_t s) {
+  if (a.nslots > 0) return LaunchPatchRowWarpT<Fast64Policy>(dir, a, grid, block, s);
   return LaunchPatchSweepT<Fast64Policy>(dir, a, grid, block, s);
 }
 
@@ -17,8 +18,8 @@ cudaError_t LaunchPatchSweepFast(int dir, const PatchSweepArgs& a, int grid, int
 cudaError_t LaunchPatchSweepMixed(int dir, const PatchSweepArgs& a, int grid, int block,
                                   int occupancy, cudaStream_t s) {
   if (dir == 0 && occupancy >= 10) {
-    if (occupancy == 15) return LaunchPatchRowWarpT<Mixed32PolicyOcc5>(a, grid, block, s);
-    return LaunchPatchRowWarpT<Mixed32Policy>(a, grid, block, s);
+    if (occupancy == 15) return LaunchPatchRowWarpT<Mixed32PolicyOcc5>(dir, a, grid, block, s);
+    return LaunchPatchRowWarpT<Mixed32Policy>(dir, a, grid, block, s);
   }
   if (occupancy == 5) return LaunchPatchSweepT<Mixed32PolicyOcc5>(dir, a, grid, block, s);
   return LaunchPatchSweepT<Mixed32Policy>(dir, a, grid, block, s);
@@ -26,6 +27,7 @@ cudaError_t LaunchPatchSweepMixed(int dir, const PatchSweepArgs& a, int grid, in
 
 cudaError_t LaunchPatchMaxSpeedFast(int dir, const MaxSpeedArgs& a, int grid, int block,
                                     cudaStream_t s) {
+  if (a.nslots > 0) return LaunchPatchMaxSpeedLanesT<Fast64Policy>(dir, a, grid, block, s);
   return LaunchPatchMaxSpeedT<Fast64Policy>(dir, a, grid, block, s);
 }
 

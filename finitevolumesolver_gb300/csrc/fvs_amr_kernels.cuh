@@ -39,8 +39,8 @@ __global__ void __launch_bounds__(128, PT<2>::kMinBlocks) PatchSweepKernel(Patch
   constexpr int K = kComp;
   const double split_dt = a.dt_scale * (*a.dt_ptr);
   const typename P::Gas eq = P::MakeGas(a.gamma);
-  const double lambda_half = 0.5 * split_dt / a.dx;
-  const double dt_dx = split_dt / a.dx;
+  const double lambda_half = ieee64::Div(0.5 * split_dt, a.dx);
+  const double dt_dx = ieee64::Div(split_dt, a.dx);
   const int64_t N = a.ncells;
   const double* __restrict__ in = a.in;
   double* __restrict__ out = a.out;
@@ -185,37 +185,101 @@ __global__ void __launch_bounds__(128, PT<2>::kMinBlocks) PatchSweepKernel(Patch
   if (status) atomicOr(&a.ctrl->step_status, status);
 }
 
-// PatchRowWarpKernel: the x sweeps of the mixed flavour with the lanes of a
-// warp along x.  The level's x rows are laid end to end as slots, n + 2 per
-// row (cells -1..n); warp w takes slots 30w .. 30w + 31 (grid-stride).  Lane
-// l holds the cell of slot 30w + l in the compute precision and gets its
-// neighbours by shuffles, or loads them where the neighbour lies in another
-// row (the halo cells -2 and n + 1) or outside the warp; it evaluates that
-// cell's MUSCL predictor once, and lanes 1..31 the flux of the face on the
-// cell's left.  Lanes 1..30 own their slots: they update interior cells
-// (0 <= c < n) with the faces on both sides (the right one from the next
-// lane), accumulate captured faces into the flux registers and fold their
-// faces' signal speeds into the sweep's maximum.  Every predictor is
-// evaluated once per row (plus those of cells -1 and n, which faces 0 and n
-// need), where PatchSweepKernel's segments repeat two per segment and load
-// four halo cells each, and a warp's loads of a row are consecutive.  The
-// arithmetic per cell and face is PatchSweepKernel's: the results are the
-// same, bit for bit.  Policies whose CFL speeds are FP32-screened (the FP64
-// flavours) keep PatchSweepKernel.
-template <template <int> class PT>
+// The cell at position x (-2..n+1) of a row: interior, or a halo cell where
+// it lives (this level or the coarser one; a reflective image's momentum
+// along the row negated).
+template <int DIR>
+__device__ __forceinline__ void LoadRowCell(double* u, const Seg* seg, int n, int x,
+                                            const double* __restrict__ in, int64_t N,
+                                            const double* __restrict__ coarse, int64_t NC) {
+  const double* src = in;
+  int64_t off, cs = N;
+  bool flip = false;
+  if (x >= 0 && x < n) {
+    off = int64_t(seg->base) + int64_t(x + kGhost) * (DIR == 0 ? 1 : seg->stride);
+  } else {
+    const int h = x < 0 ? x + 2 : x - n + 2;
+    const int32_t g = seg->halo[h];
+    if (g >= 0) {
+      off = g;
+    } else {
+      off = -int64_t(g) - 1;
+      src = coarse;
+      cs = NC;
+    }
+    flip = (seg->flip >> h) & 1;
+  }
+#pragma unroll
+  for (int k = 0; k < kComp; ++k) u[k] = __ldg(src + k * cs + off);
+  if (flip) u[1 + DIR] = -u[1 + DIR];
+}
+
+// The CFL speed of the face between a lane's cell and its left neighbour's
+// (by shuffles), folded into smax for `own` lanes.  Screened policies evaluate
+// it only in warps one of whose faces can hold the launch's maximum (the FP32
+// bound of the marching sweep against the published maximum).
+template <int DIR, class P, class Real>
+__device__ __forceinline__ void LaneFaceSpeed(const typename P::Gas& eq, const Real* c,
+                                              double gamma, unsigned long long* slot, bool own,
+                                              Real& smax) {
+  if constexpr (EinfeldtCfl<P>::value) {
+    fast::Gas<float> g32;
+    g32.gamma = static_cast<float>(gamma);
+    g32.gm1 = static_cast<float>(gamma - 1.0);
+    const float thr =
+        CflFloatBelow(BitsToDouble(*reinterpret_cast<volatile unsigned long long*>(slot)));
+    float c32[kComp];
+#pragma unroll
+    for (int k = 0; k < kComp; ++k) c32[k] = CflToF32(c[k]);
+    const fast::Wave<float> v = fast::MakeWave<2, float>(g32, c32, DIR);
+    const bool ok = gamma > 1.0 && gamma <= 2.0 && CflInRange<2>(c32) && v.a > 0.0f;
+    const fast::Wave<float> vm = ShflUp(v, 1);
+    const bool okm = __shfl_up_sync(0xffffffffu, ok ? 1 : 0, 1) != 0;
+    const float s32 = fast::FaceMaxSpeed<float>(g32, vm, v);
+    const float sh = fast::Math<float>::Sqrt(fmaxf(vm.h, v.h));
+    const float bound = fmaf(s32, kCflRel, fmaf(kCflScale, sh, kCflAbs));
+    if (!__any_sync(0xffffffffu, own && !(ok && okm && bound < thr))) return;
+  }
+  const typename P::Wave w = P::MakeWave(eq, c, DIR);
+  const typename P::Wave wm = ShflUp(w, 1);
+  const Real s = P::FaceMaxSpeed(eq, wm, w);
+  if (own) smax = s > smax ? s : smax;
+}
+
+// PatchRowWarpKernel: the sweep with the lanes of a warp along the rows.  The
+// level's rows are laid end to end as slots, n + 2 per row (cells -1..n);
+// warp w takes slots 30w .. 30w + 31 (grid-stride).  Lane l holds the cell of
+// slot 30w + l in the compute precision and gets its neighbours by shuffles,
+// or loads them where the neighbour lies in another row (the halo cells -2
+// and n + 1) or outside the warp; it evaluates that cell's MUSCL predictor
+// once, and the flux of the face on the cell's left.  Lanes 1..30 own their
+// slots: they update interior cells (0 <= c < n) with the faces on both sides
+// (the right one from the next lane), accumulate captured faces into the flux
+// registers and fold their faces' signal speeds into the sweep's maximum.
+// Every predictor is evaluated once per row (plus those of cells -1 and n,
+// which faces 0 and n need), where PatchSweepKernel's segments repeat two per
+// segment and load four halo cells each, and a warp's loads of an x row are
+// consecutive.  The arithmetic per cell and face is PatchSweepKernel's: the
+// results are the same, bit for bit.
+//
+// FP64 flavours take it in both directions: a marching thread's row is a
+// serial chain of FP64 instructions (64 clocks each in the FP64 unit that one
+// warp saturates), and a level of 65 k cells has only ~2000 rows, 60 warps on
+// the chip; as slots it has 2300 warps.  Mixed: x only (y columns would load a
+// sector per value).
+template <int DIR, template <int> class PT>
 __global__ void __launch_bounds__(128, PT<2>::kMinBlocks) PatchRowWarpKernel(PatchSweepArgs a) {
   using P = PT<2>;
   using R = typename P::Real;
   constexpr int K = kComp;
-  static_assert(!(EinfeldtCfl<P>::value && HasFluxOnly<P>::value),
-                "screened-CFL policies use PatchSweepKernel");
+  constexpr bool kFilter = EinfeldtCfl<P>::value && HasFluxOnly<P>::value;
   using Cell = CellArr<R, K>;
   using FluxT = typename FluxOf<P>::type;
   using Flx = CellArr<FluxT, K>;
   const double split_dt = a.dt_scale * (*a.dt_ptr);
   const typename P::Gas eq = P::MakeGas(a.gamma);
-  const double lambda_half = 0.5 * split_dt / a.dx;
-  const double dt_dx = split_dt / a.dx;
+  const double lambda_half = ieee64::Div(0.5 * split_dt, a.dx);
+  const double dt_dx = ieee64::Div(split_dt, a.dx);
   const int64_t N = a.ncells;
   const double* __restrict__ in = a.in;
   double* __restrict__ out = a.out;
@@ -227,82 +291,58 @@ __global__ void __launch_bounds__(128, PT<2>::kMinBlocks) PatchRowWarpKernel(Pat
   const int64_t wstride = (int64_t(gridDim.x) * blockDim.x) >> 5;
   for (int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < nwarps;
        w += wstride) {
+    // slots past the end take the last one again and own nothing
     const int64_t s = w * kRowWarpStep + lane;
     const bool valid = s < a.nslots;
-    Seg row{};
-    int c = 0;
-    if (valid) {
-      const int32_t r = a.slot_row[s];
-      row = a.segs[r];
-      c = static_cast<int>(s - a.row_slot0[r]) - 1;
-    }
-    // cell x (-2..n+1) of the slot's row: interior, or a halo cell where it
-    // lives (this level or the coarser one, a reflective image flipped)
+    const int64_t sc = valid ? s : a.nslots - 1;
+    const int32_t r = a.slot_row[sc];
+    const Seg* row = a.segs + r;
+    const int n = row->n;
+    const int c = static_cast<int>(sc - a.row_slot0[r]) - 1;
     auto load = [&](double* u, int x) {
-      const double* src = in;
-      int64_t off, cs = N;
-      bool flip = false;
-      if (x >= 0 && x < row.n) {
-        off = int64_t(row.base) + x + kGhost;
-      } else {
-        const int h = x < 0 ? x + 2 : x - row.n + 2;
-        const int32_t g = row.halo[h];
-        if (g >= 0) {
-          off = g;
-        } else {
-          off = -int64_t(g) - 1;
-          src = a.coarse;
-          cs = a.coarse_ncells;
-        }
-        flip = (row.flip >> h) & 1;
-      }
-#pragma unroll
-      for (int k = 0; k < K; ++k) u[k] = __ldg(src + k * cs + off);
-      if (flip) u[1] = -u[1];
+      LoadRowCell<DIR>(u, row, n, x, in, N, a.coarse, a.coarse_ncells);
     };
-    Cell C{}, Cm{}, Cp{};
+    Cell C, Cm, Cp;
     double u[K];
-    if (valid) {
-      load(u, c);
-      P::ToCell(C.v, u);
+    load(u, c);
+    P::ToCell(C.v, u);
+    Cm = ShflUp(C, 1);
+    Cp = ShflDown(C, 1);
+    if (c == -1 || lane == 0) {
+      load(u, c - 1);
+      P::ToCell(Cm.v, u);
     }
-    const Cell up = ShflUp(C, 1), down = ShflDown(C, 1);
-    if (valid) {
-      if (c == -1 || lane == 0) {
-        load(u, c - 1);
-        P::ToCell(Cm.v, u);
-      } else {
-        Cm = up;
-      }
-      if (c == row.n || lane == 31) {
-        load(u, c + 1);
-        P::ToCell(Cp.v, u);
-      } else {
-        Cp = down;
-      }
+    if (c == n || lane == 31) {
+      load(u, c + 1);
+      P::ToCell(Cp.v, u);
     }
-    typename P::Rec recL, recR;
-    P::Predict(eq, recL, recR, Cm.v, C.v, Cp.v, a.limiter, lambda_half, 0);
-    const typename P::Wave W = P::MakeWave(eq, C.v, 0);
-    const typename P::Rec recRm = ShflUp(recR, 1);
-    const typename P::Wave Wm = ShflUp(W, 1);
-    // face c (cells c-1 and c)
-    Flx F{};
-    R sp = R(0);
-    if (valid && lane >= 1 && c >= 0) sp = SweepFace<P>(eq, F.v, recRm, recL, Wm, W, 0, stats);
-    const Flx Fr = ShflDown(F, 1);  // face c + 1
     const bool own = valid && lane >= 1 && lane <= kRowWarpStep && c >= 0;
+    if constexpr (kFilter) LaneFaceSpeed<DIR, P, R>(eq, C.v, a.gamma, a.smax_out, own, smax);
+    typename P::Rec recL, recR;
+    P::Predict(eq, recL, recR, Cm.v, C.v, Cp.v, a.limiter, lambda_half, DIR);
+    const typename P::Rec recRm = ShflUp(recR, 1);
+    // face c (cells c-1 and c)
+    Flx F;
+    if constexpr (kFilter) {
+      SweepFluxOnly<P>(eq, F.v, recRm, recL, DIR);
+    } else {
+      const typename P::Wave W = P::MakeWave(eq, C.v, DIR);
+      const typename P::Wave Wm = ShflUp(W, 1);
+      const R sp = SweepFace<P>(eq, F.v, recRm, recL, Wm, W, DIR, stats);
+      if (own) smax = sp > smax ? sp : smax;
+    }
+    const Flx Fr = ShflDown(F, 1);  // face c + 1
     if (own) {
-      smax = sp > smax ? sp : smax;
-      for (int q = row.cap_begin; q < row.cap_end; ++q) {
+      const int cap_end = row->cap_end;
+      for (int q = row->cap_begin; q < cap_end; ++q) {
         const Cap cp = a.caps[q];
         if (cp.face != c) continue;
         double* dst = a.reg + int64_t(cp.dst) * K;
 #pragma unroll
         for (int k = 0; k < K; ++k) dst[k] = dst[k] + split_dt * FluxWiden(F.v[k]);
       }
-      if (c < row.n) {
-        const int64_t off = int64_t(row.base) + c + kGhost;
+      if (c < n) {
+        const int64_t off = int64_t(row->base) + int64_t(c + kGhost) * (DIR == 0 ? 1 : row->stride);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           const double v = __ldg(in + k * N + off) + dt_dx * FluxDiff(F.v[k], Fr.v[k]);
@@ -318,9 +358,55 @@ __global__ void __launch_bounds__(128, PT<2>::kMinBlocks) PatchRowWarpKernel(Pat
 }
 
 template <template <int> class PT>
-cudaError_t LaunchPatchRowWarpT(const PatchSweepArgs& a, int grid, int block, cudaStream_t s) {
+cudaError_t LaunchPatchRowWarpT(int dir, const PatchSweepArgs& a, int grid, int block,
+                                cudaStream_t s) {
   if (a.nslots == 0) return cudaSuccess;
-  PatchRowWarpKernel<PT><<<grid, block, 0, s>>>(a);
+  if constexpr (EinfeldtCfl<PT<2>>::value) {
+    if (dir == 1) {
+      PatchRowWarpKernel<1, PT><<<grid, block, 0, s>>>(a);
+      return cudaGetLastError();
+    }
+  }
+  PatchRowWarpKernel<0, PT><<<grid, block, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+// PatchMaxSpeedKernel (below) over the slots of PatchRowWarpKernel: one cell
+// and the face on its left per lane.
+template <int DIR, template <int> class PT>
+__global__ void __launch_bounds__(128) PatchMaxSpeedLanesKernel(MaxSpeedArgs a) {
+  using P = PT<2>;
+  using R = typename P::Real;
+  const typename P::Gas eq = P::MakeGas(a.gamma);
+  const int lane = threadIdx.x & 31;
+  R smax = R(0);
+  const int64_t nwarps = a.nslots > 1 ? (a.nslots - 1 + kLaneFaces - 1) / kLaneFaces : 0;
+  const int64_t wstride = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < nwarps;
+       w += wstride) {
+    const int64_t s = w * kLaneFaces + lane;
+    const int64_t sc = s < a.nslots ? s : a.nslots - 1;
+    const int32_t r = a.slot_row[sc];
+    const Seg* row = a.segs + r;
+    const int c = static_cast<int>(sc - a.row_slot0[r]) - 1;
+    double u[kComp];
+    LoadRowCell<DIR>(u, row, row->n, c, a.in, a.ncells, a.coarse, a.coarse_ncells);
+    R v[kComp];
+    P::ToCell(v, u);
+    const bool own = s < a.nslots && lane >= 1 && c >= 0;
+    LaneFaceSpeed<DIR, P, R>(eq, v, a.gamma, a.smax_out, own, smax);
+  }
+  const double smax_d = static_cast<double>(smax);
+  BlockMaxAtomic<1>(a.smax_out, &smax_d);
+}
+
+template <template <int> class PT>
+cudaError_t LaunchPatchMaxSpeedLanesT(int dir, const MaxSpeedArgs& a, int grid, int block,
+                                      cudaStream_t s) {
+  if (dir == 0)
+    PatchMaxSpeedLanesKernel<0, PT><<<grid, block, 0, s>>>(a);
+  else
+    PatchMaxSpeedLanesKernel<1, PT><<<grid, block, 0, s>>>(a);
   return cudaGetLastError();
 }
 
