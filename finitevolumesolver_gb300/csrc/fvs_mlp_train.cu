@@ -2,16 +2,24 @@
 // (forward, backward, Adam) and batched inference of the 5 -> 64 -> 64 -> 1
 // GELU perceptron, all hand-written for sm_103a.
 //
-// Layout of the network (B = batch rows, a multiple of 128):
-//   X   [B][16] bf16   standardised features, columns 5..15 zero
-//   Z1  [B][64] fp32 = X W1^T + b1,  H1 = GELU(Z1) (bf16 [B][64] and [64][B])
-//   Z2  [B][64] fp32 = H1 W2^T + b2, H2 = GELU(Z2)
-//   y   [B]          = H2 . w3 + b3   (CUDA cores)
-// Loss: mean squared error against y* = log(p* / max(pL, pR)).
-// Backward: dZ2 = (dy w3) * GELU'(Z2); dH1 = dZ2 W2 (tcgen05);
-// dW2 = dZ2^T H1 (tcgen05, split over the batch); dZ1 = dH1 * GELU'(Z1);
-// dW1 = dZ1^T X (tcgen05).  The M = 64 weight-gradient products run as
-// M = 128 tiles whose upper 64 rows are loaded as zeros and not stored.
+// A training step is two kernels.  FusedStepKernel: a CTA takes tiles of 128
+// batch rows through the whole forward and backward pass, every operand of
+// the five products staged in shared memory and every accumulator in tensor
+// memory (bf16 operands, fp32 accumulation):
+//   X   [128][16] bf16   sampled rows, standardised, columns 5..15 zero
+//   Z1  = X W1^T + b1,   H1 = GELU(Z1) (bf16)
+//   Z2  = H1 W2^T + b2,  y = GELU(Z2) . w3 + b3 (CUDA cores)
+//   dZ2 = (dy w3) * GELU'(Z2) (bf16), dH1 = dZ2 W2, dZ1 = dH1 * GELU'(Z1) (bf16)
+//   [dZ2 | dZ1]^T [H1 | X]: one 128 x 80 product whose diagonal blocks are dW2
+//   and dW1, accumulated in tensor memory over the CTA's tiles
+// with the loss the mean squared error against y* = log(p* / max(pL, pR)).
+// It writes the CTA's sums of the gradient; UpdateKernel adds them over the
+// CTAs in a fixed order, applies Adam and publishes the bf16 weights.
+//
+// The step is latency: 0.2 GFLOP at batch 8192.  As twelve kernels (gather,
+// one GEMM kernel per product, activations, reductions by atomics, Adam) with
+// their operands in global memory it took 121 us on the GB300; fused it takes
+// about 15 us.
 #include "../../include/fvs_gpu.h"
 #include "fvs_internal.h"
 #include "fvs_mlp.cuh"
@@ -20,6 +28,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -192,14 +201,14 @@ cudaError_t LaunchGemm(const GemmArgs& a, int splits, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// Elementwise parts
+// The network
 
-__device__ __forceinline__ float Gelu(float x) { return mlp::Gelu(x); }
-
-__device__ __forceinline__ float GeluGrad(float x) {
+// GELU and its derivative from one tanh.
+__device__ __forceinline__ float GeluBoth(float x, float* grad) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
   const float t = tanhf(k0 * fmaf(k1 * x * x, x, x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k0 * fmaf(3.0f * k1, x * x, 1.0f);
+  *grad = 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k0 * fmaf(3.0f * k1, x * x, 1.0f);
+  return 0.5f * x * (1.0f + t);
 }
 
 // Features and labels of Riemann problems given by primitive states.
@@ -253,11 +262,8 @@ struct Net {
   __nv_bfloat16* W2t;  // [64][64] transposed
 };
 
-// bf16 copies of the weights and the inference blob from the master weights.
-__global__ void PublishKernel(Net net) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= mlp::kParams) return;
-  const float w = net.master[i];
+// Parameter i's bf16 copies (weights) and its entry of the inference blob.
+__device__ __forceinline__ void PublishOne(const Net& net, int i, float w) {
   float out = w;
   if (i >= mlp::kOffW1 && i < mlp::kOffB1) {
     const int o = (i - mlp::kOffW1) / mlp::kIn, k = (i - mlp::kOffW1) % mlp::kIn;
@@ -274,29 +280,10 @@ __global__ void PublishKernel(Net net) {
   net.blob[i] = out;
 }
 
-struct StepBuffers {
-  int batch;
-  const float* feat;   // raw features [n][5]
-  const float* label;  // [n]
-  int64_t n;
-  uint64_t seed;
-  unsigned long long* step;  // device step counter
-  __nv_bfloat16* X;    // [B][16]
-  __nv_bfloat16* Xt;   // [16][B]
-  float* target;       // [B]
-  float* Z1;           // [B][64]
-  __nv_bfloat16* H1;   // [B][64]
-  __nv_bfloat16* H1t;  // [64][B]
-  float* Z2;           // [B][64]
-  __nv_bfloat16* D2;   // dZ2 [B][64]
-  __nv_bfloat16* D2t;  // dZ2^T [64][B]
-  float* dH1;          // [B][64]
-  __nv_bfloat16* D1t;  // dZ1^T [64][B]
-  float* dW2;          // [64][64]
-  float* dW1;          // [64][16]
-  float* loss;         // accumulated loss (sum of squared errors)
-  int use_given_rows;  // 1: rows are 0..B-1 of feat (gradient check)
-};
+__global__ void PublishKernel(Net net) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < mlp::kParams) PublishOne(net, i, net.master[i]);
+}
 
 __device__ __forceinline__ uint64_t Mix(uint64_t x) {
   // SplitMix64 finaliser
@@ -306,175 +293,416 @@ __device__ __forceinline__ uint64_t Mix(uint64_t x) {
   return x ^ (x >> 31);
 }
 
-// Sample the batch rows, standardise the features, write X and X^T.
-__global__ void GatherKernel(StepBuffers b, const float* stats) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= b.batch) return;
-  int64_t row;
-  if (b.use_given_rows) {
-    row = r;
-  } else {
-    const uint64_t h = Mix(b.seed ^ Mix(*b.step * 0x100000001ull + uint64_t(r)));
-    row = int64_t(h % uint64_t(b.n));
-  }
-  for (int k = 0; k < kXin; ++k) {
-    float v = 0.0f;
-    if (k < mlp::kIn)
-      v = (b.feat[row * mlp::kIn + k] - stats[mlp::kOffMean + k]) * stats[mlp::kOffInvStd + k];
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    b.X[int64_t(r) * kXin + k] = h;
-    b.Xt[int64_t(k) * b.batch + r] = h;
-  }
-  b.target[r] = b.label[row];
+// 512 threads: thread t works on row 32 (warp % 4) + lane of the tile (the
+// TMEM lanes its warp can read) and on the 16 hidden units 16 (warp / 4) ...
+constexpr int kFusedThreads = 512;
+constexpr int kTile = tc::kTileM;  // 128 rows
+// shared-memory operands (canonical K-major layout, element (r, k) at
+// (k / 8) * LBO + 16 r + 2 (k % 8)); the transposed operands' slices are
+// padded by 16 bytes so that a warp's 2-byte stores to them (consecutive k of
+// one r) fall into different banks
+constexpr uint32_t kLboRow = kTile * 16;     // X, H1, dZ2: 128 rows
+constexpr uint32_t kLboW = kH * 16;          // W1, W2, W2^T: 64 rows
+constexpr uint32_t kLboG = kTile * 16 + 16;  // [dZ2 | dZ1]^T: 128 rows
+constexpr int kNG = kH + kXin;               // columns of [H1 | X]
+constexpr uint32_t kLboN = kNG * 16 + 16;    // [H1 | X]^T: 80 rows
+constexpr uint32_t kOffSX = 0;
+constexpr uint32_t kOffSW1 = kOffSX + 2 * kLboRow;
+constexpr uint32_t kOffSW2 = kOffSW1 + 2 * kLboW;
+constexpr uint32_t kOffSH1 = kOffSW2 + 8 * kLboW;
+constexpr uint32_t kForwardSmem = kOffSH1 + 8 * kLboRow;
+constexpr uint32_t kOffSW2t = kForwardSmem;
+constexpr uint32_t kOffSD2 = kOffSW2t + 8 * kLboW;
+constexpr uint32_t kOffSG = kOffSD2 + 8 * kLboRow;
+constexpr uint32_t kOffSN = kOffSG + 16 * kLboG;
+constexpr uint32_t kFusedSmem = kOffSN + 16 * kLboN;
+// tensor-memory columns: Z1, Z2, dH1 (64 each), the weight gradients (80)
+constexpr uint32_t kColZ1 = 0, kColZ2 = 64, kColDh = 128, kColDw = 192;
+constexpr uint32_t kFusedCols = 512, kInferCols = 128;
+constexpr int kPartial = mlp::kParams + 1;  // a CTA's gradient sums and its loss
+constexpr int kMaxCtas = 152;
+constexpr uint32_t kPolls = 1u << 22;
+
+// One product into tensor-memory columns `col`: A (128 rows) and B of `slices`
+// 8-element K slices.  Issued by one thread.
+__device__ __forceinline__ void IssueMma(uint32_t tmem, uint32_t col, uint32_t a, uint32_t lbo_a,
+                                         uint32_t b, uint32_t lbo_b, int n, int slices,
+                                         bool accumulate, uint64_t* bar) {
+  tc::FenceAfterSync();
+  const uint32_t idesc = tc::InstrDescBf16(tc::kTileM, n);
+  for (int ks = 0; ks < slices / 2; ++ks)
+    tc::Mma(tmem + col, tc::SmemDesc(a + 2 * ks * lbo_a, lbo_a, 128),
+            tc::SmemDesc(b + 2 * ks * lbo_b, lbo_b, 128), idesc, (accumulate || ks > 0) ? 1u : 0u);
+  tc::Commit(bar);
 }
 
-// Tiles of 32 rows x 64 hidden units per 256-thread block: row-major
-// reads and writes are coalesced, the transposed copy goes through shared
-// memory so that its writes are coalesced too.
-constexpr int kTileRows = 32;
+// The CTA's MMAs and their completion barrier.  Every wait is bounded: after
+// a timeout `ok` is false (in every thread alike), the error flag is set and
+// no further product is issued.
+struct MmaPhases {
+  uint64_t* bar;
+  int* error;
+  uint32_t phase = 0;
+  bool ok = true;
+  // operands in shared memory are written, thread 0 issues `f`, all wait
+  template <class F> __device__ __forceinline__ void Run(F f) {
+    tc::FenceProxyAsync();
+    tc::FenceBeforeSync();
+    __syncthreads();
+    if (ok) {
+      if (threadIdx.x == 0) f();
+      const bool landed = tc::MbarWait(bar, phase, kPolls);
+      ok = !__syncthreads_or(landed ? 0 : 1);
+      if (!ok) {
+        if (threadIdx.x == 0 && error) atomicOr(error, 1);
+        tc::MbarWait(bar, phase, kPolls);  // a second bounded chance to drain
+      }
+      phase ^= 1u;
+    }
+    tc::FenceAfterSync();
+  }
+};
 
-// Z1 += b1, H1 = GELU(Z1) in both layouts.
-__global__ void __launch_bounds__(256) Act1Kernel(StepBuffers b, const float* blob) {
-  __shared__ __nv_bfloat16 tile[kH][kTileRows + 2];
-  const int r0 = blockIdx.x * kTileRows;
-  for (int e = threadIdx.x; e < kTileRows * kH; e += blockDim.x) {
-    const int r = e / kH, o = e % kH;
-    const int64_t i = int64_t(r0 + r) * kH + o;
-    const float z = b.Z1[i] + blob[mlp::kOffB1 + o];
-    b.Z1[i] = z;
-    const __nv_bfloat16 h = __float2bfloat16_rn(Gelu(z));
-    b.H1[i] = h;
-    tile[o][r] = h;
+__device__ __forceinline__ uint32_t Pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// 16 units of a row as two 16-byte K slices of a row-major operand.
+__device__ __forceinline__ void StoreUnits(uint8_t* op, int row, int group, const float* v) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint4 w;
+    w.x = Pack2(v[8 * h], v[8 * h + 1]);
+    w.y = Pack2(v[8 * h + 2], v[8 * h + 3]);
+    w.z = Pack2(v[8 * h + 4], v[8 * h + 5]);
+    w.w = Pack2(v[8 * h + 6], v[8 * h + 7]);
+    *reinterpret_cast<uint4*>(op + (2 * group + h) * kLboRow + row * 16) = w;
+  }
+}
+
+// 16 units of a row into the transposed operand (rows unit0.., K = row).
+__device__ __forceinline__ void StoreTransposed(uint8_t* op, uint32_t lbo, int unit0, int row,
+                                                const float* v) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    *reinterpret_cast<__nv_bfloat16*>(op + (row >> 3) * lbo + (unit0 + i) * 16 + (row & 7) * 2) =
+        __float2bfloat16_rn(v[i]);
+}
+
+// bf16 weights [64][width] (row-major) as K slices of 64 rows.
+__device__ __forceinline__ void LoadWeights(uint8_t* op, const __nv_bfloat16* w, int width) {
+  for (int c = threadIdx.x; c < kH * width / 8; c += blockDim.x) {
+    const int r = c / (width / 8), sl = c % (width / 8);
+    *reinterpret_cast<uint4*>(op + sl * kLboW + r * 16) =
+        *reinterpret_cast<const uint4*>(w + r * width + sl * 8);
+  }
+}
+
+// Standardised features of a row as its X operand (columns 5..15 zero).
+__device__ __forceinline__ void StoreFeatures(uint8_t* op, int row, const float* f,
+                                              const float* stats, float* x) {
+#pragma unroll
+  for (int k = 0; k < mlp::kIn; ++k)
+    x[k] = (f[k] - stats[mlp::kOffMean + k]) * stats[mlp::kOffInvStd + k];
+  uint4 w;
+  w.x = Pack2(x[0], x[1]);
+  w.y = Pack2(x[2], x[3]);
+  w.z = Pack2(x[4], 0.0f);
+  w.w = 0u;
+  *reinterpret_cast<uint4*>(op + row * 16) = w;
+  *reinterpret_cast<uint4*>(op + kLboRow + row * 16) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Sums over the warp's 32 lanes of 16 values each: lane l (even) ends with the
+// sum of value *index (16 shuffles instead of 80).
+__device__ __forceinline__ float SumUnits(float* v, int lane, int* index) {
+  int at = 0;
+#pragma unroll
+  for (int m = 16, n = 8; m >= 2; m >>= 1, n >>= 1) {
+    const bool up = (lane & m) != 0;
+    at += up ? n : 0;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n];
+      const float keep = up ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+    }
+  }
+  *index = at;
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+struct FusedArgs {
+  const float* feat;   // raw features [n][5]
+  const float* label;  // [n]
+  int64_t n;
+  uint64_t seed;
+  int batch;
+  int given_rows;      // 1: rows 0..batch-1 of feat (gradient check)
+  int count;           // 1: a training step (the step counter advances)
+  // step[0]: steps the sampling has seen (UpdateKernel advances it);
+  // step[1]: Adam's step number (this kernel advances it).  Neither kernel
+  // reads the counter it writes.
+  unsigned long long* step;
+  const float* blob;   // statistics, biases, output weights
+  const __nv_bfloat16* W1;
+  const __nv_bfloat16* W2;
+  const __nv_bfloat16* W2t;
+  float* partial;      // [gridDim.x][kPartial]
+  int* error;
+};
+
+__global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_base;
+  __shared__ float vec[mlp::kParams - mlp::kOffB2];  // b2, w3, b3
+  __shared__ float b1[kH], stats[2 * mlp::kIn];
+  __shared__ float ypart[4][kTile], target[kTile];
+  // per row-warp sums over the tiles: db1, db2, dw3 and (db3, loss)
+  __shared__ float sums[4][3 * kH + 2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rw = warp & 3, group = warp >> 2, row = rw * 32 + lane, u0 = group * 16;
+  if (warp == 0) tc::TmemAlloc(&tmem_base, kFusedCols);
+  if (tid == 0) {
+    tc::MbarInit(&bar, 1);
+    tma::FenceMbarInit();
+    if (a.count && blockIdx.x == 0) a.step[1] += 1;
+  }
+  LoadWeights(sm + kOffSW1, a.W1, kXin);
+  LoadWeights(sm + kOffSW2, a.W2, kH);
+  LoadWeights(sm + kOffSW2t, a.W2t, kH);
+  for (int i = tid; i < mlp::kParams - mlp::kOffB2; i += blockDim.x) vec[i] = a.blob[mlp::kOffB2 + i];
+  if (tid < kH) b1[tid] = a.blob[mlp::kOffB1 + tid];
+  if (tid < 2 * mlp::kIn) stats[tid] = a.blob[mlp::kOffMean + tid];
+  for (int i = tid; i < 4 * (3 * kH + 2); i += blockDim.x) (&sums[0][0])[i] = 0.0f;
+  tc::FenceBeforeSync();
+  __syncthreads();
+  tc::FenceAfterSync();
+  const uint32_t tmem = tmem_base;
+  const uint32_t lanes = tmem + (uint32_t(rw * 32) << 16);
+  const uint32_t base = tc::SmemAddr(sm);
+  const float* w3 = vec + (mlp::kOffW3 - mlp::kOffB2);
+  const float b3 = vec[mlp::kOffB3 - mlp::kOffB2];
+  const unsigned long long step = a.step[0];
+  MmaPhases mma{&bar, a.error};
+  const int tiles = a.batch / kTile;
+  bool first = true;
+  for (int tile = blockIdx.x; tile < tiles && mma.ok; tile += gridDim.x) {
+    if (group == 0) {
+      const int r = tile * kTile + row;
+      int64_t src = r;
+      if (!a.given_rows) {
+        const uint64_t h = Mix(a.seed ^ Mix(step * 0x100000001ull + uint64_t(r)));
+        src = int64_t(h % uint64_t(a.n));
+      }
+      float f[mlp::kIn], x[mlp::kIn];
+#pragma unroll
+      for (int k = 0; k < mlp::kIn; ++k) f[k] = a.feat[src * mlp::kIn + k];
+      target[row] = a.label[src];
+      StoreFeatures(sm + kOffSX, row, f, stats, x);
+#pragma unroll
+      for (int k = 0; k < kXin; ++k)
+        *reinterpret_cast<__nv_bfloat16*>(sm + kOffSN + (row >> 3) * kLboN + (kH + k) * 16 +
+                                          (row & 7) * 2) =
+            __float2bfloat16_rn(k < mlp::kIn ? x[k < mlp::kIn ? k : 0] : 0.0f);
+    }
+    float v[16], g1[16], d[16], gw[16];
+    mma.Run([&] {
+      IssueMma(tmem, kColZ1, base + kOffSX, kLboRow, base + kOffSW1, kLboW, kH, 2, false, &bar);
+    });
+    tc::TmemLoad16(lanes + kColZ1 + u0, v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = GeluBoth(v[i] + b1[u0 + i], &g1[i]);
+    StoreUnits(sm + kOffSH1, row, group, v);
+    StoreTransposed(sm + kOffSN, kLboN, u0, row, v);
+    mma.Run([&] {
+      IssueMma(tmem, kColZ2, base + kOffSH1, kLboRow, base + kOffSW2, kLboW, kH, 8, false, &bar);
+    });
+    tc::TmemLoad16(lanes + kColZ2 + u0, v);
+    float y = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      gw[i] = GeluBoth(v[i] + vec[u0 + i], &d[i]);
+      y = fmaf(w3[u0 + i], gw[i], y);
+    }
+    ypart[group][row] = y;
+    __syncthreads();
+    const float e =
+        (b3 + ypart[0][row] + ypart[1][row] + ypart[2][row] + ypart[3][row]) - target[row];
+    const float dy = 2.0f * e / float(a.batch);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      gw[i] = dy * gw[i];
+      d[i] = dy * w3[u0 + i] * d[i];
+    }
+    StoreUnits(sm + kOffSD2, row, group, d);
+    StoreTransposed(sm + kOffSG, kLboG, u0, row, d);
+    int at;
+    const float sd = SumUnits(d, lane, &at), sw = SumUnits(gw, lane, &at);
+    if (!(lane & 1)) {
+      sums[rw][kH + u0 + at] += sd;
+      sums[rw][2 * kH + u0 + at] += sw;
+    }
+    if (group == 0) {
+      float g3 = dy, e2 = e * e;
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) {
+        g3 += __shfl_xor_sync(0xffffffffu, g3, m);
+        e2 += __shfl_xor_sync(0xffffffffu, e2, m);
+      }
+      if (lane == 0) {
+        sums[rw][3 * kH] += g3;
+        sums[rw][3 * kH + 1] += e2;
+      }
+    }
+    mma.Run([&] {
+      IssueMma(tmem, kColDh, base + kOffSD2, kLboRow, base + kOffSW2t, kLboW, kH, 8, false, &bar);
+    });
+    tc::TmemLoad16(lanes + kColDh + u0, v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] *= g1[i];
+    StoreTransposed(sm + kOffSG, kLboG, kH + u0, row, v);
+    const float s1 = SumUnits(v, lane, &at);
+    if (!(lane & 1)) sums[rw][u0 + at] += s1;
+    mma.Run([&] {
+      IssueMma(tmem, kColDw, base + kOffSG, kLboG, base + kOffSN, kLboN, kNG, 16, !first, &bar);
+    });
+    first = false;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < kTileRows * kH; e += blockDim.x) {
-    const int o = e / kTileRows, r = e % kTileRows;
-    b.H1t[int64_t(o) * b.batch + r0 + r] = tile[o][r];
-  }
-}
-
-// Output layer, loss, and the backward pass down to dZ2 (one thread per row;
-// dw3, db2, db3 and the loss are reduced over the warp's 32 rows first).
-__global__ void OutKernel(StepBuffers b, const float* blob, float* grad) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = r < b.batch;
-  const int64_t row = int64_t(active ? r : 0) * kH;
-  float y = blob[mlp::kOffB3];
-  if (active) {
-#pragma unroll 8
-    for (int o = 0; o < kH; ++o) {
-      const float z = b.Z2[row + o] + blob[mlp::kOffB2 + o];
-      b.Z2[row + o] = z;
-      y = fmaf(blob[mlp::kOffW3 + o], Gelu(z), y);
+  float* out = a.partial + int64_t(blockIdx.x) * kPartial;
+  if (mma.ok && !first) {
+    // rows 0..63: dW2 [out][in]; rows 64..127, columns 64..68: dW1
+    if (rw < 2) {
+      float v[16];
+      tc::TmemLoad16(lanes + kColDw + u0, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) out[mlp::kOffW2 + row * kH + u0 + i] = v[i];
+    } else if (group == 0) {
+      float v[16];
+      tc::TmemLoad16(lanes + kColDw + kH, v);
+#pragma unroll
+      for (int k = 0; k < mlp::kIn; ++k) out[mlp::kOffW1 + (row - kH) * mlp::kIn + k] = v[k];
     }
   }
-  const float e = active ? y - b.target[r] : 0.0f;
-  const float dy = 2.0f * e / float(b.batch);
-  float e2 = e * e, g3 = dy;
-  for (int s = 16; s > 0; s >>= 1) {
-    e2 += __shfl_xor_sync(0xffffffffu, e2, s);
-    g3 += __shfl_xor_sync(0xffffffffu, g3, s);
+  if (tid < 3 * kH + 2) {
+    const float t = ((sums[0][tid] + sums[1][tid]) + sums[2][tid]) + sums[3][tid];
+    const int k = tid % kH;
+    const int at = tid < kH ? mlp::kOffB1 + k
+                 : tid < 2 * kH ? mlp::kOffB2 + k
+                 : tid < 3 * kH ? mlp::kOffW3 + k
+                 : tid == 3 * kH ? mlp::kOffB3
+                                 : mlp::kParams;
+    out[at] = t;
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(b.loss, e2);
-    atomicAdd(grad + mlp::kOffB3, g3);
-  }
-#pragma unroll 4
-  for (int o = 0; o < kH; ++o) {
-    float gw = 0.0f, d2 = 0.0f;
-    if (active) {
-      const float z = b.Z2[row + o];
-      gw = dy * Gelu(z);
-      d2 = dy * blob[mlp::kOffW3 + o] * GeluGrad(z);
-      const __nv_bfloat16 h = __float2bfloat16_rn(d2);
-      b.D2[row + o] = h;
-      b.D2t[int64_t(o) * b.batch + r] = h;
-    }
-    for (int s = 16; s > 0; s >>= 1) {
-      gw += __shfl_xor_sync(0xffffffffu, gw, s);
-      d2 += __shfl_xor_sync(0xffffffffu, d2, s);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(grad + mlp::kOffW3 + o, gw);
-      atomicAdd(grad + mlp::kOffB2 + o, d2);
-    }
-  }
-}
-
-// dZ1 = dH1 * GELU'(Z1) (transposed, bf16) and db1, per 32-row tile.
-__global__ void __launch_bounds__(256) Back1Kernel(StepBuffers b, float* grad) {
-  __shared__ float tile[kH][kTileRows + 1];
-  const int r0 = blockIdx.x * kTileRows;
-  for (int e = threadIdx.x; e < kTileRows * kH; e += blockDim.x) {
-    const int r = e / kH, o = e % kH;
-    const int64_t i = int64_t(r0 + r) * kH + o;
-    tile[o][r] = b.dH1[i] * GeluGrad(b.Z1[i]);
-  }
+  if (tid < mlp::kOffW1) out[tid] = 0.0f;
+  tc::FenceBeforeSync();
   __syncthreads();
-  for (int e = threadIdx.x; e < kTileRows * kH; e += blockDim.x) {
-    const int o = e / kTileRows, r = e % kTileRows;
-    const float d1 = tile[o][r];
-    b.D1t[int64_t(o) * b.batch + r0 + r] = __float2bfloat16_rn(d1);
-    // the 32 lanes of a warp hold the 32 rows of one hidden unit
-    float v = d1;
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    if ((threadIdx.x & 31) == 0) atomicAdd(grad + mlp::kOffB1 + o, v);
+  if (warp == 0) tc::TmemDealloc(tmem, kFusedCols);
+}
+
+// The gradient (the CTAs' partial sums added in a fixed order), and with
+// `update` Adam (lr, beta1 0.9, beta2 0.999, eps 1e-8) and the published
+// weights.  Blocks of 32 parameters x 8 parts of the CTAs.
+__global__ void __launch_bounds__(256)
+    UpdateKernel(Net net, const float* partial, int ctas, int update, float lr,
+                 unsigned long long* step, float* loss) {
+  __shared__ float part[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + x;
+  float s = 0.0f;
+  if (i < kPartial)
+    for (int c = y; c < ctas; c += 8) s += partial[int64_t(c) * kPartial + i];
+  part[y][x] = s;
+  __syncthreads();
+  if (y != 0 || i >= kPartial) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) s += part[k][x];
+  if (i == mlp::kParams) {
+    *loss += s;
+    if (update) step[0] += 1;
+    return;
   }
+  net.grad[i] = s;
+  if (!update || i < mlp::kOffW1) return;
+  const unsigned long long t = step[1];
+  const float m = 0.9f * net.m1[i] + 0.1f * s;
+  const float v = 0.999f * net.m2[i] + 0.001f * s * s;
+  net.m1[i] = m;
+  net.m2[i] = v;
+  const float mh = m / (1.0f - powf(0.9f, float(t)));
+  const float vh = v / (1.0f - powf(0.999f, float(t)));
+  const float w = net.master[i] - lr * mh / (sqrtf(vh) + 1e-8f);
+  net.master[i] = w;
+  PublishOne(net, i, w);
 }
 
-// Gather the weight gradients from the GEMM outputs into the blob layout.
-__global__ void CollectKernel(StepBuffers b, float* grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < kH * mlp::kIn) {
-    const int o = i / mlp::kIn, k = i % mlp::kIn;
-    grad[mlp::kOffW1 + i] = b.dW1[o * kXin + k];
+// Inference: the forward half of FusedStepKernel over tiles of 128 rows.
+__global__ void __launch_bounds__(kFusedThreads)
+    InferKernel(int64_t n, const float* feat, const float* blob, const __nv_bfloat16* W1,
+                const __nv_bfloat16* W2, float* y_out, int* error) {
+  extern __shared__ __align__(128) uint8_t sm[];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_base;
+  __shared__ float vec[mlp::kParams - mlp::kOffB2];
+  __shared__ float b1[kH], stats[2 * mlp::kIn];
+  __shared__ float ypart[4][kTile];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rw = warp & 3, group = warp >> 2, row = rw * 32 + lane, u0 = group * 16;
+  if (warp == 0) tc::TmemAlloc(&tmem_base, kInferCols);
+  if (tid == 0) {
+    tc::MbarInit(&bar, 1);
+    tma::FenceMbarInit();
   }
-  if (i < kH * kH) grad[mlp::kOffW2 + i] = b.dW2[i];
-}
-
-// Adam (lr, beta1 0.9, beta2 0.999, eps 1e-8) on the weights and biases.
-__global__ void AdamKernel(Net net, float lr, unsigned long long* step) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned long long t = *step + 1;
-  if (i >= mlp::kOffW1 && i < mlp::kParams) {
-    const float g = net.grad[i];
-    const float m = 0.9f * net.m1[i] + 0.1f * g;
-    const float v = 0.999f * net.m2[i] + 0.001f * g * g;
-    net.m1[i] = m;
-    net.m2[i] = v;
-    const float mh = m / (1.0f - powf(0.9f, float(t)));
-    const float vh = v / (1.0f - powf(0.999f, float(t)));
-    net.master[i] -= lr * mh / (sqrtf(vh) + 1e-8f);
+  LoadWeights(sm + kOffSW1, W1, kXin);
+  LoadWeights(sm + kOffSW2, W2, kH);
+  for (int i = tid; i < mlp::kParams - mlp::kOffB2; i += blockDim.x) vec[i] = blob[mlp::kOffB2 + i];
+  if (tid < kH) b1[tid] = blob[mlp::kOffB1 + tid];
+  if (tid < 2 * mlp::kIn) stats[tid] = blob[mlp::kOffMean + tid];
+  tc::FenceBeforeSync();
+  __syncthreads();
+  tc::FenceAfterSync();
+  const uint32_t tmem = tmem_base;
+  const uint32_t lanes = tmem + (uint32_t(rw * 32) << 16);
+  const uint32_t base = tc::SmemAddr(sm);
+  const float* w3 = vec + (mlp::kOffW3 - mlp::kOffB2);
+  MmaPhases mma{&bar, error};
+  const int64_t tiles = (n + kTile - 1) / kTile;
+  for (int64_t tile = blockIdx.x; tile < tiles && mma.ok; tile += gridDim.x) {
+    const int64_t r = tile * kTile + row;
+    if (group == 0) {
+      const int64_t src = r < n ? r : n - 1;
+      float f[mlp::kIn], x[mlp::kIn];
+#pragma unroll
+      for (int k = 0; k < mlp::kIn; ++k) f[k] = feat[src * mlp::kIn + k];
+      StoreFeatures(sm + kOffSX, row, f, stats, x);
+    }
+    float v[16], unused;
+    mma.Run([&] {
+      IssueMma(tmem, kColZ1, base + kOffSX, kLboRow, base + kOffSW1, kLboW, kH, 2, false, &bar);
+    });
+    tc::TmemLoad16(lanes + kColZ1 + u0, v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = GeluBoth(v[i] + b1[u0 + i], &unused);
+    StoreUnits(sm + kOffSH1, row, group, v);
+    mma.Run([&] {
+      IssueMma(tmem, kColZ2, base + kOffSH1, kLboRow, base + kOffSW2, kLboW, kH, 8, false, &bar);
+    });
+    tc::TmemLoad16(lanes + kColZ2 + u0, v);
+    float y = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) y = fmaf(w3[u0 + i], GeluBoth(v[i] + vec[u0 + i], &unused), y);
+    ypart[group][row] = y;
+    __syncthreads();
+    if (group == 0 && r < n && mma.ok)
+      y_out[r] = vec[mlp::kOffB3 - mlp::kOffB2] + ypart[0][row] + ypart[1][row] + ypart[2][row] +
+                 ypart[3][row];
   }
-}
-
-__global__ void StepCountKernel(unsigned long long* step) { *step += 1; }
-
-// Inference rows: standardised features -> X (bf16 [n][16]).
-__global__ void InferGatherKernel(int64_t n, const float* feat, const float* stats,
-                                  __nv_bfloat16* X) {
-  const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  for (int k = 0; k < kXin; ++k) {
-    float v = 0.0f;
-    if (k < mlp::kIn) v = (feat[r * mlp::kIn + k] - stats[mlp::kOffMean + k]) * stats[mlp::kOffInvStd + k];
-    X[r * kXin + k] = __float2bfloat16_rn(v);
-  }
-}
-
-__global__ void InferAct1Kernel(int64_t n, const float* Z1, const float* blob, __nv_bfloat16* H1) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n * kH) return;
-  const int o = static_cast<int>(i % kH);
-  H1[i] = __float2bfloat16_rn(Gelu(Z1[i] + blob[mlp::kOffB1 + o]));
-}
-
-__global__ void InferOutKernel(int64_t n, const float* Z2, const float* blob, float* y) {
-  const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  float acc = blob[mlp::kOffB3];
-  for (int o = 0; o < kH; ++o) acc = fmaf(blob[mlp::kOffW3 + o], Gelu(Z2[r * kH + o] + blob[mlp::kOffB2 + o]), acc);
-  y[r] = acc;
+  tc::FenceBeforeSync();
+  __syncthreads();
+  if (warp == 0) tc::TmemDealloc(tmem, kInferCols);
 }
 
 }  // namespace mlpk
@@ -490,25 +718,14 @@ struct fvs_mlp {
   float* buf = nullptr;  // master, m1, m2, grad, blob
   __nv_bfloat16* wbuf = nullptr;
   int* error = nullptr;
-  unsigned long long* step = nullptr;
+  unsigned long long* step = nullptr;  // [2], see FusedArgs::step
   cudaStream_t stream = nullptr;
-  // training scratch (sized for `batch`)
-  int batch = 0;
-  std::vector<void*> scratch;
-  StepBuffers sb{};
-  cudaGraphExec_t graph = nullptr;
-  const float* graph_feat = nullptr;
-  const float* graph_label = nullptr;
-  int64_t graph_n = 0;
-  float graph_lr = 0.f;
-  uint64_t graph_seed = 0;
-  // inference scratch
-  int64_t infer_cap = 0;
-  void* infer_buf = nullptr;
+  float* partial = nullptr;  // [kMaxCtas][kPartial]
+  float* loss = nullptr;     // sum of squared errors of the steps since its reset
+  int ctas = 1;              // CTAs of the fused kernels (one per SM)
   ~fvs_mlp() {
-    if (graph) cudaGraphExecDestroy(graph);
-    for (void* p : scratch) cudaFree(p);
-    if (infer_buf) cudaFree(infer_buf);
+    if (partial) cudaFree(partial);
+    if (loss) cudaFree(loss);
     if (buf) cudaFree(buf);
     if (wbuf) cudaFree(wbuf);
     if (error) cudaFree(error);
@@ -535,89 +752,30 @@ int MlpCuda(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return MlpCuda(e_, #call);   \
   } while (0)
 
-cudaError_t Alloc(fvs_mlp* m, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaSuccess) {
-    m->scratch.push_back(*p);
-    e = cudaMemset(*p, 0, bytes);
-  }
+// The fused kernels' dynamic shared memory, set once per handle.
+cudaError_t SetSmem() {
+  cudaError_t e = cudaFuncSetAttribute(
+      FusedStepKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFusedSmem));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(InferKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(kForwardSmem));
   return e;
 }
 
-int EnsureBatch(fvs_mlp* m, int batch) {
-  if (m->batch == batch) return FVS_OK;
-  if (m->graph) {
-    cudaGraphExecDestroy(m->graph);
-    m->graph = nullptr;
-  }
-  for (void* p : m->scratch) cudaFree(p);
-  m->scratch.clear();
-  StepBuffers& b = m->sb;
-  b = StepBuffers{};
-  b.batch = batch;
-  const size_t B = size_t(batch);
-  MLP_CUDA(Alloc(m, (void**)&b.X, B * kXin * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.Xt, B * kXin * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.target, B * 4));
-  MLP_CUDA(Alloc(m, (void**)&b.Z1, B * kH * 4));
-  MLP_CUDA(Alloc(m, (void**)&b.H1, B * kH * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.H1t, B * kH * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.Z2, B * kH * 4));
-  MLP_CUDA(Alloc(m, (void**)&b.D2, B * kH * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.D2t, B * kH * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.dH1, B * kH * 4));
-  MLP_CUDA(Alloc(m, (void**)&b.D1t, B * kH * 2));
-  MLP_CUDA(Alloc(m, (void**)&b.dW2, 128 * kH * 4));
-  MLP_CUDA(Alloc(m, (void**)&b.dW1, 128 * kXin * 4));
-  MLP_CUDA(Alloc(m, (void**)&b.loss, 4));
-  b.step = m->step;
-  m->batch = batch;
-  return FVS_OK;
-}
-
-// One training step (forward, backward, and optionally Adam) on the stream.
-cudaError_t EnqueueStep(fvs_mlp* m, bool update, float lr) {
-  StepBuffers& b = m->sb;
-  cudaStream_t s = m->stream;
-  const Net& net = m->net;
-  const int B = b.batch;
-  cudaError_t e = cudaMemsetAsync(net.grad, 0, sizeof(float) * fvs::mlp::kParams, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.dW2, 0, 128 * kH * 4, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.dW1, 0, 128 * kXin * 4, s);
-  if (e != cudaSuccess) return e;
-  GatherKernel<<<(B + 127) / 128, 128, 0, s>>>(b, net.blob);
-  GemmArgs g{};
-  g.error = m->error;
-  // Z1 = X W1^T
-  g.A = b.X; g.lda = kXin; g.B = net.W1; g.ldb = kXin; g.C = b.Z1; g.ldc = kH;
-  g.M = B; g.K = kXin; g.k_per_cta = kXin; g.atomic = 0;
-  if ((e = LaunchGemm<64>(g, 1, s)) != cudaSuccess) return e;
-  Act1Kernel<<<B / kTileRows, 256, 0, s>>>(b, net.blob);
-  // Z2 = H1 W2^T
-  g.A = b.H1; g.lda = kH; g.B = net.W2; g.ldb = kH; g.C = b.Z2; g.ldc = kH;
-  g.M = B; g.K = kH; g.k_per_cta = kH; g.atomic = 0;
-  if ((e = LaunchGemm<64>(g, 1, s)) != cudaSuccess) return e;
-  OutKernel<<<(B + 127) / 128, 128, 0, s>>>(b, net.blob, net.grad);
-  // dH1 = dZ2 W2  (B operand W2^T: [in][out])
-  g.A = b.D2; g.lda = kH; g.B = net.W2t; g.ldb = kH; g.C = b.dH1; g.ldc = kH;
-  g.M = B; g.K = kH; g.k_per_cta = kH; g.atomic = 0;
-  if ((e = LaunchGemm<64>(g, 1, s)) != cudaSuccess) return e;
-  // dW2 = dZ2^T H1 over the batch (split K)
-  const int kper = 256;
-  g.A = b.D2t; g.lda = B; g.B = b.H1t; g.ldb = B; g.C = b.dW2; g.ldc = kH;
-  g.M = kH; g.K = B; g.k_per_cta = kper; g.atomic = 1;
-  if ((e = LaunchGemm<64>(g, (B + kper - 1) / kper, s)) != cudaSuccess) return e;
-  Back1Kernel<<<B / kTileRows, 256, 0, s>>>(b, net.grad);
-  // dW1 = dZ1^T X
-  g.A = b.D1t; g.lda = B; g.B = b.Xt; g.ldb = B; g.C = b.dW1; g.ldc = kXin;
-  g.M = kH; g.K = B; g.k_per_cta = kper; g.atomic = 1;
-  if ((e = LaunchGemm<16>(g, (B + kper - 1) / kper, s)) != cudaSuccess) return e;
-  CollectKernel<<<(kH * kH + 255) / 256, 256, 0, s>>>(b, net.grad);
-  if (update) {
-    AdamKernel<<<(fvs::mlp::kParams + 255) / 256, 256, 0, s>>>(net, lr, b.step);
-    PublishKernel<<<(fvs::mlp::kParams + 255) / 256, 256, 0, s>>>(net);
-    StepCountKernel<<<1, 1, 0, s>>>(b.step);
-  }
+// One training step (update) or one gradient of the given rows on the stream.
+cudaError_t EnqueueStep(fvs_mlp* m, FusedArgs a, bool update, float lr) {
+  a.step = m->step;
+  a.blob = m->net.blob;
+  a.W1 = m->net.W1;
+  a.W2 = m->net.W2;
+  a.W2t = m->net.W2t;
+  a.partial = m->partial;
+  a.error = m->error;
+  a.count = update ? 1 : 0;
+  const int grid = std::min(a.batch / kTile, m->ctas);
+  FusedStepKernel<<<grid, kFusedThreads, kFusedSmem, m->stream>>>(a);
+  UpdateKernel<<<(kPartial + 31) / 32, 256, 0, m->stream>>>(m->net, m->partial, grid,
+                                                            update ? 1 : 0, lr, m->step, m->loss);
   return cudaGetLastError();
 }
 
@@ -689,11 +847,18 @@ int fvs_mlp_create(uint64_t seed, fvs_mlp** out) {
   if (e == cudaSuccess) e = cudaMalloc(&m->buf, sizeof(float) * P * 5);
   if (e == cudaSuccess) e = cudaMalloc(&m->wbuf, sizeof(__nv_bfloat16) * (64 * 16 + 2 * 64 * 64));
   if (e == cudaSuccess) e = cudaMalloc(&m->error, sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&m->step, sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&m->step, 2 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&m->partial, sizeof(float) * kMaxCtas * kPartial);
+  if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(float));
+  if (e == cudaSuccess) e = SetSmem();
+  int dev = 0, sms = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  m->ctas = std::max(1, std::min(sms, kMaxCtas));
   if (e == cudaSuccess) e = cudaMemset(m->buf, 0, sizeof(float) * P * 5);
   if (e == cudaSuccess) e = cudaMemset(m->wbuf, 0, sizeof(__nv_bfloat16) * (64 * 16 + 2 * 64 * 64));
   if (e == cudaSuccess) e = cudaMemset(m->error, 0, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(m->step, 0, sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMemset(m->step, 0, 2 * sizeof(unsigned long long));
   if (e != cudaSuccess) {
     delete m;
     return MlpCuda(e, "fvs_mlp_create");
@@ -784,37 +949,17 @@ int fvs_mlp_train(fvs_mlp* m, const float* features_dev, const float* labels_dev
     return MlpFail(FVS_ERR_INVALID, "bad arguments");
   if (batch < 128 || batch % 256 != 0 || batch > (1 << 20))
     return MlpFail(FVS_ERR_INVALID, "batch must be a multiple of 256 in [256, 2^20]");
-  if (int r = EnsureBatch(m, batch)) return r;
-  StepBuffers& b = m->sb;
-  b.feat = features_dev;
-  b.label = labels_dev;
-  b.n = n;
-  b.seed = seed;
-  b.use_given_rows = 0;
-  if (!m->graph || m->graph_feat != features_dev || m->graph_label != labels_dev ||
-      m->graph_n != n || m->graph_lr != lr || m->graph_seed != seed) {
-    if (m->graph) cudaGraphExecDestroy(m->graph);
-    m->graph = nullptr;
-    cudaGraph_t g;
-    MLP_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = EnqueueStep(m, true, lr);
-    cudaError_t e2 = cudaStreamEndCapture(m->stream, &g);
-    if (e != cudaSuccess) return MlpCuda(e, "capture training step");
-    if (e2 != cudaSuccess) return MlpCuda(e2, "end capture");
-    e = cudaGraphInstantiate(&m->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return MlpCuda(e, "instantiate training graph");
-    m->graph_feat = features_dev;
-    m->graph_label = labels_dev;
-    m->graph_n = n;
-    m->graph_lr = lr;
-    m->graph_seed = seed;
-  }
-  MLP_CUDA(cudaMemsetAsync(b.loss, 0, sizeof(float), m->stream));
-  for (int i = 0; i < steps; ++i) MLP_CUDA(cudaGraphLaunch(m->graph, m->stream));
+  FusedArgs a{};
+  a.feat = features_dev;
+  a.label = labels_dev;
+  a.n = n;
+  a.seed = seed;
+  a.batch = batch;
+  MLP_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
+  for (int i = 0; i < steps; ++i) MLP_CUDA(EnqueueStep(m, a, true, lr));
   float loss = 0.f;
   int err = 0;
-  MLP_CUDA(cudaMemcpyAsync(&loss, b.loss, sizeof loss, cudaMemcpyDeviceToHost, m->stream));
+  MLP_CUDA(cudaMemcpyAsync(&loss, m->loss, sizeof loss, cudaMemcpyDeviceToHost, m->stream));
   MLP_CUDA(cudaMemcpyAsync(&err, m->error, sizeof err, cudaMemcpyDeviceToHost, m->stream));
   MLP_CUDA(cudaStreamSynchronize(m->stream));
   if (err) return MlpFail(FVS_ERR_CUDA, "tensor-core wait timed out");
@@ -827,19 +972,19 @@ int fvs_mlp_gradients(fvs_mlp* m, const float* features_dev, const float* labels
   if (!m || !features_dev || !labels_dev || !grads_host)
     return MlpFail(FVS_ERR_INVALID, "bad arguments");
   if (batch < 128 || batch % 256 != 0) return MlpFail(FVS_ERR_INVALID, "batch multiple of 256");
-  if (int r = EnsureBatch(m, batch)) return r;
-  StepBuffers& b = m->sb;
-  b.feat = features_dev;
-  b.label = labels_dev;
-  b.n = batch;
-  b.use_given_rows = 1;
-  MLP_CUDA(cudaMemsetAsync(b.loss, 0, sizeof(float), m->stream));
-  MLP_CUDA(EnqueueStep(m, false, 0.f));
+  FusedArgs a{};
+  a.feat = features_dev;
+  a.label = labels_dev;
+  a.n = batch;
+  a.batch = batch;
+  a.given_rows = 1;
+  MLP_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
+  MLP_CUDA(EnqueueStep(m, a, false, 0.f));
   int err = 0;
   MLP_CUDA(cudaMemcpyAsync(grads_host, m->net.grad, sizeof(float) * fvs::mlp::kParams,
                            cudaMemcpyDeviceToHost, m->stream));
   float loss = 0.f;
-  MLP_CUDA(cudaMemcpyAsync(&loss, b.loss, sizeof loss, cudaMemcpyDeviceToHost, m->stream));
+  MLP_CUDA(cudaMemcpyAsync(&loss, m->loss, sizeof loss, cudaMemcpyDeviceToHost, m->stream));
   MLP_CUDA(cudaMemcpyAsync(&err, m->error, sizeof err, cudaMemcpyDeviceToHost, m->stream));
   MLP_CUDA(cudaStreamSynchronize(m->stream));
   if (err) return MlpFail(FVS_ERR_CUDA, "tensor-core wait timed out");
@@ -850,32 +995,12 @@ int fvs_mlp_gradients(fvs_mlp* m, const float* features_dev, const float* labels
 int fvs_mlp_predict(fvs_mlp* m, const float* features_dev, int64_t n, float* y_dev) {
   if (!m || !features_dev || !y_dev || n < 0) return MlpFail(FVS_ERR_INVALID, "bad arguments");
   if (n == 0) return FVS_OK;
-  const int64_t npad = (n + 127) / 128 * 128;
-  if (npad > m->infer_cap) {
-    if (m->infer_buf) cudaFree(m->infer_buf);
-    m->infer_buf = nullptr;
-    const size_t bytes = size_t(npad) * (kXin * 2 + kH * 4 * 2 + kH * 2);
-    MLP_CUDA(cudaMalloc(&m->infer_buf, bytes));
-    MLP_CUDA(cudaMemset(m->infer_buf, 0, bytes));
-    m->infer_cap = npad;
-  }
-  uint8_t* p = static_cast<uint8_t*>(m->infer_buf);
-  __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(p);
-  float* Z1 = reinterpret_cast<float*>(p + size_t(m->infer_cap) * kXin * 2);
-  float* Z2 = Z1 + size_t(m->infer_cap) * kH;
-  __nv_bfloat16* H1 = reinterpret_cast<__nv_bfloat16*>(Z2 + size_t(m->infer_cap) * kH);
   cudaStream_t s = m->stream;
-  InferGatherKernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(n, features_dev, m->net.blob, X);
-  GemmArgs g{};
-  g.error = m->error;
-  g.A = X; g.lda = kXin; g.B = m->net.W1; g.ldb = kXin; g.C = Z1; g.ldc = kH;
-  g.M = int(n); g.K = kXin; g.k_per_cta = kXin; g.atomic = 0;
-  MLP_CUDA(LaunchGemm<64>(g, 1, s));
-  InferAct1Kernel<<<unsigned((n * kH + 255) / 256), 256, 0, s>>>(n, Z1, m->net.blob, H1);
-  g.A = H1; g.lda = kH; g.B = m->net.W2; g.ldb = kH; g.C = Z2; g.ldc = kH;
-  g.M = int(n); g.K = kH; g.k_per_cta = kH; g.atomic = 0;
-  MLP_CUDA(LaunchGemm<64>(g, 1, s));
-  InferOutKernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(n, Z2, m->net.blob, y_dev);
+  // two CTAs fit an SM's shared memory several times over; their phases overlap
+  const int64_t grid = std::min<int64_t>((n + kTile - 1) / kTile, int64_t(m->ctas) * 3);
+  InferKernel<<<unsigned(grid), kFusedThreads, kForwardSmem, s>>>(
+      n, features_dev, m->net.blob, m->net.W1, m->net.W2, y_dev, m->error);
+  MLP_CUDA(cudaGetLastError());
   int err = 0;
   MLP_CUDA(cudaMemcpyAsync(&err, m->error, sizeof err, cudaMemcpyDeviceToHost, s));
   MLP_CUDA(cudaStreamSynchronize(s));
