@@ -46,11 +46,12 @@ struct Options {
 // Quotients and square roots of the solver's variable operands on the integer
 // pipes (fvs_ieee64.cuh, nearly rounded: within 0.57 and 0.75 ulp), since the
 // FP64 pipe bounds the solver; zero, negative and non-finite operands keep
-// IEEE semantics (inf, NaN).
-__device__ __forceinline__ double Div(double a, double b) {
+// IEEE semantics (inf, NaN).  Out of line: the solver has dozens of them on
+// divergent branches.
+static __device__ __noinline__ double Div(double a, double b) {
   return ieee64::Div<false, true>(a, ieee64::MakeDivisor(b));
 }
-__device__ __forceinline__ double Sqrt(double a) { return ieee64::Sqrt<true>(a); }
+static __device__ __noinline__ double Sqrt(double a) { return ieee64::Sqrt<true>(a); }
 
 // PerfectGas::CompleteFromCons and Flux (src/equations/PerfectGas.cpp:52-124)
 // with the quotients and square root above: the Godunov sweeps' cell states
