@@ -97,6 +97,8 @@ struct fvs_amr {
   std::vector<std::vector<int>> level_patch_order;
   double* reg = nullptr;
   int32_t nslots = 0;
+  PatchCopy* patch_copy = nullptr;  // the patches' flat and storage places
+  int64_t flat_values = 0;          // values of the flat host array
   float* signs = nullptr;
   AmrControl* ctrl = nullptr;
   AmrControl* ctrl_host = nullptr;
@@ -456,6 +458,20 @@ int Build(fvs_amr* a) {
       }
     }
   }
+  std::vector<PatchCopy> copies;
+  for (size_t p = 0; p < a->patches.size(); ++p) {
+    const PatchHost& P = a->patches[p];
+    PatchCopy c{};
+    c.flat = a->flat_values;
+    c.first = a->SI(int(p), P.lo[0], P.lo[1]);
+    c.level = P.level;
+    c.nx = P.n[0];
+    c.ny = P.n[1];
+    c.pitch = P.pitch;
+    copies.push_back(c);
+    a->flat_values += int64_t(kComp) * P.n[0] * P.n[1];
+  }
+  AMR_CUDA(a->Upload(&a->patch_copy, copies));
   AMR_CUDA(a->Alloc(&a->reg, size_t(std::max(a->nslots, 1)) * 3 * kComp));
   AMR_CUDA(a->Upload(&a->signs, signs_h));
   AMR_CUDA(a->Alloc(&a->ctrl, 1));
@@ -531,20 +547,14 @@ cudaError_t LaunchMaxSpeed(fvs_amr* a, int l, int d) {
     s.coarse = a->L[size_t(l - 1)].A;
     s.coarse_ncells = int32_t(a->L[size_t(l - 1)].ncells);
   }
-  s.segs = Lv.segs[d][kSplits - 1];  // rows in 8 segments
-  s.nsegs = Lv.nsegs[d][kSplits - 1];
+  s.segs = Lv.segs[d][0];
+  s.slot_row = Lv.slot_row[d];
+  s.row_slot0 = Lv.row_slot0[d];
+  s.nslots = Lv.nslots[d];
   s.gamma = a->m.gamma;
   s.smax_out = &a->ctrl->smax_stable[l][d];
   const int block = 128;
-  int64_t threads = s.nsegs;
-  if (a->m.precision != FVS_MIXED) {  // one face per lane
-    s.segs = Lv.segs[d][0];
-    s.nsegs = Lv.nsegs[d][0];
-    s.slot_row = Lv.slot_row[d];
-    s.row_slot0 = Lv.row_slot0[d];
-    s.nslots = Lv.nslots[d];
-    threads = (s.nslots - 1 + kLaneFaces - 1) / kLaneFaces * 32;
-  }
+  const int64_t threads = (s.nslots - 1 + kLaneFaces - 1) / kLaneFaces * 32;
   const int grid = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>((threads + block - 1) / block, int64_t(a->sms) * 16)));
   switch (a->m.precision) {
@@ -555,6 +565,15 @@ cudaError_t LaunchMaxSpeed(fvs_amr* a, int l, int d) {
   default:
     return LaunchPatchMaxSpeedMixed(d, s, grid, block, a->stream);
   }
+}
+
+LevelArrays Arrays(const fvs_amr* a) {
+  LevelArrays r{};
+  for (int l = 0; l < a->nlevels; ++l) {
+    r.state[l] = a->L[size_t(l)].A;
+    r.ncells[l] = a->L[size_t(l)].ncells;
+  }
+  return r;
 }
 
 LevelDx Dx(const fvs_amr* a) {
@@ -730,24 +749,21 @@ int fvs_amr_destroy(fvs_amr* a) {
   return FVS_OK;
 }
 
+// The interiors between the caller's flat array and the levels go through a
+// device copy of the flat array and one kernel (the host used to index every
+// value: 5 ms of a 0.6 M-cell upload and download).  The ghost storage of the
+// levels stays as it is (zero: no sweep reads or writes it).
 int fvs_amr_upload(fvs_amr* a, const double* host) {
   if (!a || !host) return Fail(FVS_ERR_INVALID, "NULL argument");
-  std::vector<std::vector<double>> lv(static_cast<size_t>(a->nlevels));
-  for (int l = 0; l < a->nlevels; ++l)
-    lv[size_t(l)].assign(size_t(a->L[size_t(l)].ncells) * kComp, 0.0);
-  size_t off = 0;
-  for (size_t p = 0; p < a->patches.size(); ++p) {
-    const PatchHost& P = a->patches[p];
-    const int64_t N = a->L[size_t(P.level)].ncells;
-    std::vector<double>& v = lv[size_t(P.level)];
-    for (int c = 0; c < kComp; ++c)
-      for (int j = 0; j < P.n[1]; ++j)
-        for (int i = 0; i < P.n[0]; ++i)
-          v[size_t(c * N + a->SI(int(p), P.lo[0] + i, P.lo[1] + j))] = host[off++];
-  }
-  for (int l = 0; l < a->nlevels; ++l)
-    AMR_CUDA(cudaMemcpy(a->L[size_t(l)].A, lv[size_t(l)].data(),
-                        lv[size_t(l)].size() * sizeof(double), cudaMemcpyHostToDevice));
+  const size_t bytes = size_t(a->flat_values) * sizeof(double);
+  double* flat = nullptr;
+  AMR_CUDA(cudaMallocAsync(&flat, std::max<size_t>(bytes, 8), a->stream));
+  cudaError_t e = cudaMemcpyAsync(flat, host, bytes, cudaMemcpyHostToDevice, a->stream);
+  if (e == cudaSuccess)
+    e = LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), flat, true, a->stream);
+  cudaFreeAsync(flat, a->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
+  if (e != cudaSuccess) return CudaFail(e, "fvs_amr_upload");
   a->t = 0.0;
   a->cycle = 0;
   return FVS_OK;
@@ -755,23 +771,16 @@ int fvs_amr_upload(fvs_amr* a, const double* host) {
 
 int fvs_amr_download(fvs_amr* a, double* host) {
   if (!a || !host) return Fail(FVS_ERR_INVALID, "NULL argument");
-  AMR_CUDA(cudaStreamSynchronize(a->stream));
-  std::vector<std::vector<double>> lv(static_cast<size_t>(a->nlevels));
-  for (int l = 0; l < a->nlevels; ++l) {
-    lv[size_t(l)].resize(size_t(a->L[size_t(l)].ncells) * kComp);
-    AMR_CUDA(cudaMemcpy(lv[size_t(l)].data(), a->L[size_t(l)].A,
-                        lv[size_t(l)].size() * sizeof(double), cudaMemcpyDeviceToHost));
-  }
-  size_t off = 0;
-  for (size_t p = 0; p < a->patches.size(); ++p) {
-    const PatchHost& P = a->patches[p];
-    const int64_t N = a->L[size_t(P.level)].ncells;
-    const std::vector<double>& v = lv[size_t(P.level)];
-    for (int c = 0; c < kComp; ++c)
-      for (int j = 0; j < P.n[1]; ++j)
-        for (int i = 0; i < P.n[0]; ++i)
-          host[off++] = v[size_t(c * N + a->SI(int(p), P.lo[0] + i, P.lo[1] + j))];
-  }
+  const size_t bytes = size_t(a->flat_values) * sizeof(double);
+  double* flat = nullptr;
+  AMR_CUDA(cudaMallocAsync(&flat, std::max<size_t>(bytes, 8), a->stream));
+  cudaError_t e =
+      LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), flat, false, a->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(host, flat, bytes, cudaMemcpyDeviceToHost, a->stream);
+  cudaFreeAsync(flat, a->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
+  if (e != cudaSuccess) return CudaFail(e, "fvs_amr_download");
   return FVS_OK;
 }
 

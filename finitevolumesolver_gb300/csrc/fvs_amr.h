@@ -139,11 +139,10 @@ struct MaxSpeedArgs {
   int32_t ncells;
   const double* coarse;
   int32_t coarse_ncells;
-  const Seg* segs;  // the level's rows in this direction, split into segments
-  int32_t nsegs;
+  const Seg* segs;  // the level's rows in this direction
   double gamma;
   unsigned long long* smax_out;
-  // nslots > 0: one face per lane over the rows' slots (segs: whole rows)
+  // the rows' slots (PatchSweepArgs): one face per lane
   const int32_t* slot_row;
   const int32_t* row_slot0;
   int64_t nslots;
@@ -171,6 +170,19 @@ cudaError_t LaunchReflux(double* coarse, int32_t n_coarse, const double* reg,
                          cudaStream_t s);
 cudaError_t LaunchAverageDown(double* coarse, int32_t n_coarse, const double* fine,
                               int32_t n_fine, const AvgDown* e, int32_t count, cudaStream_t s);
+// A patch's interior in the flat host layout and in its level's storage.
+struct PatchCopy {
+  int64_t flat;    // first value in the flat array
+  int64_t first;   // storage index of the first interior cell
+  int32_t level, nx, ny, pitch;
+};
+struct LevelArrays {
+  double* state[kMaxLevels];
+  int64_t ncells[kMaxLevels];
+};
+// flat -> levels (to_levels) or levels -> flat, interiors only.
+cudaError_t LaunchPatchCopy(const PatchCopy* patches, int npatches, const LevelArrays& levels,
+                            double* flat, bool to_levels, cudaStream_t s);
 struct LevelDx {
   double dx[kMaxLevels];
 };

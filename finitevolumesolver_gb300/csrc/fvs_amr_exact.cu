@@ -18,37 +18,39 @@ cudaError_t LaunchPatchSweepExact(int dir, const PatchSweepArgs& a, int grid, in
 
 cudaError_t LaunchPatchMaxSpeedExact(int dir, const MaxSpeedArgs& a, int grid, int block,
                                      cudaStream_t s) {
-  if (a.nslots > 0) return LaunchPatchMaxSpeedLanesT<ExactPolicy>(dir, a, grid, block, s);
   return LaunchPatchMaxSpeedT<ExactPolicy>(dir, a, grid, block, s);
 }
 
 // U += s * (0.5 * (F1 + F2) - Fc) / dx for each register slot of the cell,
 // in slot order (register entry 3k: coarse sum, 3k+1 and 3k+2: the fine
-// sub-faces' sums).
+// sub-faces' sums).  A thread per cell and component: what bounds it is the
+// latency of its few slots, not bandwidth (15 us with a thread per cell and
+// four IEEE divisions per slot).
 __global__ void RefluxKernel(double* coarse, int32_t n_coarse, const double* reg,
                              const RefluxCell* cells, int32_t ncells, const float* signs,
                              double dx) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t / kComp, c = t % kComp;
   if (i >= ncells) return;
   const RefluxCell rc = cells[i];
+  const ieee64::Divisor ddx = ieee64::MakeDivisor(dx);
+  double* cell = coarse + int64_t(c) * n_coarse + rc.cell;
+  double U = *cell;
   for (int k = rc.first; k < rc.first + rc.count; ++k) {
     const double sign = static_cast<double>(signs[k]);
     const double* e = reg + int64_t(3 * k) * kComp;
-#pragma unroll
-    for (int c = 0; c < kComp; ++c) {
-      const double delta = 0.5 * (e[kComp + c] + e[2 * kComp + c]) - e[c];
-      double& U = coarse[int64_t(c) * n_coarse + rc.cell];
-      U = U + sign * delta / dx;
-    }
+    const double delta = 0.5 * (e[kComp + c] + e[2 * kComp + c]) - e[c];
+    U = U + ieee64::Div(sign * delta, ddx);
   }
+  *cell = U;
 }
 
 cudaError_t LaunchReflux(double* coarse, int32_t n_coarse, const double* reg,
                          const RefluxCell* cells, int32_t ncells, const float* signs, double dx,
                          cudaStream_t s) {
   if (ncells == 0) return cudaSuccess;
-  RefluxKernel<<<(ncells + 127) / 128, 128, 0, s>>>(coarse, n_coarse, reg, cells, ncells, signs,
-                                                    dx);
+  RefluxKernel<<<(int64_t(ncells) * kComp + 127) / 128, 128, 0, s>>>(coarse, n_coarse, reg, cells,
+                                                                     ncells, signs, dx);
   return cudaGetLastError();
 }
 
@@ -73,24 +75,33 @@ cudaError_t LaunchAverageDown(double* coarse, int32_t n_coarse, const double* fi
   return cudaGetLastError();
 }
 
+// The smallest of the lanes' values in lane order (the first of equal ones; a
+// NaN is never smaller).
+__device__ __forceinline__ double WarpMin(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double w = __shfl_down_sync(0xffffffffu, v, o);
+    v = w < v ? w : v;
+  }
+  return __shfl_sync(0xffffffffu, v, 0);
+}
+
 // dt = min(t_end - t, cfl * stable), stable = min over levels l and
 // directions d of 2^l * dx_l / smax(l, d), or the failed step's dt
-// (SubcycleFineFirstSolver.hpp:100-112, RunSimulation.hpp:126-151).
+// (SubcycleFineFirstSolver.hpp:100-112, RunSimulation.hpp:126-151).  One
+// warp, a lane per level and direction.
 __global__ void AmrDtKernel(AmrControl* ctrl, int nlevels, LevelDx dx) {
-  double stable;
-  if (ctrl->failure_dt > 0.0) {
-    stable = ctrl->failure_dt;
-  } else {
-    stable = 1.7976931348623157e308;
-    for (int l = 0; l < nlevels; ++l) {
-      for (int d = 0; d < 2; ++d) {
-        const double s = BitsToDouble(ctrl->smax_stable[l][d]);
-        const double dt_l = dx.dx[l] / s;
-        const double v = double(1 << l) * dt_l;
-        stable = v < stable ? v : stable;
-      }
-    }
+  const int lane = threadIdx.x;
+  double stable = 1.7976931348623157e308;
+  if (lane < 2 * nlevels) {
+    const int l = lane >> 1, d = lane & 1;
+    const double s = BitsToDouble(ctrl->smax_stable[l][d]);
+    const double v = double(1 << l) * ieee64::Div(dx.dx[l], s);
+    stable = v < stable ? v : stable;
   }
+  stable = WarpMin(stable);
+  if (lane != 0) return;
+  if (ctrl->failure_dt > 0.0) stable = ctrl->failure_dt;
   const double a = ctrl->t_end - ctrl->t;
   const double b = ctrl->cfl * stable;
   ctrl->dt = a < b ? a : b;
@@ -98,37 +109,75 @@ __global__ void AmrDtKernel(AmrControl* ctrl, int nlevels, LevelDx dx) {
 }
 
 cudaError_t LaunchAmrDt(AmrControl* ctrl, int nlevels, LevelDx dx, cudaStream_t s) {
-  AmrDtKernel<<<1, 1, 0, s>>>(ctrl, nlevels, dx);
+  AmrDtKernel<<<1, 32, 0, s>>>(ctrl, nlevels, dx);
   return cudaGetLastError();
 }
 
 // Per-sweep checks in execution order (the first failing sweep decides the
-// retry dt, 2^l times its level's dt), then commit the step.
+// retry dt, 2^l times its level's dt), then commit the step.  One warp, 32
+// sweeps at a time (28 of a 3-level step took one thread 16 us).
 __global__ void AmrEndStepKernel(AmrControl* ctrl, const SweepInfo* sweeps, int nsweeps,
                                  LevelDx dx) {
+  const int lane = threadIdx.x;
   const double dt = ctrl->dt;
-  int failed = 0;
-  for (int s = 0; s < nsweeps && !failed; ++s) {
-    const int l = sweeps[s].level;
-    const double smax = BitsToDouble(ctrl->smax_sweep[s]);
-    const double level_dt = dx.dx[l] / smax;
-    const double split = sweeps[s].scale * dt;
-    if (level_dt < split) {
-      failed = 1;
-      ctrl->failure_dt = level_dt * double(1 << l);
+  for (int base = 0; base < nsweeps; base += 32) {
+    const int s = base + lane;
+    bool bad = false;
+    double retry = 0.0;
+    if (s < nsweeps) {
+      const int l = sweeps[s].level;
+      const double smax = BitsToDouble(ctrl->smax_sweep[s]);
+      const double level_dt = ieee64::Div(dx.dx[l], smax);
+      bad = level_dt < sweeps[s].scale * dt;
+      retry = level_dt * double(1 << l);
+    }
+    const unsigned failing = __ballot_sync(0xffffffffu, bad);
+    if (failing) {
+      if (lane == __ffs(failing) - 1) {
+        ctrl->failure_dt = retry;
+        ctrl->failed = 1;
+      }
+      return;
     }
   }
-  ctrl->failed = failed;
-  if (!failed) {
-    ctrl->t = ctrl->t + dt;
-    ctrl->failure_dt = 0.0;
-    ctrl->status |= ctrl->step_status;
-  }
+  if (lane != 0) return;
+  ctrl->failed = 0;
+  ctrl->t = ctrl->t + dt;
+  ctrl->failure_dt = 0.0;
+  ctrl->status |= ctrl->step_status;
 }
 
 cudaError_t LaunchAmrEndStep(AmrControl* ctrl, const SweepInfo* sweeps, int nsweeps,
                              LevelDx dx, cudaStream_t s) {
-  AmrEndStepKernel<<<1, 1, 0, s>>>(ctrl, sweeps, nsweeps, dx);
+  AmrEndStepKernel<<<1, 32, 0, s>>>(ctrl, sweeps, nsweeps, dx);
+  return cudaGetLastError();
+}
+
+// One block per patch: the patch's interior between the flat host layout
+// ([component][ny][nx], patches one after the other) and its level's storage.
+__global__ void PatchCopyKernel(const PatchCopy* patches, LevelArrays levels, double* flat,
+                                int to_levels) {
+  const PatchCopy p = patches[blockIdx.x];
+  const int64_t area = int64_t(p.nx) * p.ny;
+  double* level = levels.state[p.level];
+  for (int64_t i = threadIdx.x; i < area; i += blockDim.x) {
+    const int64_t at = p.first + (i / p.nx) * p.pitch + i % p.nx;
+#pragma unroll
+    for (int c = 0; c < kComp; ++c) {
+      double* f = flat + p.flat + c * area + i;
+      double* q = level + c * levels.ncells[p.level] + at;
+      if (to_levels)
+        *q = *f;
+      else
+        *f = *q;
+    }
+  }
+}
+
+cudaError_t LaunchPatchCopy(const PatchCopy* patches, int npatches, const LevelArrays& levels,
+                            double* flat, bool to_levels, cudaStream_t s) {
+  if (npatches == 0) return cudaSuccess;
+  PatchCopyKernel<<<npatches, 256, 0, s>>>(patches, levels, flat, to_levels ? 1 : 0);
   return cudaGetLastError();
 }
 

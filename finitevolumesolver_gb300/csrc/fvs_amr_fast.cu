@@ -27,7 +27,6 @@ cudaError_t LaunchPatchSweepMixed(int dir, const PatchSweepArgs& a, int grid, in
 
 cudaError_t LaunchPatchMaxSpeedFast(int dir, const MaxSpeedArgs& a, int grid, int block,
                                     cudaStream_t s) {
-  if (a.nslots > 0) return LaunchPatchMaxSpeedLanesT<Fast64Policy>(dir, a, grid, block, s);
   return LaunchPatchMaxSpeedT<Fast64Policy>(dir, a, grid, block, s);
 }
 

@@ -371,10 +371,11 @@ cudaError_t LaunchPatchRowWarpT(int dir, const PatchSweepArgs& a, int grid, int 
   return cudaGetLastError();
 }
 
-// PatchMaxSpeedKernel (below) over the slots of PatchRowWarpKernel: one cell
-// and the face on its left per lane.
+// Max signal speed over the faces 0..n of every row (the stable dt of the
+// level in that direction is dx / max): one cell and the face on its left per
+// lane over the slots of PatchRowWarpKernel.
 template <int DIR, template <int> class PT>
-__global__ void __launch_bounds__(128) PatchMaxSpeedLanesKernel(MaxSpeedArgs a) {
+__global__ void __launch_bounds__(128) PatchMaxSpeedKernel(MaxSpeedArgs a) {
   using P = PT<2>;
   using R = typename P::Real;
   const typename P::Gas eq = P::MakeGas(a.gamma);
@@ -401,144 +402,6 @@ __global__ void __launch_bounds__(128) PatchMaxSpeedLanesKernel(MaxSpeedArgs a) 
 }
 
 template <template <int> class PT>
-cudaError_t LaunchPatchMaxSpeedLanesT(int dir, const MaxSpeedArgs& a, int grid, int block,
-                                      cudaStream_t s) {
-  if (dir == 0)
-    PatchMaxSpeedLanesKernel<0, PT><<<grid, block, 0, s>>>(a);
-  else
-    PatchMaxSpeedLanesKernel<1, PT><<<grid, block, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
-// Max signal speed over the faces 0..n of every row (the stable dt of the
-// level in that direction is dx / max): a segment [j0, j1) of a row takes
-// the faces j0..j1 (neighbouring segments share a face; the max does not
-// mind), so short segments give every row several threads.
-template <int DIR, template <int> class PT>
-__global__ void __launch_bounds__(128) PatchMaxSpeedKernel(MaxSpeedArgs a) {
-  using P = PT<2>;
-  using R = typename P::Real;
-  constexpr int K = kComp;
-  const typename P::Gas eq = P::MakeGas(a.gamma);
-  const int64_t N = a.ncells;
-  constexpr bool kFilter = EinfeldtCfl<P>::value;
-  const bool screen = kFilter && a.gamma > 1.0 && a.gamma <= 2.0;
-  fast::Gas<float> g32;
-  g32.gamma = static_cast<float>(a.gamma);
-  g32.gm1 = static_cast<float>(a.gamma - 1.0);
-  float thr = 0.0f;
-  unsigned long long known = 0;
-  R smax = R(0);
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < a.nsegs;
-       r += gridDim.x * blockDim.x) {
-    const Seg w = a.segs[r];
-    // loads cell j of the segment's row; returns whether it is a reflective
-    // boundary's image, whose normal momentum `finish` negates after the
-    // conversion (a select on the loaded value would wait for the load)
-    auto fetch = [&](int j, double* u) {
-      const double* src = a.in;
-      int64_t off, cs = N;
-      bool flip = false;
-      if (j >= 0 && j < w.n) {
-        off = int64_t(w.base) + int64_t(j + kGhost) * w.stride;
-      } else {  // halo cell (j = -1 or n)
-        const int h = j < 0 ? j + 2 : j - w.n + 2;
-        const int32_t g = w.halo[h];
-        if (g >= 0) {
-          off = g;
-        } else {
-          off = -int64_t(g) - 1;
-          src = a.coarse;
-          cs = a.coarse_ncells;
-        }
-        flip = (w.flip >> h) & 1;
-      }
-#pragma unroll
-      for (int c = 0; c < K; ++c) u[c] = __ldg(src + c * cs + off);
-      return flip;
-    };
-    auto finish = [&](const double* u, bool flip, R* v) {
-      P::ToCell(v, u);
-      if (flip) v[1 + DIR] = -v[1 + DIR];
-    };
-    // the cells j0 - 1 .. j1 of faces j0 .. j1, each loaded one face before
-    // its use: shift(f, v) hands out cell f - 1 and fetches cell f
-    double un[K];
-    bool fn = fetch(w.j0 - 1, un);
-    auto shift = [&](int f, R* v) {
-      double uc[K];
-#pragma unroll
-      for (int c = 0; c < K; ++c) uc[c] = un[c];
-      const bool fc = fn;
-      if (f <= w.j1) fn = fetch(f, un);
-      finish(uc, fc, v);
-    };
-    if constexpr (kFilter) {
-      known = *reinterpret_cast<volatile unsigned long long*>(a.smax_out);
-      thr = fmaxf(thr, CflFloatBelow(__longlong_as_double(static_cast<long long>(known))));
-      // FP32 screen (see the file comment): the exact waves of a face only
-      // when its bound reaches the threshold
-      auto screen_wave = [&](const R* u, bool& ok) {
-        float c32[K];
-#pragma unroll
-        for (int c = 0; c < K; ++c) c32[c] = CflToF32(u[c]);
-        const fast::Wave<float> v = fast::MakeWave<2, float>(g32, c32, DIR);
-        ok = screen && CflInRange<2>(c32) && v.a > 0.0f;
-        return v;
-      };
-      R ul[K];
-      shift(w.j0, ul);
-      bool ok_l;
-      fast::Wave<float> vl = screen_wave(ul, ok_l);
-      typename P::Wave wl;
-      bool have_l = false;
-      for (int f = w.j0; f <= w.j1; ++f) {
-        R ur[K];
-        shift(f + 1, ur);
-        bool ok_r;
-        const fast::Wave<float> vr = screen_wave(ur, ok_r);
-        const float s32 = fast::FaceMaxSpeed<float>(g32, vl, vr);
-        const float sh = fast::Math<float>::Sqrt(fmaxf(vl.h, vr.h));
-        const float bound = fmaf(s32, kCflRel, fmaf(kCflScale, sh, kCflAbs));
-        if (!(ok_l && ok_r && bound < thr)) {
-          if (!have_l) wl = P::MakeWave(eq, ul, DIR);
-          const typename P::Wave wr = P::MakeWave(eq, ur, DIR);
-          const R s = P::FaceMaxSpeed(eq, wl, wr);
-          smax = s > smax ? s : smax;
-          thr = fmaxf(thr, CflFloatBelow(static_cast<double>(smax)));
-          wl = wr;
-          have_l = true;
-        } else {
-          have_l = false;
-        }
-#pragma unroll
-        for (int c = 0; c < K; ++c) ul[c] = ur[c];
-        vl = vr;
-        ok_l = ok_r;
-      }
-      const unsigned long long b =
-          static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(smax)));
-      if (b > known) atomicMax(a.smax_out, b);
-    } else {
-      auto wave = [&](int f) {
-        R v[K];
-        shift(f, v);
-        return P::MakeWave(eq, v, DIR);
-      };
-      typename P::Wave wl = wave(w.j0);
-      for (int f = w.j0; f <= w.j1; ++f) {
-        const typename P::Wave wr = wave(f + 1);
-        const R s = P::FaceMaxSpeed(eq, wl, wr);
-        smax = s > smax ? s : smax;
-        wl = wr;
-      }
-    }
-  }
-  const double smax_d = static_cast<double>(smax);
-  BlockMaxAtomic<1>(a.smax_out, &smax_d);
-}
-
-template <template <int> class PT>
 cudaError_t LaunchPatchSweepT(int dir, const PatchSweepArgs& a, int grid, int block,
                               cudaStream_t s) {
   if (a.nsegs == 0) return cudaSuccess;
@@ -552,7 +415,7 @@ cudaError_t LaunchPatchSweepT(int dir, const PatchSweepArgs& a, int grid, int bl
 template <template <int> class PT>
 cudaError_t LaunchPatchMaxSpeedT(int dir, const MaxSpeedArgs& a, int grid, int block,
                                  cudaStream_t s) {
-  if (a.nsegs == 0) return cudaSuccess;
+  if (a.nslots == 0) return cudaSuccess;
   if (dir == 0)
     PatchMaxSpeedKernel<0, PT><<<grid, block, 0, s>>>(a);
   else

@@ -3,6 +3,7 @@
 // context with its device-resident time stepping and CUDA graphs.
 #include "../../include/fvs_gpu.h"
 #include "fvs_cutcell.h"
+#include "fvs_ieee64.cuh"
 #include "fvs_internal.h"
 #include "fvs_plotfile.h"
 #include "fvs_tma.cuh"
@@ -159,7 +160,7 @@ __global__ void BeginStepKernel(Control* c, StepPlan plan) {
     stable = 1.7976931348623157e308;
     for (int d = 0; d < plan.rank; ++d) {
       const double s = BitsToDoubleDev(c->smax_stable[d]);
-      const double dtd = plan.dxd[d] / s;
+      const double dtd = fvs::ieee64::Div(plan.dxd[d], s);
       stable = dtd < stable ? dtd : stable;
     }
   }
@@ -186,7 +187,7 @@ __global__ void EndStepKernel(Control* c, StepPlan plan, int step_in_batch,
   if (c->abort || c->done) return;
   const double split_dt = plan.frac * c->dt;
   for (int q = 0; q < plan.nsweeps; ++q) {
-    const double level_dt = plan.dx[q] / BitsToDoubleDev(c->smax_check[q]);
+    const double level_dt = fvs::ieee64::Div(plan.dx[q], BitsToDoubleDev(c->smax_check[q]));
     if (level_dt < split_dt) {
       c->abort = 1;
       c->failed_step = step_in_batch;
