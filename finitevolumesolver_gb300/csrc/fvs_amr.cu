@@ -99,6 +99,7 @@ struct fvs_amr {
   int32_t nslots = 0;
   PatchCopy* patch_copy = nullptr;  // the patches' flat and storage places
   int64_t flat_values = 0;          // values of the flat host array
+  double* flat = nullptr;           // its device copy, made by the first transfer
   float* signs = nullptr;
   AmrControl* ctrl = nullptr;
   AmrControl* ctrl_host = nullptr;
@@ -755,15 +756,12 @@ int fvs_amr_destroy(fvs_amr* a) {
 // levels stays as it is (zero: no sweep reads or writes it).
 int fvs_amr_upload(fvs_amr* a, const double* host) {
   if (!a || !host) return Fail(FVS_ERR_INVALID, "NULL argument");
-  const size_t bytes = size_t(a->flat_values) * sizeof(double);
-  double* flat = nullptr;
-  AMR_CUDA(cudaMallocAsync(&flat, std::max<size_t>(bytes, 8), a->stream));
-  cudaError_t e = cudaMemcpyAsync(flat, host, bytes, cudaMemcpyHostToDevice, a->stream);
-  if (e == cudaSuccess)
-    e = LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), flat, true, a->stream);
-  cudaFreeAsync(flat, a->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
-  if (e != cudaSuccess) return CudaFail(e, "fvs_amr_upload");
+  if (!a->flat) AMR_CUDA(a->Alloc(&a->flat, size_t(a->flat_values)));
+  AMR_CUDA(cudaMemcpyAsync(a->flat, host, size_t(a->flat_values) * sizeof(double),
+                           cudaMemcpyHostToDevice, a->stream));
+  AMR_CUDA(LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), a->flat, true,
+                           a->stream));
+  AMR_CUDA(cudaStreamSynchronize(a->stream));
   a->t = 0.0;
   a->cycle = 0;
   return FVS_OK;
@@ -771,16 +769,12 @@ int fvs_amr_upload(fvs_amr* a, const double* host) {
 
 int fvs_amr_download(fvs_amr* a, double* host) {
   if (!a || !host) return Fail(FVS_ERR_INVALID, "NULL argument");
-  const size_t bytes = size_t(a->flat_values) * sizeof(double);
-  double* flat = nullptr;
-  AMR_CUDA(cudaMallocAsync(&flat, std::max<size_t>(bytes, 8), a->stream));
-  cudaError_t e =
-      LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), flat, false, a->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(host, flat, bytes, cudaMemcpyDeviceToHost, a->stream);
-  cudaFreeAsync(flat, a->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(a->stream);
-  if (e != cudaSuccess) return CudaFail(e, "fvs_amr_download");
+  if (!a->flat) AMR_CUDA(a->Alloc(&a->flat, size_t(a->flat_values)));
+  AMR_CUDA(LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), a->flat, false,
+                           a->stream));
+  AMR_CUDA(cudaMemcpyAsync(host, a->flat, size_t(a->flat_values) * sizeof(double),
+                           cudaMemcpyDeviceToHost, a->stream));
+  AMR_CUDA(cudaStreamSynchronize(a->stream));
   return FVS_OK;
 }
 
