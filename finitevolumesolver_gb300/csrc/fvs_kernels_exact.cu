@@ -3,6 +3,8 @@
 // Compiled with -fmad=false (see build.py): no FMA contraction, IEEE
 // division and sqrt, so every result is bit-identical to the reference's
 // x86-64 build of the same formulas.
+#include <algorithm>
+
 #include "fvs_hllem.cuh"
 #include "fvs_internal.h"
 #include "fvs_recon_hllem.cuh"
@@ -22,114 +24,6 @@ cudaError_t LaunchSweepExact(const SweepArgs& a, cudaStream_t s) {
   default:
     return LaunchSweepT<3, ExactPolicy>(a, s);
   }
-}
-
-// HLLEM sweeps: the marching sweep with Hllem<PerfectGas, Larrouturou> as
-// the face flux and its stable-dt speed as the CFL check (fvs_hllem.cuh),
-// after one of four reconstructions: none (first order), MUSCL-Hancock of
-// the conservative variables, the characteristic or the primitive
-// reconstruction of the perfect gas (fvs_recon_hllem.cuh).
-template <int D> struct HllemWave {
-  exact::Complete<D> q;
-  int dir;
-};
-
-enum HllemRecon : int { kReconNone = 0, kReconCons = 1, kReconChar = 2, kReconPrim = 3 };
-
-template <int D, int kRecon> struct HllemPolicyT {
-  using Real = double;
-  static constexpr bool kWarpX = false;
-  static constexpr int kMinBlocks = 1;
-  static constexpr int kLaneBlocks = 3;
-  static constexpr bool kHllemCfl = true;  // CFL speeds screened in FP32 (HllemScreen)
-  using Gas = exact::Gas;
-  using Rec = exact::Complete<D>;
-  using Wave = HllemWave<D>;
-  using Stats = NoStats;
-  static __device__ __forceinline__ Gas MakeGas(double gamma) {
-    return ExactPolicy<D>::MakeGas(gamma);
-  }
-  static __device__ __forceinline__ Gas MakeGasFor(const SweepArgs& a) { return MakeGas(a.gamma); }
-  static __device__ __forceinline__ void ToCell(double* c, const double* u) {
-#pragma unroll
-    for (int k = 0; k < D + 2; ++k) c[k] = u[k];
-  }
-  static __device__ __forceinline__ void Predict(const Gas& eq, Rec& recL, Rec& recR,
-                                                 const double* q0, const double* q1,
-                                                 const double* q2, int limiter,
-                                                 double lambda_half, int dir) {
-    if constexpr (kRecon == kReconCons) {
-      exact::MusclPredictBoth<D>(eq, recL, recR, q0, q1, q2, limiter, lambda_half, dir);
-    } else if constexpr (kRecon == kReconChar || kRecon == kReconPrim) {
-      // dt/dx: lambda_half is (0.5 dt)/dx, so doubling it is exact
-      const double lambda = 2.0 * lambda_half;
-      exact::Complete<D> s0, s1, s2;
-      exact::CompleteFromCons<D>(eq, s0, q0);
-      exact::CompleteFromCons<D>(eq, s1, q1);
-      exact::CompleteFromCons<D>(eq, s2, q2);
-      if constexpr (kRecon == kReconChar)
-        exact::CharPredictBoth<D>(eq, recL, recR, s0, s1, s2, lambda, dir);
-      else
-        exact::PrimPredictBoth<D>(eq, recL, recR, s0, s1, s2, lambda, dir);
-    } else {
-      exact::CompleteFromCons<D>(eq, recL, q1);
-      recR = recL;
-    }
-  }
-  static __device__ __forceinline__ Wave MakeWave(const Gas& eq, const double* u, int dir) {
-    Wave w;
-    exact::CompleteFromCons<D>(eq, w.q, u);
-    w.dir = dir;
-    return w;
-  }
-  static __device__ __forceinline__ double FaceMaxSpeed(const Gas& eq, const Wave& wL,
-                                                        const Wave& wR) {
-    return exact::HllemMaxSpeed<D>(eq, wL.q, wR.q, wL.dir);
-  }
-  static __device__ __forceinline__ void FluxOnly(const Gas& eq, double* F, const Rec& L,
-                                                  const Rec& R, int dir) {
-    exact::HllemFlux<D>(eq, F, L, R, dir);
-  }
-  static __device__ __forceinline__ double Face(const Gas& eq, double* F, const Rec& L,
-                                                const Rec& R, const Wave& wL, const Wave& wR,
-                                                int dir, Stats&) {
-    exact::HllemFlux<D>(eq, F, L, R, dir);
-    return exact::HllemMaxSpeed<D>(eq, wL.q, wR.q, dir);
-  }
-};
-
-template <int D> struct HllemPolicy : HllemPolicyT<D, kReconNone> {};
-template <int D> struct MusclHllemPolicy : HllemPolicyT<D, kReconCons> {};
-template <int D> struct CharHllemPolicy : HllemPolicyT<D, kReconChar> {};
-template <int D> struct PrimHllemPolicy : HllemPolicyT<D, kReconPrim> {};
-
-template <template <int> class PT>
-cudaError_t LaunchSweepRanks(const SweepArgs& a, cudaStream_t s) {
-  switch (a.rank) {
-  case 1:
-    return LaunchSweepT<1, PT>(a, s);
-  case 2:
-    return LaunchSweepT<2, PT>(a, s);
-  default:
-    return LaunchSweepT<3, PT>(a, s);
-  }
-}
-
-cudaError_t LaunchSweepHllem(const SweepArgs& a, int recon, cudaStream_t s) {
-  switch (recon) {
-  case kReconCons:
-    return LaunchSweepRanks<MusclHllemPolicy>(a, s);
-  case kReconChar:
-    return LaunchSweepRanks<CharHllemPolicy>(a, s);
-  case kReconPrim:
-    return LaunchSweepRanks<PrimHllemPolicy>(a, s);
-  default:
-    return LaunchSweepRanks<HllemPolicy>(a, s);
-  }
-}
-
-cudaError_t LaunchStableDtHllem(const StableDtArgs& a, cudaStream_t s) {
-  return LaunchStableDtT<HllemPolicy>(a, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -271,9 +165,11 @@ __device__ __forceinline__ void Unflatten(int64_t id, const BoxDesc& b, int* ijk
 }
 
 // FluxMethod<Base>::ComputeNumericFluxes (FluxMethod.hpp:200-215): face f
-// takes the 2w cells f-w .. f+w-1 along dir.
+// takes the 2w cells f-w .. f+w-1 along dir.  Methods 1 and 4 (HLLE, HLLEM), 6
+// and 7 (characteristic and primitive reconstruction); the conservative
+// MUSCL-Hancock methods take PatchFluxLanesKernel.
 template <int D>
-__global__ void PatchFluxKernel(int method, int limiter, double gamma,
+__global__ void PatchFluxKernel(int method, double gamma,
                                 double* fluxes, BoxDesc fbox, View st,
                                 double dt, double dx, int dir) {
   constexpr int K = D + 2;
@@ -293,7 +189,7 @@ __global__ void PatchFluxKernel(int method, int limiter, double gamma,
       exact::HllFlux<D>(eq, nf, L, R, dir);
     else
       exact::HllemFlux<D>(eq, nf, L, R, dir);
-  } else if (method == 6 || method == 7) {
+  } else {
     // characteristic / primitive reconstruction + HLLEM, stencil width 2
     // (MusclHancockCharacteristicMethod.hpp:303-317,
     // MusclHancockPrimMethod.hpp:59-182), from the stored complete states
@@ -313,28 +209,88 @@ __global__ void PatchFluxKernel(int method, int limiter, double gamma,
       exact::PrimPredictBoth<D>(eq, a1, b1, q[1], q[2], q[3], lambda, dir);
     }
     exact::HllemFlux<D>(eq, nf, b0, a1, dir);
-  } else {  // MUSCL-Hancock (conservative) + HLLE / HLLEM, stencil width 2
-    double u[4][K];
-    for (int s = 0; s < 4; ++s) {
-      int c[3] = {f[0], f[1], f[2]};
-      c[dir] += s - 2;
-#pragma unroll
-      for (int q = 0; q < K; ++q) u[s][q] = st(q, c[0], c[1], c[2]);
-    }
-    exact::Complete<D> a0, b0, a1, b1;
-    const double lambda_half = 0.5 * dt / dx;
-    exact::MusclPredictBoth<D>(eq, a0, b0, u[0], u[1], u[2], limiter,
-                               lambda_half, dir);
-    exact::MusclPredictBoth<D>(eq, a1, b1, u[1], u[2], u[3], limiter,
-                               lambda_half, dir);
-    if (method == 5)
-      exact::HllemFlux<D>(eq, nf, b0, a1, dir);
-    else
-      exact::HllFlux<D>(eq, nf, b0, a1, dir);
   }
   View fv{fluxes, fbox};
 #pragma unroll
   for (int q = 0; q < K; ++q) fluxes[fv.Index(q, f[0], f[1], f[2])] = nf[q];
+}
+
+// MUSCL-Hancock + HLLE / HLLEM fluxes with the lanes of a warp along dir: the
+// face box's lines laid end to end as slots, the cells f0-1 .. f0+n-1 of the n
+// faces of a line; a lane evaluates its cell's predictor and, with the right
+// state its left neighbour's lane hands it, the flux of the face on the
+// cell's left, so a cell's predictor is evaluated once (PatchFluxKernel: for
+// each of its two faces) and a patch's serial chain is a third shorter.  Warps
+// share a slot with their predecessor: 31 faces each.
+constexpr int kPatchStep = 31;
+
+template <int D, int dir, bool kHllem>
+__global__ void __launch_bounds__(128)
+    PatchFluxLanesKernel(int limiter, double gamma, double* fluxes, BoxDesc fbox, BoxDesc part,
+                         View st, double dt, double dx, uint32_t slots) {
+  constexpr int K = D + 2;
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t want = warp * kPatchStep + lane;
+  const uint32_t slot = want < slots ? want : slots - 1;
+  const uint32_t per = uint32_t(part.n[dir]) + 1;
+  const uint32_t line = slot / per, at = slot - line * per;
+  // the line's place in the two other directions, and the slot's cell
+  constexpr int d1 = dir == 0 ? 1 : 0, d2 = dir == 2 ? 1 : 2;
+  int f[3];
+  f[dir] = part.lo[dir] + static_cast<int>(at) - 1;
+  f[d1] = part.lo[d1] + static_cast<int>(line % uint32_t(part.n[d1]));
+  f[d2] = part.lo[d2] + static_cast<int>(line / uint32_t(part.n[d1]));
+  double u[3][K];
+  for (int s = 0; s < 3; ++s) {
+    int c[3] = {f[0], f[1], f[2]};
+    c[dir] += s - 1;
+#pragma unroll
+    for (int q = 0; q < K; ++q) u[s][q] = st(q, c[0], c[1], c[2]);
+  }
+  const exact::Gas eq = ExactPolicy<1>::MakeGas(gamma);
+  exact::Complete<D> a, b;
+  exact::MusclPredictBoth<D>(eq, a, b, u[0], u[1], u[2], limiter, exact::Div(0.5 * dt, dx), dir);
+  const exact::Complete<D> left = ShflUp(b, 1);
+  double nf[K];
+  if constexpr (kHllem)
+    exact::HllemFlux<D>(eq, nf, left, a, dir);
+  else
+    exact::HllFlux<D>(eq, nf, left, a, dir);
+  if (want >= slots || lane == 0 || at == 0) return;
+  View fv{fluxes, fbox};
+#pragma unroll
+  for (int q = 0; q < K; ++q) fluxes[fv.Index(q, f[0], f[1], f[2])] = nf[q];
+}
+
+// The lines of the face box in parts of fewer than 2^30 slots.
+template <int D, int dir>
+void LaunchPatchFluxLanes(int method, int limiter, double gamma, double* fluxes,
+                          const BoxDesc& fbox, const View& st, double dt, double dx,
+                          cudaStream_t s) {
+  constexpr int64_t kMost = int64_t(1) << 30;
+  constexpr int d1 = dir == 0 ? 1 : 0, d2 = dir == 2 ? 1 : 2;
+  const int64_t per = int64_t(fbox.n[dir]) + 1;
+  const int64_t step1 = std::max<int64_t>(1, std::min<int64_t>(fbox.n[d1], kMost / per));
+  const int64_t step2 = std::max<int64_t>(1, std::min<int64_t>(fbox.n[d2], kMost / (per * step1)));
+  for (int64_t k = 0; k < fbox.n[d2]; k += step2) {
+    for (int64_t j = 0; j < fbox.n[d1]; j += step1) {
+      BoxDesc part = fbox;
+      part.lo[d1] = fbox.lo[d1] + static_cast<int>(j);
+      part.n[d1] = static_cast<int>(std::min<int64_t>(step1, fbox.n[d1] - j));
+      part.lo[d2] = fbox.lo[d2] + static_cast<int>(k);
+      part.n[d2] = static_cast<int>(std::min<int64_t>(step2, fbox.n[d2] - k));
+      const uint32_t slots = static_cast<uint32_t>(per * part.n[d1] * part.n[d2]);
+      const uint32_t warps = (slots - 1 + kPatchStep - 1) / kPatchStep;
+      const unsigned grid = (warps + 3) / 4;
+      if (method == 5)
+        PatchFluxLanesKernel<D, dir, true>
+            <<<grid, 128, 0, s>>>(limiter, gamma, fluxes, fbox, part, st, dt, dx, slots);
+      else
+        PatchFluxLanesKernel<D, dir, false>
+            <<<grid, 128, 0, s>>>(limiter, gamma, fluxes, fbox, part, st, dt, dx, slots);
+    }
+  }
 }
 
 cudaError_t LaunchPatchFluxesExact(int method, int limiter, int rank,
@@ -347,17 +303,29 @@ cudaError_t LaunchPatchFluxesExact(int method, int limiter, int rank,
   const int block = 128;
   const unsigned grid = static_cast<unsigned>((nface + block - 1) / block);
   View st{states, cbox};
+  if (method == 0 || method == 5) {
+    auto launch = [&](auto kernels) { kernels(method, limiter, gamma, fluxes, fbox, st, dt, dx, s); };
+    if (rank == 1)
+      launch(LaunchPatchFluxLanes<1, 0>);
+    else if (rank == 2)
+      launch(dir == 0 ? LaunchPatchFluxLanes<2, 0> : LaunchPatchFluxLanes<2, 1>);
+    else
+      launch(dir == 0   ? LaunchPatchFluxLanes<3, 0>
+             : dir == 1 ? LaunchPatchFluxLanes<3, 1>
+                        : LaunchPatchFluxLanes<3, 2>);
+    return cudaGetLastError();
+  }
   switch (rank) {
   case 1:
-    PatchFluxKernel<1><<<grid, block, 0, s>>>(method, limiter, gamma, fluxes,
+    PatchFluxKernel<1><<<grid, block, 0, s>>>(method, gamma, fluxes,
                                               fbox, st, dt, dx, dir);
     break;
   case 2:
-    PatchFluxKernel<2><<<grid, block, 0, s>>>(method, limiter, gamma, fluxes,
+    PatchFluxKernel<2><<<grid, block, 0, s>>>(method, gamma, fluxes,
                                               fbox, st, dt, dx, dir);
     break;
   default:
-    PatchFluxKernel<3><<<grid, block, 0, s>>>(method, limiter, gamma, fluxes,
+    PatchFluxKernel<3><<<grid, block, 0, s>>>(method, gamma, fluxes,
                                               fbox, st, dt, dx, dir);
     break;
   }
