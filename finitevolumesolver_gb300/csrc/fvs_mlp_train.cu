@@ -310,7 +310,11 @@ constexpr uint32_t kOffSX = 0;
 constexpr uint32_t kOffSW1 = kOffSX + 2 * kLboRow;
 constexpr uint32_t kOffSW2 = kOffSW1 + 2 * kLboW;
 constexpr uint32_t kOffSH1 = kOffSW2 + 8 * kLboW;
-constexpr uint32_t kForwardSmem = kOffSH1 + 8 * kLboRow;
+// GELU(Z2) of the tile, [128][65] fp32: the output layer's sum runs over a
+// row's units in order, so that its rounding does not depend on the tiling
+constexpr int kActPitch = kH + 1;
+constexpr uint32_t kOffAct = kOffSH1 + 8 * kLboRow;
+constexpr uint32_t kForwardSmem = kOffAct + kTile * kActPitch * 4;
 constexpr uint32_t kOffSW2t = kForwardSmem;
 constexpr uint32_t kOffSD2 = kOffSW2t + 8 * kLboW;
 constexpr uint32_t kOffSG = kOffSD2 + 8 * kLboRow;
@@ -433,6 +437,14 @@ __device__ __forceinline__ float SumUnits(float* v, int lane, int* index) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// The output layer of a row.
+__device__ __forceinline__ float OutputSum(const float* act, const float* w3, float b3) {
+  float y = b3;
+#pragma unroll 16
+  for (int o = 0; o < kH; ++o) y = fmaf(w3[o], act[o], y);
+  return y;
+}
+
 struct FusedArgs {
   const float* feat;   // raw features [n][5]
   const float* label;  // [n]
@@ -459,7 +471,7 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   __shared__ uint32_t tmem_base;
   __shared__ float vec[mlp::kParams - mlp::kOffB2];  // b2, w3, b3
   __shared__ float b1[kH], stats[2 * mlp::kIn];
-  __shared__ float ypart[4][kTile], target[kTile];
+  __shared__ float residual[kTile], target[kTile];
   // per row-warp sums over the tiles: db1, db2, dw3 and (db3, loss)
   __shared__ float sums[4][3 * kH + 2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -485,6 +497,7 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   const uint32_t base = tc::SmemAddr(sm);
   const float* w3 = vec + (mlp::kOffW3 - mlp::kOffB2);
   const float b3 = vec[mlp::kOffB3 - mlp::kOffB2];
+  float* act = reinterpret_cast<float*>(sm + kOffAct);
   const unsigned long long step = a.step[0];
   MmaPhases mma{&bar, a.error};
   const int tiles = a.batch / kTile;
@@ -521,16 +534,15 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
       IssueMma(tmem, kColZ2, base + kOffSH1, kLboRow, base + kOffSW2, kLboW, kH, 8, false, &bar);
     });
     tc::TmemLoad16(lanes + kColZ2 + u0, v);
-    float y = 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       gw[i] = GeluBoth(v[i] + vec[u0 + i], &d[i]);
-      y = fmaf(w3[u0 + i], gw[i], y);
+      act[row * kActPitch + u0 + i] = gw[i];
     }
-    ypart[group][row] = y;
     __syncthreads();
-    const float e =
-        (b3 + ypart[0][row] + ypart[1][row] + ypart[2][row] + ypart[3][row]) - target[row];
+    if (group == 0) residual[row] = OutputSum(act + row * kActPitch, w3, b3) - target[row];
+    __syncthreads();
+    const float e = residual[row];
     const float dy = 2.0f * e / float(a.batch);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -648,7 +660,6 @@ __global__ void __launch_bounds__(kFusedThreads)
   __shared__ uint32_t tmem_base;
   __shared__ float vec[mlp::kParams - mlp::kOffB2];
   __shared__ float b1[kH], stats[2 * mlp::kIn];
-  __shared__ float ypart[4][kTile];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rw = warp & 3, group = warp >> 2, row = rw * 32 + lane, u0 = group * 16;
   if (warp == 0) tc::TmemAlloc(&tmem_base, kInferCols);
@@ -668,6 +679,7 @@ __global__ void __launch_bounds__(kFusedThreads)
   const uint32_t lanes = tmem + (uint32_t(rw * 32) << 16);
   const uint32_t base = tc::SmemAddr(sm);
   const float* w3 = vec + (mlp::kOffW3 - mlp::kOffB2);
+  float* act = reinterpret_cast<float*>(sm + kOffAct);
   MmaPhases mma{&bar, error};
   const int64_t tiles = (n + kTile - 1) / kTile;
   for (int64_t tile = blockIdx.x; tile < tiles && mma.ok; tile += gridDim.x) {
@@ -691,14 +703,12 @@ __global__ void __launch_bounds__(kFusedThreads)
       IssueMma(tmem, kColZ2, base + kOffSH1, kLboRow, base + kOffSW2, kLboW, kH, 8, false, &bar);
     });
     tc::TmemLoad16(lanes + kColZ2 + u0, v);
-    float y = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) y = fmaf(w3[u0 + i], GeluBoth(v[i] + vec[u0 + i], &unused), y);
-    ypart[group][row] = y;
+    for (int i = 0; i < 16; ++i)
+      act[row * kActPitch + u0 + i] = GeluBoth(v[i] + vec[u0 + i], &unused);
     __syncthreads();
     if (group == 0 && r < n && mma.ok)
-      y_out[r] = vec[mlp::kOffB3 - mlp::kOffB2] + ypart[0][row] + ypart[1][row] + ypart[2][row] +
-                 ypart[3][row];
+      y_out[r] = OutputSum(act + row * kActPitch, w3, vec[mlp::kOffB3 - mlp::kOffB2]);
   }
   tc::FenceBeforeSync();
   __syncthreads();
@@ -996,7 +1006,7 @@ int fvs_mlp_predict(fvs_mlp* m, const float* features_dev, int64_t n, float* y_d
   if (!m || !features_dev || !y_dev || n < 0) return MlpFail(FVS_ERR_INVALID, "bad arguments");
   if (n == 0) return FVS_OK;
   cudaStream_t s = m->stream;
-  // two CTAs fit an SM's shared memory several times over; their phases overlap
+  // three CTAs fit an SM's shared and tensor memory; their phases overlap
   const int64_t grid = std::min<int64_t>((n + kTile - 1) / kTile, int64_t(m->ctas) * 3);
   InferKernel<<<unsigned(grid), kFusedThreads, kForwardSmem, s>>>(
       n, features_dev, m->net.blob, m->net.W1, m->net.W2, y_dev, m->error);
