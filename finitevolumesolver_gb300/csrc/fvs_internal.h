@@ -58,6 +58,17 @@ constexpr int kTmaRows = 2;
 constexpr int kTmaStages = 4;
 constexpr int kTmaWarps = 4;
 
+// The exact Riemann solver's constants of gamma, computed on the host: kernel
+// parameters, so that they cost no registers and no FP64 divisions.
+struct RiemannConstants {
+  double gamma, gamma_minus_1_inv;
+  int root_n;                   // 0: pow(), else n with n-th roots in its place
+  double inv_n, second;         // 1 / n and (n + 1) / (2 n^2)
+  double gp1, gm1, g_ratio;     // g + 1, g - 1, (g - 1) / (g + 1)
+  double exponent, d_exponent;  // 0.5 (g - 1) / g, -0.5 (g + 1) / g
+  double z, inv_g, two_gp1;     // (g - 1) / (2 g), 1 / g, 2 / (g + 1)
+};
+
 // One directional sweep of a uniform grid: fluxes, conservative update and
 // the CFL reduction of the input state, in one pass.
 struct SweepArgs {
@@ -86,6 +97,7 @@ struct SweepArgs {
   int max_iterations;
   double tolerance;
   const float* mlp;     // learned-guess weights (guess == FVS_GUESS_MLP)
+  RiemannConstants rc;  // of gamma, set by LaunchSweepGodunov
   unsigned long long* stats_out;  // [3]: Newton iterations, non-converged, fallbacks
   // the first sweep of a step: its input's face speeds are the stable-dt
   // pass's, so the sweep computes no cell waves and no CFL speeds

@@ -15,16 +15,17 @@ struct GodunovGas {
   riemann::Options opt;
 };
 
-__device__ __forceinline__ GodunovGas MakeGodunovGas(double gamma, int guess, int max_it,
-                                                     double tol, const float* mlp) {
+__host__ __device__ __forceinline__ GodunovGas MakeGodunovGas(const RiemannConstants& c,
+                                                              int guess, int max_it, double tol,
+                                                              const float* mlp) {
   GodunovGas g;
-  g.eq.gamma = gamma;
-  g.eq.gamma_minus_1_inv = ieee64::Div(1.0, gamma - 1.0);
+  g.eq.gamma = c.gamma;
+  g.eq.gamma_minus_1_inv = c.gamma_minus_1_inv;
   g.opt.guess = guess;
   g.opt.max_iterations = max_it;
   g.opt.tol = tol;
   g.opt.mlp = mlp;
-  g.opt.root_n = riemann::RootOrder(gamma);
+  g.opt.c = c;
   return g;
 }
 
@@ -45,7 +46,7 @@ template <int D, bool kMuscl> struct GodunovPolicyT {
   using Wave = exact::Complete<D>;
   using Stats = NewtonStats;
   static __device__ __forceinline__ Gas MakeGasFor(const SweepArgs& a) {
-    return MakeGodunovGas(a.gamma, a.guess, a.max_iterations, a.tolerance, a.mlp);
+    return MakeGodunovGas(a.rc, a.guess, a.max_iterations, a.tolerance, a.mlp);
   }
   static __device__ __forceinline__ void ToCell(double* c, const double* u) {
 #pragma unroll
@@ -79,9 +80,9 @@ template <int D, bool kMuscl> struct GodunovPolicyT {
       st.iterations += c.iterations;
       st.failures += c.converged ? 0 : 1;
       st.fallbacks += c.fallback;
-      return riemann::SignalMaxSpeed<D>(g.eq, wL, wR, dir, c.p);
+      return riemann::SignalMaxSpeed<D>(g.eq, wL, wR, dir, c.p, g.opt);
     } else {
-      return riemann::SignalMaxSpeed<D>(g.eq, L, R, dir, s.p);
+      return riemann::SignalMaxSpeed<D>(g.eq, L, R, dir, s.p, g.opt);
     }
   }
 };
@@ -89,7 +90,9 @@ template <int D, bool kMuscl> struct GodunovPolicyT {
 template <int D> struct GodunovPolicy : GodunovPolicyT<D, false> {};
 template <int D> struct MusclGodunovPolicy : GodunovPolicyT<D, true> {};
 
-cudaError_t LaunchSweepGodunov(const SweepArgs& a, bool muscl, cudaStream_t s) {
+cudaError_t LaunchSweepGodunov(const SweepArgs& args, bool muscl, cudaStream_t s) {
+  SweepArgs a = args;
+  a.rc = riemann::MakeConstants(a.gamma, riemann::RootOrder(a.gamma));
   switch (a.rank) {
   case 1:
     return muscl ? LaunchSweepT<1, MusclGodunovPolicy>(a, s) : LaunchSweepT<1, GodunovPolicy>(a, s);
@@ -102,13 +105,11 @@ cudaError_t LaunchSweepGodunov(const SweepArgs& a, bool muscl, cudaStream_t s) {
 
 // Stable dt over all directions with the exact solver's signal speeds.
 template <int D>
-__global__ void __launch_bounds__(256) GodunovStableDtKernel(StableDtArgs a, int guess, int max_it,
-                                                             double tol, const float* mlp) {
+__global__ void __launch_bounds__(256) GodunovStableDtKernel(StableDtArgs a, GodunovGas g) {
   constexpr int K = D + 2;
   const int nx = a.n[0], ny = a.n[1], nz = a.n[2];
   const int64_t cs = int64_t(nx) * ny * nz;
   if (!BlockAll(!(a.ctrl && (a.ctrl->abort || a.ctrl->done)))) return;
-  const GodunovGas g = MakeGodunovGas(a.gamma, guess, max_it, tol, mlp);
   double smax[3] = {0.0, 0.0, 0.0};
   // grid-stride over cells; one atomic per block and direction at the end
   for (int64_t cell = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; cell < cs;
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(256) GodunovStableDtKernel(StableDtArgs a, int
         const exact::Complete<D>& L = (fi == 0) ? o : q;
         const exact::Complete<D>& R = (fi == 0) ? q : o;
         const riemann::Star st = riemann::ComputeMiddleState<D>(g.eq, L, R, d, g.opt);
-        const double sp = riemann::SignalMaxSpeed<D>(g.eq, L, R, d, st.p);
+        const double sp = riemann::SignalMaxSpeed<D>(g.eq, L, R, d, st.p, g.opt);
         smax[d] = sp > smax[d] ? sp : smax[d];
       }
     }
@@ -154,15 +155,17 @@ cudaError_t LaunchStableDtGodunov(const StableDtArgs& a, int guess, int max_it, 
   const int64_t cells = int64_t(a.n[0]) * a.n[1] * a.n[2];
   const int block = 256;
   const unsigned grid = GridStrideBlocks(cells, block, 8);
+  const GodunovGas g = MakeGodunovGas(
+      riemann::MakeConstants(a.gamma, riemann::RootOrder(a.gamma)), guess, max_it, tol, mlp);
   switch (a.rank) {
   case 1:
-    GodunovStableDtKernel<1><<<grid, block, 0, s>>>(a, guess, max_it, tol, mlp);
+    GodunovStableDtKernel<1><<<grid, block, 0, s>>>(a, g);
     break;
   case 2:
-    GodunovStableDtKernel<2><<<grid, block, 0, s>>>(a, guess, max_it, tol, mlp);
+    GodunovStableDtKernel<2><<<grid, block, 0, s>>>(a, g);
     break;
   default:
-    GodunovStableDtKernel<3><<<grid, block, 0, s>>>(a, guess, max_it, tol, mlp);
+    GodunovStableDtKernel<3><<<grid, block, 0, s>>>(a, g);
     break;
   }
   return cudaGetLastError();
@@ -258,7 +261,7 @@ __global__ void PatchGodunovDtKernel(int w, GodunovGas g, GView st, BoxDesc wbox
     c[dir] += 1;
     const exact::Complete<D> R = LoadC<D>(st, c);
     const riemann::Star m = riemann::ComputeMiddleState<D>(g.eq, L, R, dir, g.opt);
-    s = riemann::SignalMaxSpeed<D>(g.eq, L, R, dir, m.p);
+    s = riemann::SignalMaxSpeed<D>(g.eq, L, R, dir, m.p, g.opt);
   }
   s = WarpMax(s);
   if ((threadIdx.x & 31) == 0 && s > 0.0) AtomicMaxPositive(smax_out, s);
@@ -300,7 +303,8 @@ cudaError_t LaunchPatchGodunovFluxes(bool muscl, int limiter, int rank, double g
   if (nface == 0) return cudaSuccess;
   const int block = 128;
   const unsigned grid = static_cast<unsigned>((nface + block - 1) / block);
-  const GodunovGas g{{gamma, 1.0 / (gamma - 1.0)}, {guess, max_it, tol, mlp}};
+  const GodunovGas g =
+      MakeGodunovGas(riemann::MakeConstants(gamma, 0), guess, max_it, tol, mlp);  // pow()
   const GView st{states, cbox};
   switch (rank) {
   case 1:
@@ -330,7 +334,8 @@ cudaError_t LaunchPatchGodunovStableDt(bool muscl, int rank, double gamma, int g
   const int64_t nwin = int64_t(wbox.n[0]) * wbox.n[1] * wbox.n[2];
   const int block = 128;
   const unsigned grid = static_cast<unsigned>((nwin + block - 1) / block);
-  const GodunovGas g{{gamma, 1.0 / (gamma - 1.0)}, {guess, max_it, tol, mlp}};
+  const GodunovGas g =
+      MakeGodunovGas(riemann::MakeConstants(gamma, 0), guess, max_it, tol, mlp);  // pow()
   const GView st{states, cbox};
   switch (rank) {
   case 1:
@@ -354,7 +359,8 @@ cudaError_t LaunchExactStar(int64_t n, double gamma, int guess, int max_it, doub
   if (n <= 0) return cudaSuccess;
   const int block = 128;
   const unsigned grid = static_cast<unsigned>((n + block - 1) / block);
-  const GodunovGas g{{gamma, 1.0 / (gamma - 1.0)}, {guess, max_it, tol, mlp}};
+  const GodunovGas g =
+      MakeGodunovGas(riemann::MakeConstants(gamma, 0), guess, max_it, tol, mlp);  // pow()
   ExactStarKernel<1><<<grid, block, 0, s>>>(n, g, rhoL, uL, pL, rhoR, uR, pR, pstar, ustar, iters,
                                             converged);
   return cudaGetLastError();

@@ -26,6 +26,7 @@
 //    from it has not converged within 64 steps.
 #pragma once
 
+#include "fvs_internal.h"
 #include "fvs_mlp.cuh"
 #include "fvs_physics_exact.cuh"
 #include "fvs_roots.cuh"
@@ -40,8 +41,46 @@ struct Options {
   int max_iterations;
   double tol;
   const float* mlp;  // learned-guess parameters (kGuessMlp)
-  int root_n;        // RootOrder(gamma): 0, or n with n-th roots in place of pow()
+  RiemannConstants c;
 };
+
+// root_n: RootOrder(gamma) for n-th roots, 0 for pow().
+inline RiemannConstants MakeConstants(double g, int root_n) {
+  RiemannConstants c;
+  c.gamma = g;
+  c.gamma_minus_1_inv = 1.0 / (g - 1.0);
+  const Powers pw(root_n);
+  c.root_n = root_n;
+  c.inv_n = pw.inv_n;
+  c.second = pw.second;
+  c.gp1 = g + 1.0;
+  c.gm1 = g - 1.0;
+  c.g_ratio = c.gm1 / c.gp1;
+  c.exponent = 0.5 * c.gm1 / g;
+  c.d_exponent = -0.5 * c.gp1 / g;
+  c.z = c.gm1 / (2.0 * g);
+  c.inv_g = 1 / g;
+  c.two_gp1 = 2.0 / c.gp1;
+  return c;
+}
+__device__ __forceinline__ Powers PowersOf(const RiemannConstants& c) {
+  Powers p;
+  p.n = c.root_n;
+  p.inv_n = c.inv_n;
+  p.second = c.second;
+  return p;
+}
+
+// Comparisons on the integer pipes, with IEEE results for zeros and NaN.
+using ieee64::Less;
+using ieee64::Negative;
+using ieee64::Positive;
+__device__ __forceinline__ bool NotNegative(double x) {  // 0 <= x
+  return !Negative(x) && !ieee64::IsNan(x);
+}
+__device__ __forceinline__ bool NotPositive(double x) {  // x <= 0
+  return !Positive(x) && !ieee64::IsNan(x);
+}
 
 // Quotients and square roots of the solver's variable operands on the integer
 // pipes (fvs_ieee64.cuh, nearly rounded: within 0.57 and 0.75 ulp), since the
@@ -93,22 +132,23 @@ template <int D> __device__ __forceinline__ double SquaredNormScalar(const doubl
 // PVRS estimate, replaced by the two-rarefaction estimate below min(pL, pR)
 // (Toro, Riemann Solvers and Numerical Methods for Fluid Dynamics, 3rd ed.,
 // section 9.5); floored at 1e-8 min(pL, pR).
-__device__ __forceinline__ double PvrsTrGuess(const Powers& pw, double g, double rhoL, double uL,
+__device__ __forceinline__ double PvrsTrGuess(const Options& opt, double g, double rhoL, double uL,
                                               double pL, double aL, double rhoR, double uR,
                                               double pR, double aR) {
-  const double pmin = pL < pR ? pL : pR;
+  const Powers pw = PowersOf(opt.c);
+  const double pmin = Less(pL, pR) ? pL : pR;
   const double ppv = 0.5 * (pL + pR) - 0.125 * (uR - uL) * (rhoL + rhoR) * (aL + aR);
   double p0;
-  if (ppv >= pmin) {
+  if (!Less(ppv, pmin) && !ieee64::IsNan(ppv) && !ieee64::IsNan(pmin)) {
     p0 = ppv;
   } else {
-    const double z = (g - 1.0) / (2.0 * g);
-    const double num = aL + aR - 0.5 * (g - 1.0) * (uR - uL);
+    const double z = opt.c.z;
+    const double num = aL + aR - 0.5 * opt.c.gm1 * (uR - uL);
     const double den = Div(aL, pw.Z(pL, z)) + Div(aR, pw.Z(pR, z));
-    p0 = (num > 0.0) ? pw.N(Div(num, den), 1.0 / z) : 0.0;
+    p0 = Positive(num) ? pw.N(Div(num, den), 1.0 / z) : 0.0;
   }
   const double floor = 1e-8 * pmin;
-  return p0 > floor ? p0 : floor;
+  return Less(floor, p0) ? p0 : floor;
 }
 
 struct SideFn {
@@ -117,7 +157,7 @@ struct SideFn {
 
 __device__ __forceinline__ double FSide(const SideFn& s, double gm1, double exponent,
                                         const Powers& pw, double q) {
-  if (q > s.p) {
+  if (Less(s.p, q)) {
     return (q - s.p) * Sqrt(Div(s.A, q + s.B));
   }
   return Div(2.0 * s.a, gm1) * (pw.Z(Div(q, s.p), exponent) - 1.0);
@@ -125,7 +165,7 @@ __device__ __forceinline__ double FSide(const SideFn& s, double gm1, double expo
 
 __device__ __forceinline__ double DfSide(const SideFn& s, double d_exponent, const Powers& pw,
                                          double q) {
-  if (q > s.p) {
+  if (Less(s.p, q)) {
     return Sqrt(Div(s.A, s.B + q)) * (1.0 - Div(0.5 * (q - s.p), s.B + q));
   }
   return Div(pw.ZMinus1(Div(q, s.p), d_exponent), s.rho * s.a);
@@ -154,19 +194,19 @@ __device__ __forceinline__ FEval NewtonFrom(const SideFn& L, const SideFn& R, do
   double fx = e.fR + e.fL + du;
   int counter = 0;
   double err = fabs(fx);
-  while (err > tol && counter < max_iterations) {
+  while (Less(tol, err) && counter < max_iterations) {
     const double x = e.x;
     const double dfx = DfSide(R, d_exponent, pw, x) + DfSide(L, d_exponent, pw, x);
     const double offset = Div(fx, dfx);
     const double next = x - offset;
     e = EvalF(L, R, gm1, exponent, pw,
-              ((next - next) != (next - next) || next < 0.0) ? 0.5 * x : next);
+              ((next - next) != (next - next) || Negative(next)) ? 0.5 * x : next);
     fx = e.fR + e.fL + du;
     err = fabs(fx);
     counter += 1;
   }
   iterations = counter;
-  converged = !(err > tol);
+  converged = !Less(tol, err);
   return e;
 }
 
@@ -176,22 +216,22 @@ __device__ __forceinline__ Star ComputeMiddleState(const exact::Gas& eq,
                                                    const exact::Complete<D>& right, int dir,
                                                    const Options& opt) {
   const double g = eq.gamma;
-  const double gp1 = g + 1.0;
-  const double gm1 = g - 1.0;
+  const double gp1 = opt.c.gp1;
+  const double gm1 = opt.c.gm1;
   SideFn L, R;
   L.rho = left.rho;
   L.p = left.p;
   L.a = left.c;
   L.A = Div(2.0, gp1 * L.rho);
-  L.B = gm1 / gp1 * L.p;
+  L.B = opt.c.g_ratio * L.p;
   R.rho = right.rho;
   R.p = right.p;
   R.a = right.c;
   R.A = Div(2.0, gp1 * R.rho);
-  R.B = gm1 / gp1 * R.p;
-  const double exponent = 0.5 * gm1 / g;
-  const double d_exponent = -0.5 * gp1 / g;
-  const Powers pw(opt.root_n);
+  R.B = opt.c.g_ratio * R.p;
+  const double exponent = opt.c.exponent;
+  const double d_exponent = opt.c.d_exponent;
+  const Powers pw = PowersOf(opt.c);
   const double uL = Div(left.m[dir], left.rho);
   const double uR = Div(right.m[dir], right.rho);
   const double du = uR - uL;
@@ -201,7 +241,7 @@ __device__ __forceinline__ Star ComputeMiddleState(const exact::Gas& eq,
   if (opt.guess == kGuessMean) {
     x0 = 0.5 * (L.p + R.p);
   } else {
-    const double pv = PvrsTrGuess(pw, g, L.rho, uL, L.p, L.a, R.rho, uR, R.p, R.a);
+    const double pv = PvrsTrGuess(opt, g, L.rho, uL, L.p, L.a, R.rho, uR, R.p, R.a);
     x0 = pv;
     // Cost-aware use of the learned start: the network costs about one
     // Newton step (its 5-64-64-1 FP32 multiply-adds against two FP64 roots
@@ -284,16 +324,16 @@ template <int D>
 __device__ __forceinline__ double SignalMaxSpeed(const exact::Gas& eq,
                                                  const exact::Complete<D>& left,
                                                  const exact::Complete<D>& right, int dir,
-                                                 double pM) {
+                                                 double pM, const Options& opt) {
   const double g = eq.gamma;
-  const double gp1 = g + 1.0;
-  const double gm1 = g - 1.0;
+  const double gp1 = opt.c.gp1;
+  const double gm1 = opt.c.gm1;
   const double uL = Div(left.m[dir], left.rho);
   const double aL = left.c;
   const double pL = left.p;
   const double pL_ratio = Div(pM, pL);
   double s0, s1;
-  if (pM > pL) {
+  if (Less(pL, pM)) {
     s0 = uL - aL * Sqrt(Div(gp1 * pL_ratio + gm1, 2.0 * g));
   } else {
     s0 = uL - aL;
@@ -302,15 +342,15 @@ __device__ __forceinline__ double SignalMaxSpeed(const exact::Gas& eq,
   const double aR = right.c;
   const double pR = right.p;
   const double pR_ratio = Div(pM, pR);
-  if (pM > pR) {
+  if (Less(pR, pM)) {
     s1 = uR + aR * Sqrt(Div(gp1 * pR_ratio + gm1, 2.0 * g));
   } else {
     s1 = uR + aR;
   }
   double s = 0.0;
   const double a0 = fabs(s0), a1 = fabs(s1);
-  s = (s < a0) ? a0 : s;  // std::max(x, |y|)
-  s = (s < a1) ? a1 : s;
+  s = Less(s, a0) ? a0 : s;  // std::max(x, |y|)
+  s = Less(s, a1) ? a1 : s;
   return s;
 }
 
@@ -320,10 +360,11 @@ __device__ __forceinline__ void Sample(const exact::Gas& eq, exact::Complete<D>&
                                        const exact::Complete<D>& left,
                                        const exact::Complete<D>& right, int dir, double pM,
                                        double uM, const Options& opt) {
-  const Powers pw(opt.root_n);
+  const Powers pw = PowersOf(opt.c);
   const double g = eq.gamma;
-  const double gp1 = g + 1.0;
-  const double gm1 = g - 1.0;
+  const double gp1 = opt.c.gp1;
+  const double gm1 = opt.c.gm1;
+  const double g_ratio = opt.c.g_ratio;
   auto set_momentum = [dir](exact::Complete<D>& s, double momentum,
                             const exact::Complete<D>& side) {
     if constexpr (D == 1) {
@@ -340,15 +381,14 @@ __device__ __forceinline__ void Sample(const exact::Gas& eq, exact::Complete<D>&
     s.E = rhoE_internal + rhoE_kin;
     s.c = Sqrt(Div(eq.gamma * s.p, s.rho));
   };
-  if (0.0 <= uM) {
+  if (NotNegative(uM)) {
     const double uL = Div(left.m[dir], left.rho);
     const double aL = left.c;
     const double pL = left.p;
     const double p_ratio = Div(pM, pL);
-    const double g_ratio = gm1 / gp1;
-    if (pM > pL) {
+    if (Less(pL, pM)) {
       const double shock_speed = uL - aL * Sqrt(Div(gp1 * p_ratio + gm1, 2.0 * g));
-      if (shock_speed < 0.0) {
+      if (Negative(shock_speed)) {
         state.rho = Div(left.rho * (p_ratio + g_ratio), g_ratio * p_ratio + 1.0);
         set_momentum(state, state.rho * uM, left);
         state.p = pM;
@@ -357,21 +397,21 @@ __device__ __forceinline__ void Sample(const exact::Gas& eq, exact::Complete<D>&
         state = left;
       }
     } else {
-      const double aM = aL * pw.Z(p_ratio, gm1 / (2.0 * g));
+      const double aM = aL * pw.Z(p_ratio, opt.c.z);
       const double shock_speed_TL = uM - aM;
       const double shock_speed_HL = uL - aL;
-      if (0.0 < shock_speed_HL) {
+      if (Positive(shock_speed_HL)) {
         state = left;
-      } else if (shock_speed_TL < 0.0) {
-        state.rho = left.rho * pw.InvGamma(p_ratio, 1 / g);
+      } else if (Negative(shock_speed_TL)) {
+        state.rho = left.rho * pw.InvGamma(p_ratio, opt.c.inv_g);
         set_momentum(state, state.rho * uM, left);
         state.p = pM;
         from_prim(state);
       } else {
-        state.rho = left.rho * pw.N2(2.0 / gp1 + Div(g_ratio * uL, aL), 2.0 / gm1);
-        const double u = 2.0 / gp1 * (aL + 0.5 * gm1 * uL);
+        state.rho = left.rho * pw.N2(opt.c.two_gp1 + Div(g_ratio * uL, aL), 2.0 / gm1);
+        const double u = opt.c.two_gp1 * (aL + 0.5 * gm1 * uL);
         set_momentum(state, state.rho * u, left);
-        state.p = pL * pw.N(2.0 / gp1 + Div(g_ratio * uL, aL), 2.0 * g / gm1);
+        state.p = pL * pw.N(opt.c.two_gp1 + Div(g_ratio * uL, aL), 2.0 * g / gm1);
         from_prim(state);
       }
     }
@@ -380,10 +420,9 @@ __device__ __forceinline__ void Sample(const exact::Gas& eq, exact::Complete<D>&
     const double aR = right.c;
     const double pR = right.p;
     const double p_ratio = Div(pM, pR);
-    const double g_ratio = gm1 / gp1;
-    if (pM > pR) {
+    if (Less(pR, pM)) {
       const double shock_speed = uR + aR * Sqrt(Div(gp1 * p_ratio + gm1, 2.0 * g));
-      if (0.0 < shock_speed) {
+      if (Positive(shock_speed)) {
         state.rho = Div(right.rho * (p_ratio + g_ratio), g_ratio * p_ratio + 1.0);
         set_momentum(state, state.rho * uM, right);
         state.p = pM;
@@ -392,21 +431,21 @@ __device__ __forceinline__ void Sample(const exact::Gas& eq, exact::Complete<D>&
         state = right;
       }
     } else {
-      const double aM = aR * pw.Z(p_ratio, gm1 / (2.0 * g));
+      const double aM = aR * pw.Z(p_ratio, opt.c.z);
       const double shock_speed_TR = uM + aM;
       const double shock_speed_HR = uR + aR;
-      if (shock_speed_HR <= 0.0) {
+      if (NotPositive(shock_speed_HR)) {
         state = right;
-      } else if (shock_speed_TR >= 0.0) {
-        state.rho = right.rho * pw.InvGamma(p_ratio, 1 / g);
+      } else if (NotNegative(shock_speed_TR)) {
+        state.rho = right.rho * pw.InvGamma(p_ratio, opt.c.inv_g);
         set_momentum(state, state.rho * uM, right);
         state.p = pM;
         from_prim(state);
       } else {
-        state.rho = right.rho * pw.N2(2.0 / gp1 - Div(g_ratio * uR, aR), 2.0 / gm1);
-        const double u = 2.0 / gp1 * (-aR + 0.5 * gm1 * uR);
+        state.rho = right.rho * pw.N2(opt.c.two_gp1 - Div(g_ratio * uR, aR), 2.0 / gm1);
+        const double u = opt.c.two_gp1 * (-aR + 0.5 * gm1 * uR);
         set_momentum(state, state.rho * u, right);
-        state.p = pR * pw.N(2.0 / gp1 - Div(g_ratio * uR, aR), 2.0 * g / gm1);
+        state.p = pR * pw.N(opt.c.two_gp1 - Div(g_ratio * uR, aR), 2.0 * g / gm1);
         from_prim(state);
       }
     }
@@ -423,7 +462,7 @@ __device__ __forceinline__ Star GodunovFlux(const exact::Gas& eq, double* nf,
                                             const Options& opt) {
   exact::Complete<D> sol = L;
   Star st{0.0, 0.0, 0, 1, 0};
-  if (0.0 < L.rho && 0.0 < R.rho) {
+  if (Positive(L.rho) && Positive(R.rho)) {
     st = ComputeMiddleState<D>(eq, L, R, dir, opt);
     Sample<D>(eq, sol, L, R, dir, st.p, st.u, opt);
   }

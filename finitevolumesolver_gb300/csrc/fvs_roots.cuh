@@ -5,6 +5,7 @@
 #include <cmath>
 
 #include "fvs_convert.cuh"
+#include "fvs_ieee64.cuh"
 
 namespace fvs {
 namespace riemann {
@@ -15,9 +16,10 @@ namespace riemann {
 // r = x^(-1/n): x^z = x r^(n-1), x^(z-1) = x^(-(gamma+1)/(2 gamma)) = r^(n-1),
 // x^(1/gamma) = x^((n-2)/n) = x r^2, and the integer powers b^(n-2) =
 // b^(2/(gamma-1)) and b^n = b^(2 gamma/(gamma-1)).  r is Newton's method for
-// r^-n = x, r <- r (1 + (1 - x r^n) / n) (no division), from an FP32 estimate
-// (relative error ~1e-6): two steps square the error twice, below FP64
-// rounding.  That is ~20 FP64 operations where pow() evaluates a logarithm
+// r^-n = x with its second-order term, r <- r (1 + e / n + (n + 1) e^2 / (2 n^2)),
+// e = 1 - x r^n (no division), from an FP32 estimate whose relative error is
+// at most 2e-5 / n: one step cubes the error to n^2 / 3 of it, below FP64
+// rounding.  That is ~11 FP64 operations where pow() evaluates a logarithm
 // and an exponential in extended precision; the results are within 2e-14
 // relative of pow() with the solver's FP64 exponents, which are themselves
 // roundings of the rationals above (tests/cpp/root_check.cu).  Other gammas,
@@ -48,26 +50,30 @@ __host__ __device__ __forceinline__ double IPow(double b, int k) {
 
 struct Powers {
   int n;
-  double inv_n;
-  __host__ __device__ explicit Powers(int root_n) : n(root_n), inv_n(root_n > 0 ? 1.0 / root_n : 0.0) {}
-  // true where x^(-1/n) replaces pow()
-  __host__ __device__ bool Fast(double x) const { return n > 0 && x > 1e-30 && x < 1e30; }
+  double inv_n, second;  // 1 / n and (n + 1) / (2 n^2)
+  __host__ __device__ Powers() : n(0), inv_n(0.0), second(0.0) {}
+  __host__ __device__ explicit Powers(int root_n)
+      : n(root_n),
+        inv_n(root_n > 0 ? 1.0 / root_n : 0.0),
+        second(0.5 * (root_n + 1) * inv_n * inv_n) {}
+  // true where x^(-1/n) replaces pow(): 1e-30 < x < 1e30, compared as the bit
+  // patterns that order like positive numbers
+  __host__ __device__ bool Fast(double x) const {
+    const uint64_t lo = ieee64::Bits(1e-30), hi = ieee64::Bits(1e30);
+    return n > 0 && ieee64::Bits(x) - (lo + 1) < hi - lo - 1;
+  }
   // x^(-1/n) for Fast(x)
   __host__ __device__ double RecipRoot(double x) const {
 #ifdef __CUDA_ARCH__
     // the estimate's conversions on the integer pipe (the FP64 pipe is the
     // solver's bottleneck)
     const float xf = DoubleToFloatBits(x);
-    double r = FloatToDoubleBits(exp2f(-__log2f(xf) * static_cast<float>(inv_n)));
+    const double r = FloatToDoubleBits(exp2f(-__log2f(xf) * static_cast<float>(inv_n)));
 #else
-    double r = static_cast<double>(exp2f(-log2f(static_cast<float>(x)) * static_cast<float>(inv_n)));
+    const double r = static_cast<double>(exp2f(-log2f(static_cast<float>(x)) * static_cast<float>(inv_n)));
 #endif
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-      const double e = fma(-x, IPow(r, n), 1.0);
-      r = fma(r, e * inv_n, r);
-    }
-    return r;
+    const double e = fma(-x, IPow(r, n), 1.0);
+    return fma(r * e, fma(second, e, inv_n), r);
   }
   // x^z (z = the caller's (gamma-1)/(2 gamma) expression, for pow())
   __host__ __device__ double Z(double x, double z) const {
