@@ -94,8 +94,34 @@ template <class T> __device__ __forceinline__ void AddMomentum(T* f, int d, T x)
     f[2] += x;
 }
 
-template <class T> __device__ __forceinline__ T PMinT(T a, T b) { return a < b ? a : b; }
-template <class T> __device__ __forceinline__ T PMaxT(T a, T b) { return a > b ? a : b; }
+// FP64 comparisons on the integer pipes (one takes the FP64 pipe as long as an
+// addition).
+template <class T> __device__ __forceinline__ bool LessT(T a, T b) {
+  if constexpr (sizeof(T) == 8) return ieee64::Less(a, b);
+  else return a < b;
+}
+template <class T> __device__ __forceinline__ bool PositiveT(T a) {
+  if constexpr (sizeof(T) == 8) return ieee64::Positive(a);
+  else return a > T(0);
+}
+template <class T> __device__ __forceinline__ T PMinT(T a, T b) { return LessT(a, b) ? a : b; }
+template <class T> __device__ __forceinline__ T PMaxT(T a, T b) { return LessT(b, a) ? a : b; }
+// PMinT(a, 0) and PMaxT(a, 0)
+template <class T> __device__ __forceinline__ T PMin0T(T a) {
+  if constexpr (sizeof(T) == 8) return exact::PMin0(a);
+  else return a < T(0) ? a : T(0);
+}
+template <class T> __device__ __forceinline__ T PMax0T(T a) {
+  return PositiveT(a) ? a : T(0);
+}
+// (gamma - 1) (roeH - 0.5 roeU roeU); FP64: the half folded into an FMA
+// (exact::RoeA2), the same bits
+template <class T, class G> __device__ __forceinline__ T RoeA2T(const G& eq, T roeU, T roeH) {
+  if constexpr (sizeof(T) == 8)
+    return (eq.gamma - 1.0) * __fma_rn(-0.5, __dmul_rn(roeU, roeU), roeH);
+  else
+    return (eq.gamma - T(1)) * (roeH - T(0.5) * roeU * roeU);
+}
 
 template <class T, class M = CcIeee> __device__ __forceinline__ GasT<T, M> MakeGasT(double gamma) {
   GasT<T, M> g;
@@ -151,7 +177,7 @@ __device__ __forceinline__ void EinfeldtT(const GasT<T, M>& eq, const C2T<T>& L,
   const T hL = M::Div(L.E + L.p, rhoL);
   const T hR = M::Div(R.E + R.p, rhoR);
   const T roeH = (hL * sqRhoL + hR * sqRhoR) * oosqRhoSum;
-  const T roeA2 = (eq.gamma - T(1)) * (roeH - T(0.5) * roeU * roeU);
+  const T roeA2 = RoeA2T<T>(eq, roeU, roeH);
   const T roeA = M::Sqrt(roeA2);
   sL = PMinT(uL - L.c, roeU - roeA);
   sR = PMaxT(roeU + roeA, uR + R.c);
@@ -161,7 +187,7 @@ __device__ __forceinline__ void EinfeldtT(const GasT<T, M>& eq, const C2T<T>& L,
 template <class T, class M>
 __device__ __forceinline__ void CompleteMasked(const GasT<T, M>& eq, C2T<T>& q, const T* u,
                                                bool mask) {
-  if (!(mask && u[0] > T(0))) {
+  if (!(mask && PositiveT(u[0]))) {
     q.rho = T(0);
     q.m[0] = T(0);
     q.m[1] = T(0);
@@ -176,7 +202,7 @@ __device__ __forceinline__ void CompleteMasked(const GasT<T, M>& eq, C2T<T>& q, 
 // Flux masked by `rho > 0` (PerfectGas.cpp:79-93, mask true).
 template <class M, class T>
 __device__ __forceinline__ void FluxMasked(T* f, const C2T<T>& q, int dir) {
-  const T rho = (q.rho > T(0)) ? q.rho : T(1);
+  const T rho = PositiveT(q.rho) ? q.rho : T(1);
   const T velocity = M::Div(Sel(q.m, dir), rho);
   f[0] = Sel(q.m, dir);
   f[1] = velocity * q.m[0];
@@ -212,7 +238,7 @@ __device__ __forceinline__ void EinfeldtMasked(const GasT<T, M>& eq, const C2T<T
   }
   const T roeU = uL * wL + uR * wR;
   const T roeH = hL * wL + hR * wR;
-  const T roeA2 = (eq.gamma - T(1)) * (roeH - T(0.5) * roeU * roeU);
+  const T roeA2 = RoeA2T<T>(eq, roeU, roeH);
   const T roeA = M::Sqrt(roeA2);
   sL = PMinT(uL - L.c, roeU - roeA);
   sR = PMaxT(roeU + roeA, uR + R.c);
@@ -227,6 +253,12 @@ __device__ __forceinline__ void PredictMasked(const GasT<T, M>& eq, C2T<T>& recL
   T uL[4], uR[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
+    if constexpr (sizeof(T) == 8) {
+      const T hs = smask ? exact::HalfSlope(limiter, q0[k], q1[k], q2[k]) : 0.0;
+      uL[k] = q1[k] - hs;
+      uR[k] = q1[k] + hs;
+      continue;
+    }
     const T sL = smask ? q1[k] - q0[k] : T(0);
     const T sR = smask ? q2[k] - q1[k] : T(0);
     T slope;
@@ -271,8 +303,8 @@ __device__ __forceinline__ void HllMasked(const GasT<T, M>& eq, T* nf, const C2T
   FluxMasked<M>(fR, R, dir);
   const T qL[4] = {L.rho, L.m[0], L.m[1], L.E};
   const T qR[4] = {R.rho, R.m[0], R.m[1], R.E};
-  const T sL = PMinT(s0, T(0));
-  const T sR = PMaxT(s1, T(0));
+  const T sL = PMin0T(s0);
+  const T sR = PMax0T(s1);
   const T sLsR = sL * sR;
   const T ds = sR - sL;
   if constexpr (M::kFast) {
@@ -715,7 +747,7 @@ template <class T> constexpr size_t KbnTileSmemBytes(int dir) {
          (dir == 0 ? sizeof(T) * 4 * (kTileCells + 1) * kTilePitch : 0);
 }
 
-template <class T, class M>
+template <class T, class M, int dir>
 __global__ void __launch_bounds__(256, 3) KbnRegularTileKernel(CcSweepArgs a) {
   constexpr int kL = kTileLines, kNSeg = kTileSegs, kC = kTileCells, kH = kTileHalo,
                 kP = kTilePitch;
@@ -727,7 +759,6 @@ __global__ void __launch_bounds__(256, 3) KbnRegularTileKernel(CcSweepArgs a) {
   T (*sf)[kC + 1][kP] = reinterpret_cast<T (*)[kC + 1][kP]>(
       tile_smem + ((sizeof(T) * 4 * kH * kP + size_t(kH) * kP + 15) / 16) * 16);
   const CcGeom& g = a.s.g;
-  const int dir = a.dir;
   const int nd = dir == 0 ? g.nx : g.ny;
   const int nt = dir == 0 ? g.ny : g.nx;
   const int ntl = g.NTiles(dir);
@@ -847,9 +878,10 @@ __global__ void __launch_bounds__(256, 3) KbnRegularTileKernel(CcSweepArgs a) {
                   d = DiffToDouble(f_prev[k], f[k]);
                 else
                   d = Widen(f_prev[k] + T(0)) - Widen(f[k] + T(0));
-                a.out[k * cs + o] = prev + dt_dx * d;
+                const double v = prev + dt_dx * d;
+                a.out[k * cs + o] = v;
+                if (k == 0 && __double_as_longlong(v) <= 0) status |= kStatusNonPositiveDensity;
               }
-              if (__double_as_longlong(a.out[o]) <= 0) status |= kStatusNonPositiveDensity;
             } else {
 #pragma unroll
               for (int k = 0; k < 4; ++k) a.out[k * cs + o] = 0.0;
@@ -893,9 +925,10 @@ __global__ void __launch_bounds__(256, 3) KbnRegularTileKernel(CcSweepArgs a) {
           d = DiffToDouble(sf[k][cell][line], sf[k][cell + 1][line]);
         else
           d = Widen(sf[k][cell][line] + T(0)) - Widen(sf[k][cell + 1][line] + T(0));
-        a.out[k * cs + o] = prev + dt_dx * d;
+        const double v = prev + dt_dx * d;
+        a.out[k * cs + o] = v;
+        if (k == 0 && __double_as_longlong(v) <= 0) status |= kStatusNonPositiveDensity;
       }
-      if (__double_as_longlong(a.out[o]) <= 0) status |= kStatusNonPositiveDensity;
     }
   }
   const double smax_d = static_cast<double>(smax);
@@ -911,10 +944,9 @@ __global__ void __launch_bounds__(256, 3) KbnRegularTileKernel(CcSweepArgs a) {
 // fvs_sweep.cuh), none in a step's first sweep.  Tiles without a regular
 // cell only write their covered cells (0).  The tile flag is the warp's, so
 // the control flow is warp-uniform.
-template <class T, class M, int kMinBlocks>
+template <class T, class M, int kMinBlocks, int dir>
 __global__ void __launch_bounds__(128, kMinBlocks) KbnRegularSweepKernel(CcSweepArgs a) {
   const CcGeom& g = a.s.g;
-  const int dir = a.dir;
   const int nd = dir == 0 ? g.nx : g.ny;
   const int nt = dir == 0 ? g.ny : g.nx;
   const int64_t t64 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -996,6 +1028,7 @@ __global__ void __launch_bounds__(128, kMinBlocks) KbnRegularSweepKernel(CcSweep
       bool ok_prev = false;
       bool have_prev = false;
       int cls_prev = CellClassAt(g, dir, t, j0 - 1);
+      int cls_next = CellClassAt(g, dir, t, j0);  // loaded one face ahead of its use
       for (int j = j0 - 1; j <= j1; ++j) {
         finish(dn, fl_dn, up);
         if (j + 2 <= j1 + 1) fl_dn = fetch(j + 2, dn);
@@ -1016,7 +1049,8 @@ __global__ void __launch_bounds__(128, kMinBlocks) KbnRegularSweepKernel(CcSweep
           CompleteMasked(eq, q, uc, true);
         }
         if (j >= j0) {
-          const int cls = CellClassAt(g, dir, t, j);
+          const int cls = cls_next;
+          cls_next = CellClassAt(g, dir, t, j + 1);
           const bool count = cls == kCcRegular || cls_prev == kCcRegular;
           if constexpr (kScreen) {
             if (!skip_cfl) {
@@ -1072,9 +1106,10 @@ __global__ void __launch_bounds__(128, kMinBlocks) KbnRegularSweepKernel(CcSweep
                   d = DiffToDouble(f_prev[c], f[c]);
                 else
                   d = Widen(f_prev[c] + T(0)) - Widen(f[c] + T(0));
-                a.out[c * cs + o] = prev + dt_dx * d;
+                const double v = prev + dt_dx * d;
+                a.out[c * cs + o] = v;
+                if (c == 0 && __double_as_longlong(v) <= 0) status |= kStatusNonPositiveDensity;
               }
-              if (__double_as_longlong(a.out[o]) <= 0) status |= kStatusNonPositiveDensity;
             } else {
 #pragma unroll
               for (int c = 0; c < 4; ++c) a.out[c * cs + o] = 0.0;
@@ -1197,22 +1232,29 @@ cudaError_t LaunchKbnSweep(const CcSweepArgs& a, bool band, cudaStream_t s) {
     if (n > 0) KbnBandKernel<T, M><<<unsigned((n + 63) / 64), 64, 0, s>>>(a);
     return cudaGetLastError();
   }
-  if (sizeof(T) == 4 && !(a.dir == 1 && a.occupancy == 10)) {
+  bool tiles = false;
+  if constexpr (sizeof(T) == 4) {
     // mixed: tiles staged in shared memory, 32 lines x 64 cells per block
+    tiles = !(a.dir == 1 && a.occupancy == 10);
     const int64_t blocks = int64_t(a.s.g.NGroups(a.dir)) * ((a.s.g.NTiles(a.dir) + 7) / 8);
-    static bool attr_set = false;
-    if (!attr_set) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(KbnRegularTileKernel<T, M>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(KbnTileSmemBytes<T>(0) + 16));
+    auto launch = [&](auto kernel, bool* attr_set) {
+      if (!*attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(KbnTileSmemBytes<T>(0) + 16));
+        if (e != cudaSuccess) return e;
+        *attr_set = true;
+      }
+      if (blocks > 0) kernel<<<unsigned(blocks), 256, KbnTileSmemBytes<T>(a.dir) + 16, s>>>(a);
+      return cudaSuccess;
+    };
+    static bool attr_set[2] = {false, false};
+    if (tiles) {
+      const cudaError_t e = a.dir == 0 ? launch(KbnRegularTileKernel<T, M, 0>, &attr_set[0])
+                                       : launch(KbnRegularTileKernel<T, M, 1>, &attr_set[1]);
       if (e != cudaSuccess) return e;
-      attr_set = true;
     }
-    if (blocks > 0)
-      KbnRegularTileKernel<T, M>
-          <<<unsigned(blocks), 256, KbnTileSmemBytes<T>(a.dir) + 16, s>>>(a);
-  } else {
+  }
+  if (!tiles) {
     // FP64 flavours (bound by the FP64 pipe), and the mixed flavour's y
     // sweeps as launch variant 10: threads march runs of tiles, one
     // predictor per cell
@@ -1222,10 +1264,12 @@ cudaError_t LaunchKbnSweep(const CcSweepArgs& a, bool band, cudaStream_t s) {
     CcSweepArgs b = a;
     b.seg_len = seg;
     dim3 grid(unsigned((nt + block - 1) / block), unsigned((nd + seg - 1) / seg));
-    if constexpr (sizeof(T) == 4)
-      KbnRegularSweepKernel<T, M, 5><<<grid, block, 0, s>>>(b);
+    if constexpr (sizeof(T) == 4)  // y only
+      KbnRegularSweepKernel<T, M, 5, 1><<<grid, block, 0, s>>>(b);
+    else if (a.dir == 0)
+      KbnRegularSweepKernel<T, M, 3, 0><<<grid, block, 0, s>>>(b);
     else
-      KbnRegularSweepKernel<T, M, 3><<<grid, block, 0, s>>>(b);
+      KbnRegularSweepKernel<T, M, 3, 1><<<grid, block, 0, s>>>(b);
   }
   return cudaGetLastError();
 }
