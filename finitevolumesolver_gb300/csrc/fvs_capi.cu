@@ -660,9 +660,9 @@ cudaError_t EnqueueStep(fvs_solver* s, int start, int64_t cycle, int step_in_bat
     if (e != cudaSuccess) return e;
   }
   if (!stable_enqueued) {
-    // the pass's max slots start at zero (its screened speeds need it)
-    e = cudaMemsetAsync(s->ctrl->smax_stable, 0, sizeof(s->ctrl->smax_stable), s->stream);
-    if (e != cudaSuccess) return e;
+    // the pass's max slots start at zero (the run's control block, then
+    // EndStepKernel) or, in a restarted step, at the same state's maxima, as
+    // its screened speeds need them to
     e = LaunchStable(s, s->buf[start], s->ctrl->smax_stable, s->ctrl);
     if (e != cudaSuccess) return e;
   }
