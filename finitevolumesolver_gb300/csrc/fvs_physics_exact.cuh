@@ -189,9 +189,7 @@ enum Limiter : int { kVanLeer = 0, kMinMod = 1, kNoLimiter = 2, kNoGradient = 3 
 // Half the limited slope, what the predictor adds and subtracts.  Van Leer:
 // 0.5 ((2 sL sR) / (sL + sR)) has the bits of (sL sR) / (sL + sR) unless
 // sL sR leaves the range of ieee64's quotients.
-__device__ __forceinline__ double HalfSlope(int limiter, double qL, double qM, double qR) {
-  const double sL = qM - qL;
-  const double sR = qR - qM;
+__device__ __forceinline__ double HalfSlopeOf(int limiter, double sL, double sR) {
   if (limiter == kVanLeer) {
     const double c = sL * sR;
     const bool pos = ieee64::Positive(c);
@@ -210,23 +208,26 @@ __device__ __forceinline__ double HalfSlope(int limiter, double qL, double qM, d
   return 0.0;
 }
 
+__device__ __forceinline__ double HalfSlope(int limiter, double qL, double qM, double qR) {
+  return HalfSlopeOf(limiter, qM - qL, qR - qM);
+}
+
 // MUSCL-Hancock predictor of one cell: the Hancock-evolved states at its left
 // face (recL, the reference's rec_[1] when the cell is stencil[2]) and at its
 // right face (recR, rec_[0] when the cell is stencil[1]).  Computing both once
 // per cell gives bit-identical face states to the reference, which computes
 // each cell's predictor twice (once for each of its faces).
+// From the cell's state and its differences to the two neighbours.
 template <int D>
-__device__ __forceinline__ void MusclPredictBoth(const Gas& eq, Complete<D>& recL,
-                                                 Complete<D>& recR,
-                                                 const double* q0,
-                                                 const double* q1,
-                                                 const double* q2, int limiter,
+__device__ __forceinline__ void MusclPredictDiff(const Gas& eq, Complete<D>& recL,
+                                                 Complete<D>& recR, const double* q1,
+                                                 const double* sL, const double* sR, int limiter,
                                                  double lambda_half, int dir) {
   constexpr int K = D + 2;
   double uL[K], uR[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const double hs = HalfSlope(limiter, q0[k], q1[k], q2[k]);
+    const double hs = HalfSlopeOf(limiter, sL[k], sR[k]);
     uL[k] = q1[k] - hs;
     uR[k] = q1[k] + hs;
   }
@@ -245,6 +246,21 @@ __device__ __forceinline__ void MusclPredictBoth(const Gas& eq, Complete<D>& rec
   }
   CompleteFromCons<D>(eq, recR, b);
   CompleteFromCons<D>(eq, recL, a);
+}
+
+template <int D>
+__device__ __forceinline__ void MusclPredictBoth(const Gas& eq, Complete<D>& recL,
+                                                 Complete<D>& recR, const double* q0,
+                                                 const double* q1, const double* q2, int limiter,
+                                                 double lambda_half, int dir) {
+  constexpr int K = D + 2;
+  double sL[K], sR[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    sL[k] = q1[k] - q0[k];
+    sR[k] = q2[k] - q1[k];
+  }
+  MusclPredictDiff<D>(eq, recL, recR, q1, sL, sR, limiter, lambda_half, dir);
 }
 
 }  // namespace exact

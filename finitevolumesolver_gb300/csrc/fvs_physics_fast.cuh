@@ -253,9 +253,7 @@ __device__ __forceinline__ void HllFlux(const Gas<T>& eq, T* nf, const State<D, 
 // (2 sL sR / (sL + sR)) / 2 = sL sR / (sL + sR), the factors 2 and 1/2 being
 // exact they are left out.
 template <typename T>
-__device__ __forceinline__ T HalfSlope(int limiter, T qL, T qM, T qR) {
-  const T sL = qM - qL;
-  const T sR = qR - qM;
+__device__ __forceinline__ T HalfSlopeOf(int limiter, T sL, T sR) {
   if (limiter == 0) {  // van Leer
     const T c = sL * sR;
     if constexpr (kIsF64<T>) {
@@ -273,17 +271,17 @@ __device__ __forceinline__ T HalfSlope(int limiter, T qL, T qM, T qR) {
   return T(0);  // NoGradient
 }
 
-// MUSCL-Hancock predictor of one cell: its left-face and right-face states.
+// MUSCL-Hancock predictor of one cell: its left-face and right-face states,
+// from its state and its differences to the two neighbours.
 template <int D, typename T>
-__device__ __forceinline__ void PredictBoth(const Gas<T>& eq, State<D, T>& recL,
-                                            State<D, T>& recR, const T* q0, const T* q1,
-                                            const T* q2, int limiter, T lambda_half,
-                                            int dir) {
+__device__ __forceinline__ void PredictDiff(const Gas<T>& eq, State<D, T>& recL,
+                                            State<D, T>& recR, const T* q1, const T* sL,
+                                            const T* sR, int limiter, T lambda_half, int dir) {
   constexpr int K = D + 2;
   T uL[K], uR[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const T hs = HalfSlope<T>(limiter, q0[k], q1[k], q2[k]);
+    const T hs = HalfSlopeOf<T>(limiter, sL[k], sR[k]);
     uL[k] = q1[k] - hs;
     uR[k] = q1[k] + hs;
   }
@@ -299,6 +297,21 @@ __device__ __forceinline__ void PredictBoth(const Gas<T>& eq, State<D, T>& recL,
   }
   Prepare<D, T>(eq, recR, b, dir);
   Prepare<D, T>(eq, recL, a, dir);
+}
+
+template <int D, typename T>
+__device__ __forceinline__ void PredictBoth(const Gas<T>& eq, State<D, T>& recL,
+                                            State<D, T>& recR, const T* q0, const T* q1,
+                                            const T* q2, int limiter, T lambda_half,
+                                            int dir) {
+  constexpr int K = D + 2;
+  T sL[K], sR[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    sL[k] = q1[k] - q0[k];
+    sR[k] = q2[k] - q1[k];
+  }
+  PredictDiff<D, T>(eq, recL, recR, q1, sL, sR, limiter, lambda_half, dir);
 }
 
 // Cell data of the stable-dt estimate.

@@ -40,6 +40,13 @@ template <int D> struct ExactPolicy {
     exact::MusclPredictBoth<D>(eq, recL, recR, q0, q1, q2, limiter,
                                lambda_half, dir);
   }
+  static constexpr bool kDiff = true;  // the marching sweep carries differences
+  static __device__ __forceinline__ void PredictDiff(const Gas& eq, Rec& recL, Rec& recR,
+                                                     const double* q1, const double* sL,
+                                                     const double* sR, int limiter,
+                                                     double lambda_half, int dir) {
+    exact::MusclPredictDiff<D>(eq, recL, recR, q1, sL, sR, limiter, lambda_half, dir);
+  }
   using Stats = NoStats;
   static __device__ __forceinline__ void FluxOnly(const Gas& eq, double* F, const Rec& L,
                                                   const Rec& R, int dir) {

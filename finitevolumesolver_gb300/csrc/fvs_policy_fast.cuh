@@ -54,6 +54,13 @@ template <int D, typename T> struct FastBase {
                                                  int limiter, double lambda_half, int dir) {
     fast::PredictBoth<D, T>(eq, recL, recR, q0, q1, q2, limiter, T(lambda_half), dir);
   }
+  // FP64: the marching sweep carries differences
+  static constexpr bool kDiff = std::is_same_v<T, double>;
+  static __device__ __forceinline__ void PredictDiff(const Gas& eq, Rec& recL, Rec& recR,
+                                                     const T* q1, const T* sL, const T* sR,
+                                                     int limiter, double lambda_half, int dir) {
+    fast::PredictDiff<D, T>(eq, recL, recR, q1, sL, sR, limiter, T(lambda_half), dir);
+  }
   using Stats = NoStats;
   // the mixed flavour hands its FP32 fluxes to the sweep unwidened
   static constexpr bool kFloatFlux = sizeof(T) == 4;

@@ -175,6 +175,13 @@ template <class P>
 struct HasFluxOnly<P, std::void_t<decltype(&P::FluxOnly)>>
     : std::bool_constant<std::is_same_v<typename FluxOf<P>::type, double>> {};
 
+// Policies whose predictor takes a cell's differences to its neighbours
+// (PredictDiff): the marching sweep then carries the difference of the last
+// two cells instead of the cell before, and forms each difference once for the
+// two cells it belongs to (an FP64 subtraction per component less).
+template <class P, class = void> struct HasDiff : std::false_type {};
+template <class P> struct HasDiff<P, std::enable_if_t<P::kDiff>> : std::true_type {};
+
 template <class P, class F>
 __device__ __forceinline__ void SweepFluxOnly(const typename P::Gas& eq, F* flux,
                                               const typename P::Rec& L,
@@ -424,6 +431,11 @@ __device__ __forceinline__ void MarchSegment(const SweepArgs& a, Line& line, int
   P::ToCell(cc, dn);
   if (flip_cc) cc[1 + DIR] = -cc[1 + DIR];
   bool flip_dn = line.Load(dn, j0);
+  constexpr bool kDiff = HasDiff<P>::value;
+  if constexpr (kDiff) {  // cm: the difference cc - cm from here on
+#pragma unroll
+    for (int c = 0; c < K; ++c) cm[c] = cc[c] - cm[c];
+  }
   using FluxT = typename FluxOf<P>::type;
   typename P::Rec recR_prev;
   typename P::Wave w_prev;
@@ -456,7 +468,19 @@ __device__ __forceinline__ void MarchSegment(const SweepArgs& a, Line& line, int
           const bool need = !(ok && ok_prev && bound < thr);
           if (__any_sync(amask, need)) {
             // the whole warp evaluates (the same instructions as some lanes)
-            const typename P::Wave wl = have_prev ? w_prev : P::MakeWave(eq, cm, DIR);
+            typename P::Wave wl;
+            if (have_prev) {
+              wl = w_prev;
+            } else if constexpr (kDiff) {  // cell j - 1 again (an L1 hit)
+              double ud[K];
+              R um[K];
+              const bool flip = line.Load(ud, j - 1);
+              P::ToCell(um, ud);
+              if (flip) um[1 + DIR] = -um[1 + DIR];
+              wl = P::MakeWave(eq, um, DIR);
+            } else {
+              wl = P::MakeWave(eq, cm, DIR);
+            }
             w_prev = P::MakeWave(eq, cc, DIR);
             const R s = P::FaceMaxSpeed(eq, wl, w_prev);
             smax = s > smax ? s : smax;
@@ -476,7 +500,14 @@ __device__ __forceinline__ void MarchSegment(const SweepArgs& a, Line& line, int
     if (flip_dn) cp[1 + DIR] = -cp[1 + DIR];  // a reflective wall's image
     if (j + 2 <= j1 + 1) flip_dn = line.Load(dn, j + 2);
     typename P::Rec recL, recR;
-    P::Predict(eq, recL, recR, cm, cc, cp, a.limiter, lambda_half, DIR);
+    R dp[K];
+    if constexpr (kDiff) {
+#pragma unroll
+      for (int c = 0; c < K; ++c) dp[c] = cp[c] - cc[c];
+      P::PredictDiff(eq, recL, recR, cc, cm, dp, a.limiter, lambda_half, DIR);
+    } else {
+      P::Predict(eq, recL, recR, cm, cc, cp, a.limiter, lambda_half, DIR);
+    }
     typename P::Wave w{};
     if (!kFilter && !skip_cfl) w = P::MakeWave(eq, cc, DIR);
     if (j >= j0) {
@@ -513,7 +544,8 @@ __device__ __forceinline__ void MarchSegment(const SweepArgs& a, Line& line, int
     if constexpr (!kFilter) w_prev = w;
 #pragma unroll
     for (int c = 0; c < K; ++c) {
-      cm[c] = cc[c];
+      if constexpr (kDiff) cm[c] = dp[c];
+      else cm[c] = cc[c];
       cc[c] = cp[c];
     }
   }
