@@ -13,16 +13,16 @@ namespace fvs {
 //
 // double -> float: round to nearest (ties away from zero); magnitudes below
 // the FP32 normal range flush to a signed zero, above it saturate to inf.
+// The exponent moves with the mantissa: its low 8 bits land in the FP32 field
+// off by 128 (896 mod 256), which the addition of 2^30 takes out.
 __device__ __forceinline__ float DoubleToFloatBits(double x) {
-  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
-  const unsigned hi = static_cast<unsigned>(b >> 32);
-  const unsigned lo = static_cast<unsigned>(b);
-  const unsigned e = (hi >> 20) & 0x7FFu;
-  const unsigned sign = hi & 0x80000000u;
-  unsigned f = sign | ((e - 896u) << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-  f += (lo >> 28) & 1u;
-  f = (e <= 896u) ? sign : f;
-  f = (e >= 1151u) ? (sign | 0x7F800000u) : f;
+  const unsigned hi = static_cast<unsigned>(__double2hiint(x));
+  const unsigned lo = static_cast<unsigned>(__double2loint(x));
+  const unsigned mag = hi & 0x7FFFFFFFu, sign = hi & 0x80000000u;
+  unsigned f = __funnelshift_l(lo, hi, 3) + 0x40000000u + ((lo >> 28) & 1u);
+  f = (f & 0x7FFFFFFFu) | sign;
+  f = mag < (897u << 20) ? sign : f;
+  f = mag >= (1151u << 20) ? (sign | 0x7F800000u) : f;
   return __uint_as_float(f);
 }
 
@@ -60,6 +60,15 @@ __host__ __device__ __forceinline__ double DoubleFromBits(unsigned long long b) 
 #endif
 }
 
+// x >> s, 0 for s outside [0, 31].
+__host__ __device__ __forceinline__ unsigned ShiftRightClamped(unsigned x, int s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_rc(x, 0u, static_cast<unsigned>(s));
+#else
+  return static_cast<unsigned>(s) > 31u ? 0u : x >> s;
+#endif
+}
+
 // a - b of two FP32 numbers as an FP64 number, without the FP64 pipe.
 // Knuth's TwoSum in FP32 splits the exact difference into s + e with
 // s = fl32(a - b) and |e| <= ulp32(s) / 2, so e's exponent is at least 24
@@ -92,8 +101,9 @@ __host__ __device__ __forceinline__ double DiffToDouble(float a, float b) {
   // two s into the binade below: k = m_e 2^(5 - shift)
   const int finer = (shrink && (sb & 0x7FFFFFu) == 0u) ? 1 : 0;
   const int shift = es - ee - 24 - finer;  // >= 0 for a nonzero normal e
-  unsigned k = (((eb & 0x7FFFFFu) | 0x800000u) << 5) >> (shift & 31);
-  k = (ee == 0 || shift < 0 || shift > 31) ? 0u : k;
+  // (a shift outside 0..31 leaves 0)
+  unsigned k = ShiftRightClamped(((eb & 0x7FFFFFu) | 0x800000u) << 5, shift);
+  k = ee == 0 ? 0u : k;
   bits = shrink ? bits - k : bits + k;
   if (es == 0) bits = static_cast<unsigned long long>(sign) << 32;
   if (es == 255)
