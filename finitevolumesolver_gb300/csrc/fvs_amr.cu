@@ -449,13 +449,18 @@ int Build(fvs_amr* a) {
     for (auto& kv : h)
       Lv.hist += std::to_string(kv.first.first) + "x" + std::to_string(kv.first.second) + ":" +
                  std::to_string(kv.second) + ",";
+    // launch shapes of an untuned solver: the lanes along the rows (mixed: in
+    // x), where one thread per row gave a level of 65 k cells 60 warps (fast
+    // FP64 sweep 0.58 ms, now 20 us); mixed y columns split until the level
+    // has 64 k threads (four steps of a 0.6 M-cell mixed set 7.9 -> 2.9 ms)
     for (int d = 0; d < 2; ++d) {
-      Lv.grid[d] = std::max(1, std::min((Lv.nsegs[d][0] + 127) / 128, a->sms * 4));
-      // FP64 levels start with the lanes along the rows (a 65 k-cell level's
-      // sweep: 0.58 ms marching one thread per row, 20 us so)
-      if (a->m.precision != FVS_MIXED) {
+      if (d == 0 || a->m.precision != FVS_MIXED) {
         Lv.split[d] = kSplits;
         Lv.grid[d] = static_cast<int>(std::min<int64_t>((Lv.RowWarps(d) + 3) / 4, a->sms * 64));
+      } else {
+        while (Lv.split[d] + 1 < kSplits && Lv.nsegs[d][Lv.split[d]] < 65536) ++Lv.split[d];
+        Lv.block[d] = 64;
+        Lv.grid[d] = std::max(1, std::min((Lv.nsegs[d][Lv.split[d]] + 63) / 64, a->sms * 16));
       }
     }
   }
