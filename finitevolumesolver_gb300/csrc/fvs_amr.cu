@@ -107,6 +107,10 @@ struct fvs_amr {
   int nsweeps = 0;
   double* tune_dt = nullptr;
   cudaStream_t stream = nullptr;
+  // what the start of a step can do beside the x max-speed passes (backups, y
+  // passes), forked from and joined back into `stream`
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int64_t cycle = 0;
   double t = 0.0;
@@ -119,6 +123,9 @@ struct fvs_amr {
       if (g) cudaGraphExecDestroy(g);
     for (void* p : allocations) cudaFree(p);
     if (ctrl_host) cudaFreeHost(ctrl_host);
+    if (ev_fork) cudaEventDestroy(ev_fork);
+    if (ev_join) cudaEventDestroy(ev_join);
+    if (side) cudaStreamDestroy(side);
     if (stream) cudaStreamDestroy(stream);
   }
   template <class T> cudaError_t Alloc(T** p, size_t count) {
@@ -544,7 +551,7 @@ cudaError_t LaunchSweep(fvs_amr* a, int l, int d, const double* in, double* out,
   }
 }
 
-cudaError_t LaunchMaxSpeed(fvs_amr* a, int l, int d) {
+cudaError_t LaunchMaxSpeed(fvs_amr* a, int l, int d, cudaStream_t stream) {
   const LevelHost& Lv = a->L[size_t(l)];
   MaxSpeedArgs s{};
   s.in = Lv.A;
@@ -565,11 +572,11 @@ cudaError_t LaunchMaxSpeed(fvs_amr* a, int l, int d) {
       1, std::min<int64_t>((threads + block - 1) / block, int64_t(a->sms) * 16)));
   switch (a->m.precision) {
   case FVS_FP64_EXACT:
-    return LaunchPatchMaxSpeedExact(d, s, grid, block, a->stream);
+    return LaunchPatchMaxSpeedExact(d, s, grid, block, stream);
   case FVS_FP64_FAST:
-    return LaunchPatchMaxSpeedFast(d, s, grid, block, a->stream);
+    return LaunchPatchMaxSpeedFast(d, s, grid, block, stream);
   default:
-    return LaunchPatchMaxSpeedMixed(d, s, grid, block, a->stream);
+    return LaunchPatchMaxSpeedMixed(d, s, grid, block, stream);
   }
 }
 
@@ -586,6 +593,17 @@ LevelDx Dx(const fvs_amr* a) {
   LevelDx dx{};
   for (int l = 0; l < a->nlevels; ++l) dx.dx[l] = a->L[size_t(l)].dx;
   return dx;
+}
+
+// The side stream starts behind the main one's work so far; the main one
+// waits for the side stream's.
+cudaError_t Fork(fvs_amr* a) {
+  const cudaError_t e = cudaEventRecord(a->ev_fork, a->stream);
+  return e == cudaSuccess ? cudaStreamWaitEvent(a->side, a->ev_fork, 0) : e;
+}
+cudaError_t Join(fvs_amr* a) {
+  const cudaError_t e = cudaEventRecord(a->ev_join, a->side);
+  return e == cudaSuccess ? cudaStreamWaitEvent(a->stream, a->ev_join, 0) : e;
 }
 
 cudaError_t AdvanceLevel(fvs_amr* a, int l, int parity, int sub, int& counter) {
@@ -620,30 +638,37 @@ cudaError_t AdvanceLevel(fvs_amr* a, int l, int parity, int sub, int& counter) {
   }
   if (l + 1 < nl) {
     const LevelHost& F = a->L[size_t(l + 1)];
-    if ((e = LaunchReflux(Lv.A, int32_t(Lv.ncells), a->reg, F.reflux, F.nreflux, a->signs,
-                          Lv.dx, a->stream)) != cudaSuccess)
-      return e;
-    if ((e = LaunchAverageDown(Lv.A, int32_t(Lv.ncells), F.A, int32_t(F.ncells), F.avg, F.navg,
-                               a->stream)) != cudaSuccess)
-      return e;
+    // side by side: the refluxed cells lie outside the fine level's footprint,
+    // the averaged ones under it
+    e = Fork(a);
+    if (e == cudaSuccess)
+      e = LaunchAverageDown(Lv.A, int32_t(Lv.ncells), F.A, int32_t(F.ncells), F.avg, F.navg,
+                            a->side);
+    if (e == cudaSuccess)
+      e = LaunchReflux(Lv.A, int32_t(Lv.ncells), a->reg, F.reflux, F.nreflux, a->signs, Lv.dx,
+                       a->stream);
+    if (e == cudaSuccess) e = Join(a);
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
 cudaError_t EnqueueStep(fvs_amr* a, int parity) {
-  cudaError_t e;
-  for (int l = 0; l < a->nlevels; ++l) {
-    const LevelHost& Lv = a->L[size_t(l)];
-    e = cudaMemcpyAsync(Lv.backup, Lv.A, size_t(Lv.ncells) * kComp * sizeof(double),
-                        cudaMemcpyDeviceToDevice, a->stream);
-    if (e != cudaSuccess) return e;
-  }
-  e = cudaMemsetAsync(&a->ctrl->smax_stable[0][0], 0,
+  cudaError_t e =
+      cudaMemsetAsync(&a->ctrl->smax_stable[0][0], 0,
                       sizeof(a->ctrl->smax_stable) + sizeof(a->ctrl->smax_sweep), a->stream);
+  if (e == cudaSuccess) e = Fork(a);
+  for (int l = 0; l < a->nlevels && e == cudaSuccess; ++l) {
+    const LevelHost& Lv = a->L[size_t(l)];
+    e = LaunchMaxSpeed(a, l, 0, a->stream);
+    if (e == cudaSuccess) e = LaunchMaxSpeed(a, l, 1, a->side);
+    // no sweep writes A before the join
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(Lv.backup, Lv.A, size_t(Lv.ncells) * kComp * sizeof(double),
+                          cudaMemcpyDeviceToDevice, a->side);
+  }
+  if (e == cudaSuccess) e = Join(a);
   if (e != cudaSuccess) return e;
-  for (int l = 0; l < a->nlevels; ++l)
-    for (int d = 0; d < 2; ++d)
-      if ((e = LaunchMaxSpeed(a, l, d)) != cudaSuccess) return e;
   if ((e = LaunchAmrDt(a->ctrl, a->nlevels, Dx(a), a->stream)) != cudaSuccess) return e;
   int counter = 0;
   if ((e = AdvanceLevel(a, 0, parity, 0, counter)) != cudaSuccess) return e;
@@ -738,6 +763,9 @@ int fvs_amr_create(const fvs_amr_desc* d, const fvs_method* m, fvs_amr** out) {
     }
   }
   cudaError_t e = cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&a->side, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a->ev_fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a->ev_join, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     delete a;
     return CudaFail(e, "cudaStreamCreate");
@@ -878,7 +906,7 @@ int fvs_amr_stable_dt(fvs_amr* a, double* dt) {
   AMR_CUDA(cudaMemsetAsync(&a->ctrl->smax_stable[0][0], 0, sizeof(a->ctrl->smax_stable),
                            a->stream));
   for (int l = 0; l < a->nlevels; ++l)
-    for (int d = 0; d < 2; ++d) AMR_CUDA(LaunchMaxSpeed(a, l, d));
+    for (int d = 0; d < 2; ++d) AMR_CUDA(LaunchMaxSpeed(a, l, d, a->stream));
   unsigned long long bits[kMaxLevels][2];
   AMR_CUDA(cudaMemcpyAsync(bits, a->ctrl->smax_stable, sizeof bits, cudaMemcpyDeviceToHost,
                            a->stream));
