@@ -1,6 +1,6 @@
 // fvs_amr_exact.cu -- AMR patch kernels with the reference's exact FP64
-// arithmetic, and the table-driven kernels of the AMR step (ghost fill,
-// reflux, average-down, dt selection, per-sweep checks).  Compiled with
+// arithmetic, and the table-driven kernels of the AMR step (reflux,
+// average-down, dt selection, per-sweep checks).  Compiled with
 // -fmad=false: the results are bit-identical to the CPU oracle's
 // restatement (oracle/fvs_oracle_amr.cpp).
 #include "fvs_amr.h"

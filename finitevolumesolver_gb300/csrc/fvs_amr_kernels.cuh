@@ -13,7 +13,10 @@
 // they live (Seg::halo): the same level's current buffer or the coarser
 // level, which is the ghost fill of those strips at sweep time.
 //
-// For EinfeldtCfl policies (exact and fast FP64) both kernels screen the CFL
+// PatchRowWarpKernel and PatchMaxSpeedKernel put a cell on each lane, the rows
+// laid end to end: the FP64 sweeps' default and every max-speed pass.
+//
+// For EinfeldtCfl policies (exact and fast FP64) the kernels screen the CFL
 // speeds in FP32 as the uniform sweeps do (fvs_sweep.cuh): a face's exact
 // speed is evaluated only when its FP32 speed plus error bound reaches the
 // thread's threshold.  The rows of a warp can differ in length, so the

@@ -3,9 +3,9 @@
 // speeds:
 //   T = double in a -fmad=false translation unit: the exact flavour, bit for
 //     bit the CPU oracle's restatement of the reference;
-//   T = double with FMA contraction and the refined reciprocals and
-//     reciprocal square roots of fvs_physics_fast.cuh (math policy CcFast):
-//     the fast FP64 flavour, within 1e-12 of the exact one;
+//   T = double with FMA contraction and the nearly rounded quotients and
+//     square roots of fvs_ieee64.cuh (math policy CcFast): the fast FP64
+//     flavour, within 1e-12 of the exact one;
 //   T = float: the mixed flavour -- masked MUSCL-Hancock, HLL/Einfeldt,
 //     boundary (wall) states and CFL speeds in FP32; the state, the face
 //     fractions, the h-box flux combination and the cut-cell update in FP64.

@@ -1,5 +1,5 @@
-// fvs_kernels_cutcell_mixed.cu -- the fast FP64 (FMA contraction, refined
-// reciprocals and square roots: math policy CcFast) and the
+// fvs_kernels_cutcell_mixed.cu -- the fast FP64 (FMA contraction, quotients
+// and roots nearly rounded on the integer pipes: math policy CcFast) and the
 // mixed-precision (FP32 reconstruction, fluxes, wall states and CFL speeds;
 // FP64 state, fractions, h-box combination and update) instantiations of the
 // KBN cut-cell kernels (fvs_cutcell_kbn.cuh); the mixed flavour's FP32

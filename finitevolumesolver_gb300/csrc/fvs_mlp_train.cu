@@ -19,7 +19,7 @@
 // The step is latency: 0.2 GFLOP at batch 8192.  As twelve kernels (gather,
 // one GEMM kernel per product, activations, reductions by atomics, Adam) with
 // their operands in global memory it took 121 us on the GB300; fused it takes
-// about 15 us.
+// 20 us.
 #include "../../include/fvs_gpu.h"
 #include "fvs_internal.h"
 #include "fvs_mlp.cuh"

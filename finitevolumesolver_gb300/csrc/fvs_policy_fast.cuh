@@ -2,9 +2,10 @@
 // mixed-precision flavours (shared by the uniform-grid and the AMR patch
 // sweeps).
 //
-// Fast FP64: the reference's formulas with shared reciprocals, FMA
-// contraction and Newton-refined reciprocal / reciprocal-square-root seeds;
-// per call within ~1e-13 relative of the exact flavour.
+// Fast FP64: the reference's formulas with FMA contraction, written for few
+// FP64 operations; quotients and square roots on the integer pipes, rounded to
+// within 0.75 ulp (fvs_ieee64.cuh); per call within ~1e-13 relative of the
+// exact flavour.
 // Mixed: MUSCL-Hancock reconstruction, limiter, HLLE flux and the CFL
 // speeds in FP32; state storage and the conservative update
 // U' = U + dt/dx (F_L - F_R) in FP64 (the fluxes are widened to FP64 before

@@ -327,7 +327,8 @@ int fvs_solver_state_device(fvs_solver* s, double** cons_dev);
  * include/fub/AMReX/cutcell/PatchHierarchy.hpp:265-314). */
 int fvs_solver_write_plotfile(fvs_solver* s, const char* dir);
 /* Threads per block / cells per thread segment of the sweep kernels
- * (0 = automatic). */
+ * (0 = automatic; 1 in the FP64 and mixed flavours = one cell per lane of a
+ * warp, the automatic choice of the FP64 flavours up to 2^22 cells). */
 int fvs_solver_set_tiling(fvs_solver* s, int seg_len);
 /* Autotuner: times the sweep kernel on the current state for candidate
  * segment lengths (cells per thread along the sweep direction) and keeps
@@ -505,8 +506,9 @@ int fvs_amr_set_launch(fvs_amr* a, int level, int dir, int block, int grid, int 
  * (threads per row, threads per block, blocks, and for the mixed flavour a
  * register/occupancy variant) and keeps the fastest; results are cached per
  * process under the key (precision, direction, the level's patch-size
- * histogram), so hierarchies with the same histogram reuse them.  configs
- * (may be NULL) receives [nlevels][2 directions][block, grid, threads per
+ * histogram), so hierarchies with the same histogram reuse them.  The FP64
+ * flavours have one shape, a lane per cell, reported as 32 threads per row.
+ * configs (may be NULL) receives [nlevels][2 directions][block, grid, threads per
  * row]. */
 int fvs_amr_autotune(fvs_amr* a, int32_t* configs);
 
