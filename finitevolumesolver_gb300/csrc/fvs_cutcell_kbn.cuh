@@ -94,6 +94,22 @@ template <class T> __device__ __forceinline__ void AddMomentum(T* f, int d, T x)
     f[2] += x;
 }
 
+// f[1], f[2] of a flux along d: v m + p on the component along d.  FP32: rounded
+// the same whether the compiler knows d or not (it would contract the products
+// with p and with the differences that follow otherwise).
+template <class T>
+__device__ __forceinline__ void FluxMomentum(T* f, int d, T v, const T* m, T p) {
+  if constexpr (sizeof(T) == 4) {
+    const T a = __fmul_rn(v, m[0]), b = __fmul_rn(v, m[1]);
+    f[1] = d == 0 ? __fadd_rn(a, p) : a;
+    f[2] = d == 0 ? b : __fadd_rn(b, p);
+  } else {
+    f[1] = v * m[0];
+    f[2] = v * m[1];
+    AddMomentum(f, d, p);
+  }
+}
+
 // FP64 comparisons on the integer pipes (one takes the FP64 pipe as long as an
 // addition).
 template <class T> __device__ __forceinline__ bool LessT(T a, T b) {
@@ -156,9 +172,7 @@ __device__ __forceinline__ void CompleteT(const GasT<T, M>& eq, C2T<T>& q, const
 template <class M, class T> __device__ __forceinline__ void FluxT(T* f, const C2T<T>& q, int dir) {
   const T velocity = M::Div(Sel(q.m, dir), q.rho);
   f[0] = Sel(q.m, dir);
-  f[1] = velocity * q.m[0];
-  f[2] = velocity * q.m[1];
-  AddMomentum(f, dir, q.p);
+  FluxMomentum(f, dir, velocity, q.m, q.p);
   f[3] = velocity * (q.E + q.p);
 }
 
@@ -205,9 +219,7 @@ __device__ __forceinline__ void FluxMasked(T* f, const C2T<T>& q, int dir) {
   const T rho = PositiveT(q.rho) ? q.rho : T(1);
   const T velocity = M::Div(Sel(q.m, dir), rho);
   f[0] = Sel(q.m, dir);
-  f[1] = velocity * q.m[0];
-  f[2] = velocity * q.m[1];
-  AddMomentum(f, dir, q.p);
+  FluxMomentum(f, dir, velocity, q.m, q.p);
   f[3] = velocity * (q.E + q.p);
 }
 
