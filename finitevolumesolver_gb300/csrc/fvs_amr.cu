@@ -128,12 +128,14 @@ struct fvs_amr {
     if (side) cudaStreamDestroy(side);
     if (stream) cudaStreamDestroy(stream);
   }
+  // Zeroed and filled on the solver's stream, which no other stream orders:
+  // work of the default stream could run after whatever comes next on this one.
   template <class T> cudaError_t Alloc(T** p, size_t count) {
     void* v = nullptr;
     cudaError_t e = cudaMalloc(&v, std::max<size_t>(count, 1) * sizeof(T));
     if (e == cudaSuccess) {
       allocations.push_back(v);
-      e = cudaMemset(v, 0, std::max<size_t>(count, 1) * sizeof(T));
+      e = cudaMemsetAsync(v, 0, std::max<size_t>(count, 1) * sizeof(T), stream);
     }
     *p = static_cast<T*>(v);
     return e;
@@ -141,8 +143,9 @@ struct fvs_amr {
   template <class T> cudaError_t Upload(T** p, const std::vector<T>& h) {
     cudaError_t e = Alloc(p, h.size());
     if (e == cudaSuccess && !h.empty())
-      e = cudaMemcpy(*p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
-    return e;
+      e = cudaMemcpyAsync(*p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
+    // the caller's vector may go before the copy has read it
+    return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
   }
   int32_t SI(int p, int i, int j) const {  // storage index of cell (i, j) of patch p
     const PatchHost& P = patches[size_t(p)];
@@ -504,6 +507,7 @@ int Build(fvs_amr* a) {
   if (int(sw.size()) > kMaxSweeps) return Fail(FVS_ERR_INVALID, "too many levels");
   a->nsweeps = int(sw.size());
   AMR_CUDA(a->Upload(&a->sweeps, sw));
+  AMR_CUDA(cudaStreamSynchronize(a->stream));
   return FVS_OK;
 }
 
