@@ -596,8 +596,8 @@ class AmrSolver:
 
     def set_launch(self, level, dir, block, grid, threads_per_row=1) -> None:
         """Launch shape of a level's sweeps in direction dir: threads per
-        block, blocks, threads per patch row (1, 2, 4, 8; 32 for the mixed x
-        sweep with the lanes of a warp along x)."""
+        block, blocks, threads per patch row (1, 2, 4, 8; 32 for the lanes of
+        a warp along the rows, in mixed precision x sweeps only)."""
         _capi.check(lib().fvs_amr_set_launch(self._h, int(level), int(dir), int(block),
                                              int(grid), int(threads_per_row)))
 

@@ -983,10 +983,11 @@ int fvs_amr_set_launch(fvs_amr* a, int level, int dir, int block, int grid,
   int si = -1;
   for (int k = 0; k < kSplits; ++k)
     if (kSplitOf[k] == threads_per_row) si = k;
-  if (threads_per_row == 32 && dir == 0 && a->m.precision == FVS_MIXED) si = kSplits;
+  if (threads_per_row == 32 && (dir == 0 || a->m.precision != FVS_MIXED)) si = kSplits;
   if (si < 0)
     return Fail(FVS_ERR_INVALID,
-                "threads per row must be 1, 2, 4 or 8 (or 32: x rows with lanes along x, mixed)");
+                "threads per row must be 1, 2, 4 or 8 (or 32: the lanes of a warp along the rows; "
+                "mixed: x rows)");
   a->L[size_t(level)].block[dir] = block;
   a->L[size_t(level)].grid[dir] = grid;
   a->L[size_t(level)].split[dir] = si;

@@ -499,17 +499,19 @@ int fvs_amr_run(fvs_amr* a, double cfl, double t_end, int max_steps, double* dt_
                 int log_len, fvs_run_stats* stats);
 /* Persistent launch shape of a level's sweeps in direction dir: threads per
  * block, blocks, and threads per patch row (1, 2, 4 or 8: each row split into
- * that many segments; 32, mixed flavour x sweeps only: the rows laid end to
- * end with the lanes of a warp along x). */
+ * that many segments; 32: the rows laid end to end with the lanes of a warp
+ * along them, a cell per lane; not for the mixed flavour's y sweeps).  Every
+ * shape that fvs_amr_autotune returns is accepted. */
 int fvs_amr_set_launch(fvs_amr* a, int level, int dir, int block, int grid, int threads_per_row);
 /* Times the sweeps of every level and direction for a set of launch shapes
  * (threads per row, threads per block, blocks, and for the mixed flavour a
  * register/occupancy variant) and keeps the fastest; results are cached per
  * process under the key (precision, direction, the level's patch-size
- * histogram), so hierarchies with the same histogram reuse them.  The FP64
- * flavours have one shape, a lane per cell, reported as 32 threads per row.
- * configs (may be NULL) receives [nlevels][2 directions][block, grid, threads per
- * row]. */
+ * histogram), so hierarchies with the same histogram reuse them.  A lane per
+ * cell is reported as 32 threads per row; it is the FP64 flavours' shape in
+ * both directions, and the mixed flavour's in x, until this call or
+ * fvs_amr_set_launch chooses another.  configs (may be NULL) receives
+ * [nlevels][2 directions][block, grid, threads per row]. */
 int fvs_amr_autotune(fvs_amr* a, int32_t* configs);
 
 /* ---- Learned start value of the exact Riemann solver ------------------- */
