@@ -5,6 +5,7 @@
 #include "fvs_cutcell.h"
 #include "fvs_ieee64.cuh"
 #include "fvs_internal.h"
+#include "fvs_launch_rule.h"
 #include "fvs_plotfile.h"
 #include "fvs_tma.cuh"
 
@@ -408,36 +409,16 @@ const void* TmaMapOf(const fvs_solver* s, const double* in, int dir) {
   return nullptr;
 }
 
-// Slots of the one-cell-per-lane sweep (a segment length of 1).
-int64_t LaneSlots(const fvs_solver* s, int dir) {
-  return s->cells / s->g.n[dir] * (int64_t(s->g.n[dir]) + 2);
-}
-
 int SegLen(const fvs_solver* s, int dir) {
   if (s->seg_len > 0) return s->seg_len;
   if (s->seg_tuned[dir] > 0) return s->seg_tuned[dir];
-  const int nd = s->g.n[dir];
-  int64_t ntrans = s->cells / nd;
-  const bool mixed = s->m.precision == FVS_MIXED;
-  // Small grids: one cell per lane (SweepLanesKernel) instead of marching
-  // segments, whose serial chains leave the chip idle.  Measured per sweep
-  // against the best marching segment (16 cells, the shortest default, in
-  // brackets): exact FP64 64^3 0.13 / 0.18 ms (0.26), 128^3 0.99 / 1.03 ms,
-  // 192^3 3.25 / 2.95 ms; double-float 128^3 0.44 / 0.46 ms; mixed, where
-  // lanes along y or z load a sector per value: 64^2 25 / 31 us (38), 32^3
-  // equal, 64^3 20 / 11 us.
-  if (!s->cc && (mixed ? s->g.rank == 1 || s->cells <= (int64_t(1) << 14)
-                       : s->cells <= (int64_t(1) << 22)) &&
-      LaneSlots(s, dir) < (int64_t(1) << 31))
-    return 1;
-  // Enough threads for several waves of resident blocks on 152 SMs
-  // (~60K threads per wave at 150 registers per thread); never shorter than
-  // 16 cells, mixed 8 (the 2-cell halo of a segment is recomputed).
-  const int64_t target = 262144;
-  const int shortest = mixed && !s->cc ? 8 : 16;
-  int seg = nd;
-  while (seg > shortest && ntrans * ((nd + seg - 1) / seg) < target) seg = (seg + 1) / 2;
-  return seg;
+  fvs::SweepShape q;
+  q.rank = s->g.rank;
+  q.cells = s->cells;
+  q.n = s->g.n[dir];
+  q.mixed = s->m.precision == FVS_MIXED;
+  q.cut_cells = s->cc;
+  return fvs::AutoSegment(q);
 }
 
 fvs::CcStateArgs MakeCcState(const fvs_solver* s, const double* in) {
@@ -525,7 +506,7 @@ cudaError_t LaunchSweep(const fvs_solver* s, const double* in, double* out,
   a.mlp = s->m.mlp_params;
   a.stats_out = ctrl ? ctrl->newton : s->newton_words;
   a.skip_cfl = skip_cfl ? 1 : 0;
-  a.lanes = a.seg_len == 1 && a.occupancy < 20 && LaneSlots(s, dir) < (int64_t(1) << 31) ? 1 : 0;
+  a.lanes = a.seg_len == 1 && a.occupancy < 20 && fvs::LanesFit(s->cells, a.n[dir]) ? 1 : 0;
   a.tmap = a.occupancy >= 20 ? TmaMapOf(s, in, dir) : nullptr;
   a.t_lo = t_lo;
   a.t_hi = t_hi;
@@ -1197,7 +1178,9 @@ int fvs_solver_autotune(fvs_solver* s, int* seg_out) {
       for (int c : cands) {
         if (c > 2 * nd && c > 8) break;
         // one cell per lane: one candidate, under the first variant
-        if (c == 1 && (s->cc || oi > 0)) continue;
+        const bool lanes = c == 1;
+        if (lanes && (s->cc || oi > 0 || !fvs::LanesFit(s->cells, nd))) continue;
+        if (!lanes && !warp_x && fvs::Segments(nd, c) > fvs::kMaxSegments) continue;
         // the tile kernels (mixed cut cells, variant 0) have no segment length
         if ((warp_x || (cc_cell && occs[oi] == 0)) && c > 8) break;
         s->seg_len = c;
