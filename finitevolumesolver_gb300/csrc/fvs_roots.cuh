@@ -17,14 +17,18 @@ namespace riemann {
 // x^(1/gamma) = x^((n-2)/n) = x r^2, and the integer powers b^(n-2) =
 // b^(2/(gamma-1)) and b^n = b^(2 gamma/(gamma-1)).  r is Newton's method for
 // r^-n = x with its second-order term, r <- r (1 + e / n + (n + 1) e^2 / (2 n^2)),
-// e = 1 - x r^n (no division), from an FP32 estimate whose relative error is
-// at most 2e-5 / n: one step cubes the error to n^2 / 3 of it, below FP64
-// rounding.  That is ~11 FP64 operations where pow() evaluates a logarithm
-// and an exponential in extended precision; the results are within 2e-14
-// relative of pow() with the solver's FP64 exponents, which are themselves
-// roundings of the rationals above (tests/cpp/root_check.cu).  Other gammas,
-// and ratios outside [1e-30, 1e30], take pow() with the reference's
-// exponents.
+// e = 1 - x r^n (no division), from an FP32 estimate.  One step leaves
+// (n + 1) (2 n + 1) e^3 / (6 n^3).  The device's estimate has |e| < 9e-6 (n up
+// to 64, largest toward the ends 1e+-30 of the range; 6e-6 at n = 3, 7e-6 at
+// n = 5), so that is at most 0.35 of an FP64 rounding (2^-53), and the largest
+// error measured, 1.6 roundings, is below that of two Newton steps, 1.8, which
+// round twice (tests/cpp/root_device_check.cu holds the device to it).  An
+// estimate off by 2 FP32 ulp more leaves 5 to 12 at n = 3.  That is ~11 FP64
+// operations where pow() evaluates a logarithm and an exponential in extended
+// precision; the powers are within 2e-14 relative of pow() with the solver's
+// FP64 exponents, which are themselves roundings of the rationals above
+// (tests/cpp/root_check.cu).  Other gammas, and ratios outside [1e-30, 1e30],
+// take pow() with the reference's exponents.
 __host__ __device__ inline int RootOrder(double gamma) {
   if (!(gamma > 1.0)) return 0;
   const double q = 2.0 * gamma / (gamma - 1.0);
