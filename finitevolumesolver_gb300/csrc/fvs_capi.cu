@@ -418,6 +418,7 @@ int SegLen(const fvs_solver* s, int dir) {
   q.n = s->g.n[dir];
   q.mixed = s->m.precision == FVS_MIXED;
   q.cut_cells = s->cc;
+  q.variant = s->occ_tuned[dir];
   return fvs::AutoSegment(q);
 }
 

@@ -13,6 +13,7 @@ struct SweepShape {
   int n = 0;           // cells along the sweep direction
   bool mixed = false;
   bool cut_cells = false;
+  int variant = 0;     // launch variant of the marching sweep, 0: not chosen
 };
 
 // Segments of a line are blocks in the grid's second dimension.
@@ -33,9 +34,11 @@ inline int AutoSegment(const SweepShape& s) {
   // brackets): exact FP64 64^3 0.13 / 0.18 ms (0.26), 128^3 0.99 / 1.03 ms,
   // 192^3 3.25 / 2.95 ms; double-float 128^3 0.44 / 0.46 ms; mixed, where
   // lanes along y or z load a sector per value: 64^2 25 / 31 us (38), 32^3
-  // equal, 64^3 20 / 11 us.
-  if (!s.cut_cells && (s.mixed ? s.rank == 1 || s.cells <= (int64_t(1) << 14)
-                               : s.cells <= (int64_t(1) << 22)) &&
+  // equal, 64^3 20 / 11 us.  Not where the caller has chosen a variant of the
+  // marching sweep.
+  if (!s.cut_cells && s.variant == 0 &&
+      (s.mixed ? s.rank == 1 || s.cells <= (int64_t(1) << 14)
+               : s.cells <= (int64_t(1) << 22)) &&
       LanesFit(s.cells, s.n))
     return 1;
   // Enough threads for several waves of resident blocks on 152 SMs

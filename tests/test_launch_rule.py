@@ -52,6 +52,19 @@ def test_segments_fit_a_launch(auto):
             assert _segments(c["n"], seg) <= 65535, c
 
 
+@pytest.mark.parametrize("mixed,variants", [(0, (3,)), (1, (4, 5, 10, 14, 15, 20, 24, 25))])
+def test_a_chosen_variant_marches(auto, mixed, variants):
+    """fvs_solver_set_launch(dir, 0, variant): the automatic length of that
+    variant of the marching sweep, never one cell per lane."""
+    cases = [dict(rank=rank, cells=n ** rank, n=n, mixed=mixed, variant=v)
+             for rank in (1, 2, 3) for n in (16, 25, 64, 160) for v in (0, *variants)]
+    for c, seg in zip(cases, auto(cases)):
+        if c["variant"]:
+            assert seg > 1, c
+        elif not mixed:
+            assert seg == 1, c
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [(2, 600000), (2, 2, 600000)])
 def test_long_narrow_mixed_grid(fvs, n):
