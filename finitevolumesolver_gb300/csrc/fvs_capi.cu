@@ -414,6 +414,9 @@ int SegLen(const fvs_solver* s, int dir) {
   if (s->seg_tuned[dir] > 0) return s->seg_tuned[dir];
   fvs::SweepShape q;
   q.rank = s->g.rank;
+  q.family = IsGodunov(s->m.flux_method)         ? fvs::SweepFamily::kGodunov
+             : HllemRecon(s->m.flux_method) >= 0 ? fvs::SweepFamily::kHllem
+                                                 : fvs::SweepFamily::kHlle;
   q.cells = s->cells;
   q.n = s->g.n[dir];
   q.mixed = s->m.precision == FVS_MIXED;

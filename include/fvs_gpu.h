@@ -328,7 +328,8 @@ int fvs_solver_state_device(fvs_solver* s, double** cons_dev);
 int fvs_solver_write_plotfile(fvs_solver* s, const char* dir);
 /* Threads per block / cells per thread segment of the sweep kernels
  * (0 = automatic; 1 in the FP64 and mixed flavours = one cell per lane of a
- * warp, the automatic choice of the FP64 flavours up to 2^22 cells). */
+ * warp, the automatic choice of the FP64 flavours on small grids, up to 2^22
+ * cells depending on the flux method and the rank). */
 int fvs_solver_set_tiling(fvs_solver* s, int seg_len);
 /* Autotuner: times the sweep kernel on the current state for candidate
  * segment lengths (cells per thread along the sweep direction) and keeps

@@ -22,6 +22,7 @@ int main() {
       else if (key == "n") q.n = int(v);
       else if (key == "mixed") q.mixed = v != 0;
       else if (key == "cut_cells") q.cut_cells = v != 0;
+      else if (key == "family") q.family = static_cast<fvs::SweepFamily>(v);
       else if (key == "variant") q.variant = int(v);
       else return 2;
     }

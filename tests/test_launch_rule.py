@@ -40,9 +40,9 @@ LENGTHS = sorted({m for k in range(31) for m in ((1 << k) - 1, 1 << k, (1 << k) 
 def test_segments_fit_a_launch(auto):
     """A marching sweep's segments of a line are the grid's second dimension, at
     most 65535; one cell per lane counts its slots in 32 bits."""
-    cases = [dict(rank=rank, cells=n * other, n=n, mixed=mixed, cut_cells=cc)
+    cases = [dict(rank=rank, cells=n * other, n=n, mixed=mixed, cut_cells=cc, family=family)
              for n in LENGTHS for other in (1, 2, 4, 1000, 1 << 20)
-             for rank in (1, 2, 3) for mixed in (0, 1) for cc in (0, 1)
+             for rank in (1, 2, 3) for mixed in (0, 1) for cc in (0, 1) for family in range(3)
              if (rank > 1 or other == 1) and (rank == 2 or not cc) and n * other < 1 << 34]
     for c, seg in zip(cases, auto(cases)):
         assert 1 <= seg <= max(c["n"], 1), c
@@ -63,6 +63,26 @@ def test_a_chosen_variant_marches(auto, mixed, variants):
             assert seg > 1, c
         elif not mixed:
             assert seg == 1, c
+
+
+# (family, n of the direction, other extents' product, rank): one cell per lane?
+HLLE, HLLEM, GODUNOV = range(3)
+MEASURED = [(HLLE, 160, 160 ** 2, 3, True), (HLLE, 192, 192 ** 2, 3, False),
+            (HLLE, 1448, 1448, 2, True), (HLLE, 2048, 2048, 2, False),
+            (HLLE, 1 << 22, 1, 1, True), (HLLEM, 2048, 2048, 2, True),
+            (HLLEM, 160, 160 ** 2, 3, True), (GODUNOV, 80, 80 ** 2, 3, True),
+            (GODUNOV, 96, 96 ** 2, 3, False), (GODUNOV, 128, 128 ** 2, 3, False),
+            (GODUNOV, 512, 512, 2, True), (GODUNOV, 512, 1024, 2, True),
+            (GODUNOV, 2048, 2048, 2, True), (GODUNOV, 64, 8192, 2, False),
+            (GODUNOV, 8192, 64, 2, True), (GODUNOV, 64, 2048, 2, True),
+            (GODUNOV, 1 << 22, 1, 1, True)]
+
+
+def test_one_cell_per_lane_where_it_is_faster(auto):
+    """The side of the rule that each measured sweep falls on."""
+    cases = [dict(family=f, n=n, cells=n * other, rank=rank) for f, n, other, rank, _ in MEASURED]
+    for m, seg in zip(MEASURED, auto(cases)):
+        assert (seg == 1) == m[4], m
 
 
 @pytest.mark.gpu
