@@ -454,8 +454,8 @@ struct FusedArgs {
   int given_rows;      // 1: rows 0..batch-1 of feat (gradient check)
   int count;           // 1: a training step (the step counter advances)
   // step[0]: steps the sampling has seen (UpdateKernel advances it);
-  // step[1]: Adam's step number (this kernel advances it).  Neither kernel
-  // reads the counter it writes.
+  // step[1]: Adam's step number (this kernel advances it, UpdateKernel takes
+  // that back for a failed step).  Neither kernel reads the counter it writes.
   unsigned long long* step;
   const float* blob;   // statistics, biases, output weights
   const __nv_bfloat16* W1;
@@ -472,6 +472,7 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   __shared__ float vec[mlp::kParams - mlp::kOffB2];  // b2, w3, b3
   __shared__ float b1[kH], stats[2 * mlp::kIn];
   __shared__ float residual[kTile], target[kTile];
+  __shared__ int failed;  // a wait of an earlier step ran out
   // per row-warp sums over the tiles: db1, db2, dw3 and (db3, loss)
   __shared__ float sums[4][3 * kH + 2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -480,8 +481,9 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   if (tid == 0) {
     tc::MbarInit(&bar, 1);
     tma::FenceMbarInit();
-    if (a.count && blockIdx.x == 0) a.step[1] += 1;
   }
+  if (tid == 32 && a.count && blockIdx.x == 0) a.step[1] += 1;
+  if (tid == 64) failed = *a.error;
   LoadWeights(sm + kOffSW1, a.W1, kXin);
   LoadWeights(sm + kOffSW2, a.W2, kH);
   LoadWeights(sm + kOffSW2t, a.W2t, kH);
@@ -500,6 +502,7 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   float* act = reinterpret_cast<float*>(sm + kOffAct);
   const unsigned long long step = a.step[0];
   MmaPhases mma{&bar, a.error};
+  mma.ok = failed == 0;
   const int tiles = a.batch / kTile;
   bool first = true;
   for (int tile = blockIdx.x; tile < tiles && mma.ok; tile += gridDim.x) {
@@ -598,6 +601,9 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
 #pragma unroll
       for (int k = 0; k < mlp::kIn; ++k) out[mlp::kOffW1 + (row - kH) * mlp::kIn + k] = v[k];
     }
+  } else {  // (UpdateKernel does not use sums of a failed step)
+    for (int i = tid; i < kH * kH; i += blockDim.x) out[mlp::kOffW2 + i] = 0.0f;
+    for (int i = tid; i < kH * mlp::kIn; i += blockDim.x) out[mlp::kOffW1 + i] = 0.0f;
   }
   if (tid < 3 * kH + 2) {
     const float t = ((sums[0][tid] + sums[1][tid]) + sums[2][tid]) + sums[3][tid];
@@ -617,13 +623,16 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
 
 // The gradient (the CTAs' partial sums added in a fixed order), and with
 // `update` Adam (lr, beta1 0.9, beta2 0.999, eps 1e-8) and the published
-// weights.  Blocks of 32 parameters x 8 parts of the CTAs.
+// weights.  Blocks of 32 parameters x 8 parts of the CTAs.  Once a wait for the
+// tensor cores has run out (*error), the sums are not a gradient: the weights,
+// the moments and the counters stay as they were before the step.
 __global__ void __launch_bounds__(256)
     UpdateKernel(Net net, const float* partial, int ctas, int update, float lr,
-                 unsigned long long* step, float* loss) {
+                 unsigned long long* step, float* loss, const int* error) {
   __shared__ float part[8][32];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + x;
+  const bool failed = *error != 0;
   float s = 0.0f;
   if (i < kPartial)
     for (int c = y; c < ctas; c += 8) s += partial[int64_t(c) * kPartial + i];
@@ -633,10 +642,15 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int k = 1; k < 8; ++k) s += part[k][x];
   if (i == mlp::kParams) {
+    if (failed) {
+      if (update) step[1] -= 1;
+      return;
+    }
     *loss += s;
     if (update) step[0] += 1;
     return;
   }
+  if (failed) return;
   net.grad[i] = s;
   if (!update || i < mlp::kOffW1) return;
   const unsigned long long t = step[1];
@@ -785,7 +799,8 @@ cudaError_t EnqueueStep(fvs_mlp* m, FusedArgs a, bool update, float lr) {
   const int grid = std::min(a.batch / kTile, m->ctas);
   FusedStepKernel<<<grid, kFusedThreads, kFusedSmem, m->stream>>>(a);
   UpdateKernel<<<(kPartial + 31) / 32, 256, 0, m->stream>>>(m->net, m->partial, grid,
-                                                            update ? 1 : 0, lr, m->step, m->loss);
+                                                            update ? 1 : 0, lr, m->step, m->loss,
+                                                            m->error);
   return cudaGetLastError();
 }
 
