@@ -87,23 +87,67 @@ int HllemRecon(int method) {
   }
 }
 
-// What fvs_compute_stable_dt keeps per calling thread and device: 8 bytes of
+// The driver's number of the current context, another one after cudaDeviceReset
+// (0 where the driver does not tell), and whether a device's primary context
+// exists.
+template <class Fn> Fn DriverFn(const char* name) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      q != cudaDriverEntryPointSuccess) {
+    cudaGetLastError();
+    p = nullptr;
+  }
+  return reinterpret_cast<Fn>(p);
+}
+unsigned long long ContextId() {
+  static const auto fn =
+      DriverFn<CUresult (*)(CUcontext, unsigned long long*)>("cuCtxGetId");
+  unsigned long long id = 0;
+  return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+bool PrimaryContextActive(int dev) {
+  static const auto fn =
+      DriverFn<CUresult (*)(CUdevice, unsigned*, int*)>("cuDevicePrimaryCtxGetState");
+  unsigned flags = 0;
+  int active = 0;
+  return fn && fn(dev, &flags, &active) == CUDA_SUCCESS && active != 0;
+}
+
+// What fvs_compute_stable_dt keeps per calling thread and context: 8 bytes of
 // page-locked host memory for its result (a call waits for its stream, so a
 // thread has one in flight), and 8 bytes of the device's stream-ordered pool.
 // The pool returns a chunk that nothing lives in at every synchronisation, so
 // the call's own 8 bytes mapped and unmapped one each time: 140 of its 160 us.
-// Both are given back when the thread ends.
+// Both are given back when the thread ends; what belonged to a context that
+// cudaDeviceReset has destroyed went with it and is not touched again.
 struct SpeedWord {
   unsigned long long* resident = nullptr;
   unsigned long long* host = nullptr;
 };
 struct SpeedWords {
-  std::map<int, SpeedWord> by_device;
+  std::map<std::pair<int, unsigned long long>, SpeedWord> by_context;  // (device, ContextId)
   ~SpeedWords() {
-    for (auto& kv : by_device) {
+    int cur = 0;
+    // relaxed: another thread may be capturing, and these frees are no part of it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (by_context.empty() || cudaGetDevice(&cur) != cudaSuccess ||
+        cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess)
+      return;
+    int dev = cur;
+    for (auto& kv : by_context) {
+      const int d = kv.first.first;
+      if (!PrimaryContextActive(d)) continue;
+      if (d != dev) {
+        if (cudaSetDevice(d) != cudaSuccess) continue;
+        dev = d;
+      }
+      if (ContextId() != kv.first.second) continue;
       cudaFree(kv.second.resident);
       cudaFreeHost(kv.second.host);
     }
+    if (dev != cur) cudaSetDevice(cur);
+    cudaThreadExchangeStreamCaptureMode(&mode);
   }
 };
 thread_local SpeedWords g_speed_words;
@@ -117,7 +161,7 @@ cudaError_t ThreadSpeedWord(cudaStream_t st, unsigned long long** host) {
   int dev = 0;
   e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  SpeedWord& w = g_speed_words.by_device[dev];
+  SpeedWord& w = g_speed_words.by_context[{dev, ContextId()}];
   if (!w.resident) e = cudaMallocAsync(&w.resident, sizeof *w.resident, st);
   if (e == cudaSuccess && !w.host) e = cudaMallocHost(&w.host, sizeof *w.host);
   *host = w.host;

@@ -143,7 +143,10 @@ int fvs_compute_numeric_fluxes(const fvs_method* m, int rank,
  * Direction dir)  include/fub/flux_method/FluxMethod.hpp:154-170, 295-382.
  * window_rule 0 = sequential tag windows, 1 = simd tag windows (the
  * reference's default OpenMpSimdTag).  Synchronises `stream`; writes the
- * minimum stable dt of the patch to *dt_out (host). */
+ * minimum stable dt of the patch to *dt_out (host).  Allocates 8 bytes of the
+ * device's default pool per call, so not while a stream capture refuses that;
+ * a calling thread keeps 8 more bytes of the pool and of page-locked memory
+ * until it ends (or cudaDeviceReset takes them). */
 int fvs_compute_stable_dt(const fvs_method* m, int rank,
                           const double* states_dev, fvs_box cell_box,
                           double dx, int dir, int window_rule, double* dt_out,
