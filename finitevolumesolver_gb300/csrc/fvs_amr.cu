@@ -37,6 +37,9 @@ using namespace fvs::amr;
 
 namespace {
 
+// Values of the transfers' device buffer (64 MiB).
+constexpr int64_t kStageValues = int64_t(1) << 23;
+
 struct PatchHost {
   int level;
   int lo[2], hi[2], n[2];
@@ -97,9 +100,15 @@ struct fvs_amr {
   std::vector<std::vector<int>> level_patch_order;
   double* reg = nullptr;
   int32_t nslots = 0;
-  PatchCopy* patch_copy = nullptr;  // the patches' flat and storage places
-  int64_t flat_values = 0;          // values of the flat host array
-  double* flat = nullptr;           // its device copy, made by the first transfer
+  // transfers between the caller's flat array and the levels, chunk by chunk
+  // through a device buffer of at most kStageValues values (or one row)
+  PatchCopy* parts = nullptr;
+  struct Chunk {
+    int first, count;       // parts
+    int64_t base, values;   // of the flat array
+  };
+  std::vector<Chunk> chunks;
+  double* stage = nullptr;
   float* signs = nullptr;
   AmrControl* ctrl = nullptr;
   AmrControl* ctrl_host = nullptr;
@@ -474,20 +483,34 @@ int Build(fvs_amr* a) {
       }
     }
   }
-  std::vector<PatchCopy> copies;
+  std::vector<PatchCopy> parts;
+  int64_t flat = 0, stage = 0;
+  auto add = [&](int p, int j0, int rows, int comp, int ncomp) {
+    const PatchHost& P = a->patches[size_t(p)];
+    const PatchCopy c{flat, a->SI(p, P.lo[0], P.lo[1] + j0), P.level, P.n[0], rows, P.pitch,
+                      comp, ncomp};
+    const int64_t values = int64_t(ncomp) * P.n[0] * rows;
+    if (a->chunks.empty() || flat + values - a->chunks.back().base > kStageValues)
+      a->chunks.push_back({int(parts.size()), 0, flat, 0});
+    fvs_amr::Chunk& k = a->chunks.back();
+    k.count += 1;
+    k.values += values;
+    stage = std::max(stage, k.values);
+    flat += values;
+    parts.push_back(c);
+  };
   for (size_t p = 0; p < a->patches.size(); ++p) {
     const PatchHost& P = a->patches[p];
-    PatchCopy c{};
-    c.flat = a->flat_values;
-    c.first = a->SI(int(p), P.lo[0], P.lo[1]);
-    c.level = P.level;
-    c.nx = P.n[0];
-    c.ny = P.n[1];
-    c.pitch = P.pitch;
-    copies.push_back(c);
-    a->flat_values += int64_t(kComp) * P.n[0] * P.n[1];
+    if (int64_t(kComp) * P.n[0] * P.n[1] <= kPatchCopyValues) {
+      add(int(p), 0, P.n[1], 0, kComp);
+      continue;
+    }
+    const int rows = std::max(1, kPatchCopyValues / P.n[0]);
+    for (int c = 0; c < kComp; ++c)
+      for (int j = 0; j < P.n[1]; j += rows) add(int(p), j, std::min(rows, P.n[1] - j), c, 1);
   }
-  AMR_CUDA(a->Upload(&a->patch_copy, copies));
+  AMR_CUDA(a->Upload(&a->parts, parts));
+  AMR_CUDA(a->Alloc(&a->stage, size_t(stage)));
   AMR_CUDA(a->Alloc(&a->reg, size_t(std::max(a->nslots, 1)) * 3 * kComp));
   AMR_CUDA(a->Upload(&a->signs, signs_h));
   AMR_CUDA(a->Alloc(&a->ctrl, 1));
@@ -788,16 +811,18 @@ int fvs_amr_destroy(fvs_amr* a) {
 }
 
 // The interiors between the caller's flat array and the levels go through a
-// device copy of the flat array and one kernel (the host used to index every
-// value: 5 ms of a 0.6 M-cell upload and download).  The ghost storage of the
-// levels stays as it is (zero: no sweep reads or writes it).
+// device copy of the flat array and a kernel (the host used to index every
+// value: 5 ms of a 0.6 M-cell upload and download), in chunks that keep the
+// copy's memory bounded.  The ghost storage of the levels stays as it is (zero:
+// no sweep reads or writes it).
 int fvs_amr_upload(fvs_amr* a, const double* host) {
   if (!a || !host) return Fail(FVS_ERR_INVALID, "NULL argument");
-  if (!a->flat) AMR_CUDA(a->Alloc(&a->flat, size_t(a->flat_values)));
-  AMR_CUDA(cudaMemcpyAsync(a->flat, host, size_t(a->flat_values) * sizeof(double),
-                           cudaMemcpyHostToDevice, a->stream));
-  AMR_CUDA(LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), a->flat, true,
-                           a->stream));
+  for (const fvs_amr::Chunk& k : a->chunks) {
+    AMR_CUDA(cudaMemcpyAsync(a->stage, host + k.base, size_t(k.values) * sizeof(double),
+                             cudaMemcpyHostToDevice, a->stream));
+    AMR_CUDA(LaunchPatchCopy(a->parts + k.first, k.count, Arrays(a), a->stage, k.base, true,
+                             a->stream));
+  }
   AMR_CUDA(cudaStreamSynchronize(a->stream));
   a->t = 0.0;
   a->cycle = 0;
@@ -806,11 +831,12 @@ int fvs_amr_upload(fvs_amr* a, const double* host) {
 
 int fvs_amr_download(fvs_amr* a, double* host) {
   if (!a || !host) return Fail(FVS_ERR_INVALID, "NULL argument");
-  if (!a->flat) AMR_CUDA(a->Alloc(&a->flat, size_t(a->flat_values)));
-  AMR_CUDA(LaunchPatchCopy(a->patch_copy, int(a->patches.size()), Arrays(a), a->flat, false,
-                           a->stream));
-  AMR_CUDA(cudaMemcpyAsync(host, a->flat, size_t(a->flat_values) * sizeof(double),
-                           cudaMemcpyDeviceToHost, a->stream));
+  for (const fvs_amr::Chunk& k : a->chunks) {
+    AMR_CUDA(LaunchPatchCopy(a->parts + k.first, k.count, Arrays(a), a->stage, k.base, false,
+                             a->stream));
+    AMR_CUDA(cudaMemcpyAsync(host + k.base, a->stage, size_t(k.values) * sizeof(double),
+                             cudaMemcpyDeviceToHost, a->stream));
+  }
   AMR_CUDA(cudaStreamSynchronize(a->stream));
   return FVS_OK;
 }

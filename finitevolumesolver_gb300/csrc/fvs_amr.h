@@ -170,19 +170,26 @@ cudaError_t LaunchReflux(double* coarse, int32_t n_coarse, const double* reg,
                          cudaStream_t s);
 cudaError_t LaunchAverageDown(double* coarse, int32_t n_coarse, const double* fine,
                               int32_t n_fine, const AvgDown* e, int32_t count, cudaStream_t s);
-// A patch's interior in the flat host layout and in its level's storage.
+// A part of a patch's interior in the flat host layout and in its level's
+// storage: `ncomp` components from `comp` on of `rows` rows of nx cells, all of
+// a small patch, or rows of one component of a larger one.  Contiguous in the
+// flat array.
 struct PatchCopy {
   int64_t flat;    // first value in the flat array
-  int64_t first;   // storage index of the first interior cell
-  int32_t level, nx, ny, pitch;
+  int64_t first;   // storage index of the first cell
+  int32_t level, nx, rows, pitch;
+  int32_t comp, ncomp;
 };
+// Values of a part: a block's share, so that one large patch takes many blocks.
+constexpr int kPatchCopyValues = 16384;
 struct LevelArrays {
   double* state[kMaxLevels];
   int64_t ncells[kMaxLevels];
 };
-// flat -> levels (to_levels) or levels -> flat, interiors only.
-cudaError_t LaunchPatchCopy(const PatchCopy* patches, int npatches, const LevelArrays& levels,
-                            double* flat, bool to_levels, cudaStream_t s);
+// stage -> levels (to_levels) or levels -> stage, `stage` holding the flat
+// array's values from `base` on.
+cudaError_t LaunchPatchCopy(const PatchCopy* parts, int nparts, const LevelArrays& levels,
+                            double* stage, int64_t base, bool to_levels, cudaStream_t s);
 struct LevelDx {
   double dx[kMaxLevels];
 };

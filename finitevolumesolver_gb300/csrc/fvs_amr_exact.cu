@@ -153,18 +153,19 @@ cudaError_t LaunchAmrEndStep(AmrControl* ctrl, const SweepInfo* sweeps, int nswe
   return cudaGetLastError();
 }
 
-// One block per patch: the patch's interior between the flat host layout
+// One block per part: a part of a patch's interior between the flat host layout
 // ([component][ny][nx], patches one after the other) and its level's storage.
-__global__ void PatchCopyKernel(const PatchCopy* patches, LevelArrays levels, double* flat,
-                                int to_levels) {
-  const PatchCopy p = patches[blockIdx.x];
-  const int64_t area = int64_t(p.nx) * p.ny;
-  double* level = levels.state[p.level];
-  for (int64_t i = threadIdx.x; i < area; i += blockDim.x) {
-    const int64_t at = p.first + (i / p.nx) * p.pitch + i % p.nx;
-#pragma unroll
-    for (int c = 0; c < kComp; ++c) {
-      double* f = flat + p.flat + c * area + i;
+__global__ void PatchCopyKernel(const PatchCopy* parts, LevelArrays levels, double* stage,
+                                int64_t base, int to_levels) {
+  const PatchCopy p = parts[blockIdx.x];
+  const int area = p.nx * p.rows;  // of one component: at most kPatchCopyValues, or one row
+  double* level = levels.state[p.level] + p.comp * levels.ncells[p.level] + p.first;
+  double* flat = stage + (p.flat - base);
+  for (int i = threadIdx.x; i < area; i += blockDim.x) {
+    const int row = i / p.nx;
+    const int64_t at = int64_t(row) * p.pitch + (i - row * p.nx);
+    for (int c = 0; c < p.ncomp; ++c) {
+      double* f = flat + int64_t(c) * area + i;
       double* q = level + c * levels.ncells[p.level] + at;
       if (to_levels)
         *q = *f;
@@ -174,10 +175,10 @@ __global__ void PatchCopyKernel(const PatchCopy* patches, LevelArrays levels, do
   }
 }
 
-cudaError_t LaunchPatchCopy(const PatchCopy* patches, int npatches, const LevelArrays& levels,
-                            double* flat, bool to_levels, cudaStream_t s) {
-  if (npatches == 0) return cudaSuccess;
-  PatchCopyKernel<<<npatches, 256, 0, s>>>(patches, levels, flat, to_levels ? 1 : 0);
+cudaError_t LaunchPatchCopy(const PatchCopy* parts, int nparts, const LevelArrays& levels,
+                            double* stage, int64_t base, bool to_levels, cudaStream_t s) {
+  if (nparts == 0) return cudaSuccess;
+  PatchCopyKernel<<<nparts, 256, 0, s>>>(parts, levels, stage, base, to_levels ? 1 : 0);
   return cudaGetLastError();
 }
 
