@@ -145,12 +145,23 @@ __host__ __device__ __forceinline__ bool Negative(double x) {
 }
 __host__ __device__ __forceinline__ bool IsNan(double x) { return (Bits(x) & ~kSign) > kInf; }
 __host__ __device__ __forceinline__ bool IsZero(double x) { return (Bits(x) & ~kSign) == 0u; }
-// a < b, and -0 < +0 (the callers' minima and maxima do not depend on it)
+// a < b, and -0 < +0 (its callers differ by the sign of a zero at most; MinMod
+// avoids that)
 __host__ __device__ __forceinline__ bool Less(double a, double b) {
   const int64_t x = static_cast<int64_t>(Bits(a)), y = static_cast<int64_t>(Bits(b));
   const int64_t kx = x ^ static_cast<int64_t>(static_cast<uint64_t>(x >> 63) >> 1);
   const int64_t ky = y ^ static_cast<int64_t>(static_cast<uint64_t>(y >> 63) >> 1);
   return kx < ky && !IsNan(a) && !IsNan(b);
+}
+
+// The reference's MinMod, (sR > 0) ? max(0, min(sL, sR)) : min(0, max(sL, sR))
+// with its a < b ? a : b and a > b ? a : b: which of two zeros, and which side
+// of a NaN, comes out as there.
+__host__ __device__ __forceinline__ double MinMod(double sL, double sR) {
+  const bool up = Positive(sR);
+  const bool left = up ? Less(sL, sR) : Less(sR, sL) && !(IsZero(sL) && IsZero(sR));
+  const double m = left ? sL : sR;
+  return (up ? Negative(m) : Positive(m)) ? 0.0 : m;
 }
 
 // A divisor prepared for several quotients.

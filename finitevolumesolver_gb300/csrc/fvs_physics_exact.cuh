@@ -187,23 +187,24 @@ __device__ __forceinline__ double FaceMaxSpeed(const Gas& eq, const CellWave& L,
 enum Limiter : int { kVanLeer = 0, kMinMod = 1, kNoLimiter = 2, kNoGradient = 3 };
 
 // Half the limited slope, what the predictor adds and subtracts.  Van Leer:
-// 0.5 ((2 sL sR) / (sL + sR)) has the bits of (sL sR) / (sL + sR) unless
-// sL sR leaves the range of ieee64's quotients.
+// 0.5 ((2 sL sR) / (sL + sR)) has the bits of (sL sR) / (sL + sR) unless the
+// product or the sum leaves the range of ieee64's quotients.
 __device__ __forceinline__ double HalfSlopeOf(int limiter, double sL, double sR) {
   if (limiter == kVanLeer) {
     const double c = sL * sR;
     const bool pos = ieee64::Positive(c);
-    double hs = Div(c, pos ? sL + sR : 1.0);
+    const ieee64::Divisor sum = MakeDivisor(pos ? sL + sR : 1.0);
+    double hs = Div(c, sum);
     hs = pos ? hs : 0.0;
-    if (ieee64::Span(ieee64::Hi(c)) >= ieee64::kSpan && !ieee64::IsZero(sL) && !ieee64::IsZero(sR)) {
+    const uint32_t span = ieee64::Span(ieee64::Hi(c));
+    if ((span > sum.span ? span : sum.span) >= ieee64::kSpan && !ieee64::IsZero(sL) &&
+        !ieee64::IsZero(sR)) {
       const double c2 = 2.0 * sL * sR;
       hs = 0.5 * ((c2 > 0.0) ? ieee64::IeeeDiv(c2, sL + sR) : 0.0);
     }
     return hs;
   }
-  if (limiter == kMinMod) {
-    return 0.5 * ((sR > 0) ? PMax(0.0, PMin(sL, sR)) : PMin(0.0, PMax(sL, sR)));
-  }
+  if (limiter == kMinMod) return 0.5 * ieee64::MinMod(sL, sR);
   if (limiter == kNoLimiter) return 0.5 * (0.5 * (sL + sR));
   return 0.0;
 }

@@ -265,7 +265,8 @@ __device__ __forceinline__ T HalfSlopeOf(int limiter, T sL, T sR) {
     }
   }
   if (limiter == 1) {  // MinMod
-    return T(0.5) * ((sR > T(0)) ? Max(T(0), Min(sL, sR)) : Min(T(0), Max(sL, sR)));
+    if constexpr (kIsF64<T>) return 0.5 * ieee64::MinMod(sL, sR);
+    else return T(0.5) * ((sR > T(0)) ? Max(T(0), Min(sL, sR)) : Min(T(0), Max(sL, sR)));
   }
   if (limiter == 2) return T(0.25) * (sL + sR);  // NoLimiter: half of 0.5 (sL + sR)
   return T(0);  // NoGradient
