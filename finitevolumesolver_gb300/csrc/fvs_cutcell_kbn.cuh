@@ -132,11 +132,11 @@ template <class T> __device__ __forceinline__ T PMin0T(T a) {
 template <class T> __device__ __forceinline__ T PMax0T(T a) {
   return PositiveT(a) ? a : T(0);
 }
-// (gamma - 1) (roeH - 0.5 roeU roeU); FP64: the half folded into an FMA
-// (exact::RoeA2), the same bits
+// (gamma - 1) (roeH - 0.5 roeU roeU); FP64: the half off the FP64 pipe, the same
+// bits (exact::RoeA2)
 template <class T, class G> __device__ __forceinline__ T RoeA2T(const G& eq, T roeU, T roeH) {
   if constexpr (sizeof(T) == 8)
-    return (eq.gamma - 1.0) * __fma_rn(-0.5, __dmul_rn(roeU, roeU), roeH);
+    return (eq.gamma - 1.0) * __dsub_rn(roeH, __dmul_rn(ieee64::HalfFactor(roeU), roeU));
   else
     return (eq.gamma - T(1)) * (roeH - T(0.5) * roeU * roeU);
 }

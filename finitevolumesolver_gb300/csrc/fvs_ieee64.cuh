@@ -164,6 +164,13 @@ __host__ __device__ __forceinline__ double MinMod(double sL, double sR) {
   return (up ? Negative(m) : Positive(m)) ? 0.0 : m;
 }
 
+// A factor y with the bits of (0.5 x) x in y x, off the FP64 pipe: x / 2, or x
+// itself below 2^-1021, where either product is zero.
+__host__ __device__ __forceinline__ double HalfFactor(double x) {
+  const uint32_t h = Hi(x);
+  return (h & 0x7FE00000u) ? Make(h - (1u << 20), Lo(x)) : x;
+}
+
 // A divisor prepared for several quotients.
 struct Divisor {
   double b;

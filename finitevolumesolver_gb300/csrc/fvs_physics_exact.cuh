@@ -10,8 +10,8 @@
 // same bits elsewhere is taken off it: quotients and square roots run on the
 // integer pipes (fvs_ieee64.cuh: 137 and 143 clocks of the FP64 pipe per warp
 // become about 25 of the integer pipes), comparisons of signs and magnitudes
-// are integer ones, and products with 0.5 and 2 are left out or folded into
-// an FMA whose product they make exact.
+// are integer ones, and products with 0.5 and 2 are left out or done on the
+// exponent.
 //
 // Reference functions restated here (maikel/FiniteVolumeSolver):
 //   PerfectGas<D>::CompleteFromCons, Flux   src/equations/PerfectGas.cpp:25-124
@@ -97,9 +97,10 @@ __device__ __forceinline__ void AsCons(double* u, const Complete<D>& q) {
   u[1 + D] = q.E;
 }
 
-// (gamma - 1) (roeH - 0.5 roeU roeU), the half folded into an FMA
+// (gamma - 1) (roeH - 0.5 roeU roeU), rounded as written in every translation
+// unit, the half off the FP64 pipe
 __device__ __forceinline__ double RoeA2(const Gas& eq, double roeU, double roeH) {
-  return (eq.gamma - 1.0) * __fma_rn(-0.5, roeU * roeU, roeH);
+  return (eq.gamma - 1.0) * __dsub_rn(roeH, __dmul_rn(ieee64::HalfFactor(roeU), roeU));
 }
 
 template <int D>

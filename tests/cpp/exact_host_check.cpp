@@ -1,7 +1,8 @@
 // Host check of pieces of the exact FP64 physics (csrc/fvs_physics_exact.cuh,
 // its device functions compiled as plain C++ without contraction) against the
 // reference's expressions in IEEE arithmetic, bit for bit (any NaN equals any
-// other): the half slopes of every limiter, over zeros of both signs, ties,
+// other): the half slopes of every limiter and the Roe mean's squared sound
+// speed, over zeros of both signs, ties,
 // subnormals, infinities, NaN, neighbours and random numbers of every exponent.
 // Prints "bad 0" and exits 0 when all agree.
 #include <cmath>
@@ -15,7 +16,8 @@
 #define __host__
 #define __forceinline__ inline
 #define __noinline__
-static inline double __fma_rn(double a, double b, double c) { return std::fma(a, b, c); }
+static inline double __dmul_rn(double a, double b) { return a * b; }
+static inline double __dsub_rn(double a, double b) { return a - b; }
 
 #include "fvs_physics_exact.cuh"
 
@@ -48,6 +50,11 @@ int SlopesDiffer(double sL, double sR) {
   return bad;
 }
 
+int RoeDiffers(double u, double h) {
+  const exact::Gas eq{1.4, 1.0 / (1.4 - 1.0)};
+  return Differ(exact::RoeA2(eq, u, h), (eq.gamma - 1.0) * (h - 0.5 * u * u));
+}
+
 }  // namespace
 
 int main() {
@@ -58,14 +65,14 @@ int main() {
       -1.7976931348623157e308, 0x1p511, 0x1p512, -0x1p512, 0x1p-510, 0x1p-511, -0x1p-537, 1e154};
   long bad = 0;
   for (double a : special)
-    for (double b : special) bad += SlopesDiffer(a, b);
+    for (double b : special) bad += SlopesDiffer(a, b) + RoeDiffers(a, b);
   std::mt19937_64 rng(11);
   std::uniform_real_distribution<double> u(-2.0, 2.0);
   for (int i = 0; i < 2000000; ++i) {
     const int span = i % 3 == 0 ? 1 : i % 3 == 1 ? 250 : 500;
     auto draw = [&] { return std::ldexp(u(rng), int(rng() % (2 * span + 1)) - span); };
     const double a = draw(), b = i % 8 ? draw() : a;
-    bad += SlopesDiffer(a, b);
+    bad += SlopesDiffer(a, b) + RoeDiffers(a, b);
   }
   std::printf("bad %ld\n", bad);
   return bad ? 1 : 0;
