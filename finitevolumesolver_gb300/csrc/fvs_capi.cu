@@ -1026,8 +1026,11 @@ int fvs_solver_create(const fvs_grid_desc* grid, const fvs_method* m,
   if (e == cudaSuccess) e = cudaMallocHost(&s->ctrl_host, sizeof(fvs::Control));
   if (e == cudaSuccess) e = cudaMalloc(&s->scratch_words, 8 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc(&s->newton_words, 3 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(s->newton_words, 0, 3 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(s->ctrl, 0, sizeof(fvs::Control));
+  // on the solver's stream, which nothing orders behind the default stream:
+  // there they could run in the middle of the first steps
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(s->newton_words, 0, 3 * sizeof(unsigned long long), s->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s->ctrl, 0, sizeof(fvs::Control), s->stream);
   if (e != cudaSuccess) {
     delete s;
     return CudaFail(e, "fvs_solver_create");
