@@ -3,9 +3,9 @@
 // speeds:
 //   T = double in a -fmad=false translation unit: the exact flavour, bit for
 //     bit the CPU oracle's restatement of the reference;
-//   T = double with FMA contraction and the nearly rounded quotients and
-//     square roots of fvs_ieee64.cuh (math policy CcFast): the fast FP64
-//     flavour, within 1e-12 of the exact one;
+//   T = double with FMA contraction and the nearly rounded quotients,
+//     reciprocals and square roots of fvs_ieee64.cuh (math policy CcFast): the
+//     fast FP64 flavour, within 1e-12 of the exact one;
 //   T = float: the mixed flavour -- masked MUSCL-Hancock, HLL/Einfeldt,
 //     boundary (wall) states and CFL speeds in FP32; the state, the face
 //     fractions, the h-box flux combination and the cut-cell update in FP64.
@@ -35,9 +35,15 @@ namespace fvs {
 namespace cc {
 
 // Arithmetic of the physics below: IEEE quotients and square roots (CcIeee:
-// the exact flavour, on the integer pipes; and FP32 for the mixed one) or the fast FP64 flavour's
-// (CcFast: nearly rounded ones on the integer pipes, within 0.57 and 0.75
-// ulp; the square root of a non-positive number is 0).
+// the exact flavour, on the integer pipes; and FP32 for the mixed one) or the
+// fast FP64 flavour's (CcFast: nearly rounded ones on the integer pipes, within
+// 0.57 and 0.75 ulp, quotients of a shared divisor as products with its
+// reciprocal; the square root of a non-positive number is 0).  On small grids
+// the kernels are the latency of one thread's instructions: two steps of 256^2
+// and 1024^2 take 1.98 and 3.80 ms with shared reciprocals (16-cell segments),
+// 2.74 and 4.62 ms with a quotient each, and 1.94 and 5.45 ms with reciprocals
+// refined by FP64 FMAs from the approximate instruction, which were less close
+// (2 ulp).
 // The policy is a template argument of every kernel and launcher, so the
 // exact and the fast FP64 instantiations, compiled with different flags in
 // different translation units, never share a symbol.
@@ -49,10 +55,11 @@ struct CcIeee {
   static __device__ __forceinline__ float Sqrt(float a) { return sqrtf(a); }
 };
 struct CcFast {
-  static constexpr bool kFast = false;  // divides: a reciprocal's product costs the FP64 pipe more
+  static constexpr bool kFast = true;
   static __device__ __forceinline__ double Div(double a, double b) {
     return fast::Math<double>::Div(a, b);
   }
+  static __device__ __forceinline__ double Rcp(double a) { return fast::Math<double>::Rcp(a); }
   static __device__ __forceinline__ double Sqrt(double a) { return fast::Math<double>::Sqrt(a); }
 };
 

@@ -64,11 +64,13 @@ inline int AutoSegment(const SweepShape& s) {
   if (!s.cut_cells && s.variant == 0 && LanesPay(s) && LanesFit(s.cells, s.n)) return 1;
   // Enough threads for several waves of resident blocks on 152 SMs
   // (~60K threads per wave at 150 registers per thread); never shorter than
-  // 16 cells, mixed 8 (the 2-cell halo of a segment is recomputed), nor more
-  // segments than a launch takes.
+  // 16 cells, mixed 8 (the 2-cell halo of a segment is recomputed), FP64 cut
+  // cells 8, a tile (exact / fast, two steps of 256^2: 1.80 / 1.22 ms, at 16
+  // cells 2.98 / 1.98; 1024^2 5.29 / 3.79 against 5.41 / 3.80); nor more segments
+  // than a launch takes.
   const int64_t target = 262144;
   const int64_t ntrans = s.cells / s.n;
-  const int shortest = s.mixed && !s.cut_cells ? 8 : 16;
+  const int shortest = s.mixed != s.cut_cells ? 8 : 16;
   int seg = s.n;
   while (seg > shortest && ntrans * Segments(s.n, seg) < target &&
          Segments(s.n, (seg + 1) / 2) <= kMaxSegments)
