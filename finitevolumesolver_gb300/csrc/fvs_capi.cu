@@ -463,6 +463,7 @@ int SegLen(const fvs_solver* s, int dir) {
                                                  : fvs::SweepFamily::kHlle;
   q.cells = s->cells;
   q.n = s->g.n[dir];
+  q.exact = s->m.precision == FVS_FP64_EXACT;
   q.mixed = s->m.precision == FVS_MIXED;
   q.cut_cells = s->cc;
   q.variant = s->occ_tuned[dir];

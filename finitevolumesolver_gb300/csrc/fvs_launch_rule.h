@@ -15,6 +15,7 @@ struct SweepShape {
   SweepFamily family = SweepFamily::kHlle;
   int64_t cells = 0;
   int n = 0;           // cells along the sweep direction
+  bool exact = false;  // exact FP64
   bool mixed = false;
   bool cut_cells = false;
   int variant = 0;     // launch variant of the marching sweep, 0: not chosen
@@ -36,12 +37,14 @@ inline bool LanesFit(int64_t cells, int n) {
 // sizes, over that with one cell per lane; 1-D: of a sweep):
 //   HLLE, exact / fast / double-float: 1-D 2^10 cells 5 / 4 / 3, 2^22 cells
 //     59 / 55 / 77; 2-D 1024^2 1.32 / 1.24 / 1.20, 1448^2 1.18 / 1.10 / 1.06,
-//     1800^2 1.03 / 0.97 / 0.99, 2048^2 1.01 / 0.95 / 0.93; 3-D 64^3 1.7 / 1.6 /
-//     1.9, 128^3 1.08 / 1.07 / 1.09, 160^3 1.02 / 1.01 / 1.06
+//     1500^2 1.13 / 1.07 / 1.02, 1600^2 1.08 / 1.02 / 1.01, 1800^2 1.03 / 0.97 /
+//     0.99, 2048^2 1.01 / 0.95 / 0.93; 3-D 64^3 1.7 / 1.6 / 1.9, 128^3 1.08 /
+//     1.07 / 1.09, 160^3 1.02 / 1.01 / 1.06
 //   HLLEM and its reconstructions: 2-D 2048^2 1.06 to 1.10, 3-D 64^3 1.5 to 1.7,
 //     160^3 1.03 to 1.16
 //   Godunov / MUSCL-Godunov: 1-D 2^22 cells 96 / 90; 2-D 512^2 1.6 / 1.6, 1024^2
-//     1.12 / 1.04, 2048^2 1.08 / 1.02, but along the lines of 64 cells of 8192 x
+//     1.12 / 1.04, 2048^2 1.08 / 1.02 (from the mean start the first steps of
+//     1024^2 0.92, twenty 1.06), but along the lines of 64 cells of 8192 x
 //     64 (sweeps) 0.5 / 0.4, where a lane beside a line's end solves a Riemann
 //     problem of two unrelated cells and its warp waits; 3-D 64^3 1.19 / 1.13,
 //     80^3 1.06 / 1.02, 96^3 0.87 / 0.80
@@ -54,7 +57,7 @@ inline bool LanesPay(const SweepShape& s) {
     if (s.rank == 3) return s.cells <= (k1 << 19);
     if (s.rank == 2 && s.cells > (k1 << 18) && s.n < 256) return false;
   }
-  if (s.family == SweepFamily::kHlle && s.rank == 2) return s.cells <= (k1 << 21);
+  if (s.family == SweepFamily::kHlle && s.rank == 2 && !s.exact) return s.cells <= 5 * (k1 << 19);
   return s.cells <= (k1 << 22);
 }
 

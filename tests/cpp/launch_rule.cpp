@@ -20,6 +20,7 @@ int main() {
       if (key == "rank") q.rank = int(v);
       else if (key == "cells") q.cells = v;
       else if (key == "n") q.n = int(v);
+      else if (key == "exact") q.exact = v != 0;
       else if (key == "mixed") q.mixed = v != 0;
       else if (key == "cut_cells") q.cut_cells = v != 0;
       else if (key == "family") q.family = static_cast<fvs::SweepFamily>(v);

@@ -66,9 +66,10 @@ def test_a_chosen_variant_marches(auto, mixed, variants):
 
 
 # (family, n of the direction, other extents' product, rank): one cell per lane?
+# (HLLE: fast FP64 and double-float, then exact)
 HLLE, HLLEM, GODUNOV = range(3)
 MEASURED = [(HLLE, 160, 160 ** 2, 3, True), (HLLE, 192, 192 ** 2, 3, False),
-            (HLLE, 1448, 1448, 2, True), (HLLE, 2048, 2048, 2, False),
+            (HLLE, 1600, 1600, 2, True), (HLLE, 1800, 1800, 2, False),
             (HLLE, 1 << 22, 1, 1, True), (HLLEM, 2048, 2048, 2, True),
             (HLLEM, 160, 160 ** 2, 3, True), (GODUNOV, 80, 80 ** 2, 3, True),
             (GODUNOV, 96, 96 ** 2, 3, False), (GODUNOV, 128, 128 ** 2, 3, False),
@@ -83,6 +84,8 @@ def test_one_cell_per_lane_where_it_is_faster(auto):
     cases = [dict(family=f, n=n, cells=n * other, rank=rank) for f, n, other, rank, _ in MEASURED]
     for m, seg in zip(MEASURED, auto(cases)):
         assert (seg == 1) == m[4], m
+    exact = [dict(family=HLLE, n=n, cells=n ** 2, rank=2, exact=1) for n in (1800, 2048, 2100)]
+    assert [seg == 1 for seg in auto(exact)] == [True, True, False]
 
 
 @pytest.mark.gpu
