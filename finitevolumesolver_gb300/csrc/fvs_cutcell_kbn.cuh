@@ -3,8 +3,8 @@
 // speeds:
 //   T = double in a -fmad=false translation unit: the exact flavour, bit for
 //     bit the CPU oracle's restatement of the reference;
-//   T = double with FMA contraction and the nearly rounded quotients,
-//     reciprocals and square roots of fvs_ieee64.cuh (math policy CcFast): the
+//   T = double with FMA contraction, the nearly rounded quotients and square
+//     roots of fvs_ieee64.cuh and refined reciprocals (math policy CcFast): the
 //     fast FP64 flavour, within 1e-12 of the exact one;
 //   T = float: the mixed flavour -- masked MUSCL-Hancock, HLL/Einfeldt,
 //     boundary (wall) states and CFL speeds in FP32; the state, the face
@@ -37,13 +37,15 @@ namespace cc {
 // Arithmetic of the physics below: IEEE quotients and square roots (CcIeee:
 // the exact flavour, on the integer pipes; and FP32 for the mixed one) or the
 // fast FP64 flavour's (CcFast: nearly rounded ones on the integer pipes, within
-// 0.57 and 0.75 ulp, quotients of a shared divisor as products with its
-// reciprocal; the square root of a non-positive number is 0).  On small grids
-// the kernels are the latency of one thread's instructions: two steps of 256^2
-// and 1024^2 take 1.98 and 3.80 ms with shared reciprocals (16-cell segments),
-// 2.74 and 4.62 ms with a quotient each, and 1.94 and 5.45 ms with reciprocals
-// refined by FP64 FMAs from the approximate instruction, which were less close
-// (2 ulp).
+// 0.57 and 0.75 ulp, but quotients of a shared divisor as products with its
+// reciprocal; the square root of a non-positive number is 0).
+//
+// The reciprocal is y (1 + r + r^2), r = 1 - a y, of the approximate
+// instruction's y (|r| < 2^-20): 0.51 ulp.  On small grids the kernels are the
+// latency of one thread's instructions, on large ones the FP64 pipe's; two steps
+// of 256^2 / 1024^2 / 2048^2 in ms: 1.00 / 3.89 / 11.7; with the reciprocal on
+// the integer pipes 1.21 / 3.70 / 10.6; with a quotient on the integer pipes for
+// each 1.63 / 4.39 / 12.0; with the roots from FP64 FMAs too 1.06 / 5.04 / 15.8.
 // The policy is a template argument of every kernel and launcher, so the
 // exact and the fast FP64 instantiations, compiled with different flags in
 // different translation units, never share a symbol.
@@ -59,7 +61,12 @@ struct CcFast {
   static __device__ __forceinline__ double Div(double a, double b) {
     return fast::Math<double>::Div(a, b);
   }
-  static __device__ __forceinline__ double Rcp(double a) { return fast::Math<double>::Rcp(a); }
+  static __device__ __forceinline__ double Rcp(double a) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double r = fma(-a, y, 1.0);
+    return fma(y, fma(r, r, r), y);
+  }
   static __device__ __forceinline__ double Sqrt(double a) { return fast::Math<double>::Sqrt(a); }
 };
 

@@ -68,9 +68,9 @@ inline int AutoSegment(const SweepShape& s) {
   // Enough threads for several waves of resident blocks on 152 SMs
   // (~60K threads per wave at 150 registers per thread); never shorter than
   // 16 cells, mixed 8 (the 2-cell halo of a segment is recomputed), FP64 cut
-  // cells 8, a tile (exact / fast, two steps of 256^2: 1.80 / 1.22 ms, at 16
-  // cells 2.98 / 1.98; 1024^2 5.29 / 3.79 against 5.41 / 3.80); nor more segments
-  // than a launch takes.
+  // cells 8, a tile (exact / fast, two steps of 256^2: 1.80 / 1.00 ms, at 16
+  // cells 2.98 / 1.58; 900^2 4.74 / 3.48 against 5.13 / 3.51; 1024^2 5.26 / 3.89
+  // against 5.39 / 3.72); nor more segments than a launch takes.
   const int64_t target = 262144;
   const int64_t ntrans = s.cells / s.n;
   const int shortest = s.mixed != s.cut_cells ? 8 : 16;
