@@ -263,7 +263,8 @@ __device__ __forceinline__ void LaneFaceSpeed(const typename P::Gas& eq, const R
 // which faces 0 and n need), where PatchSweepKernel's segments repeat two per
 // segment and load four halo cells each, and a warp's loads of an x row are
 // consecutive.  The arithmetic per cell and face is PatchSweepKernel's: the
-// results are the same, bit for bit.
+// results are the same, bit for bit, in the exact and mixed flavours; in fast
+// FP64 the compiler may contract other products.
 //
 // FP64 flavours take it in both directions: a marching thread's row is a
 // serial chain of FP64 instructions (64 clocks each in the FP64 unit that one

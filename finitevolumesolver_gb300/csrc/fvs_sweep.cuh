@@ -1012,7 +1012,9 @@ struct HasLanes<P, std::enable_if_t<(P::kLaneBlocks > 0)>> : std::true_type {};
 // and the lanes 1..30 own their slots (CFL speed of the face, update of the
 // cell with the right neighbour's face).  Where a line ends or the warp does,
 // a lane loads the missing neighbour cell itself.  Every face and cell takes
-// the marching sweep's arithmetic, so the results are the same bits.
+// the marching sweep's arithmetic: the same bits in the translation units
+// without contraction (exact FP64); elsewhere the compiler may contract other
+// products in the two kernels, and they agree to the flavour's tolerance.
 //
 // It is the sweep of grids whose lines are too few to fill the chip by
 // marching: a marching thread's segment is a serial chain over its cells (16
