@@ -472,7 +472,6 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   __shared__ float vec[mlp::kParams - mlp::kOffB2];  // b2, w3, b3
   __shared__ float b1[kH], stats[2 * mlp::kIn];
   __shared__ float residual[kTile], target[kTile];
-  __shared__ int failed;  // a wait of an earlier step ran out
   // per row-warp sums over the tiles: db1, db2, dw3 and (db3, loss)
   __shared__ float sums[4][3 * kH + 2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -482,8 +481,8 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
     tc::MbarInit(&bar, 1);
     tma::FenceMbarInit();
   }
-  if (tid == 32 && a.count && blockIdx.x == 0) a.step[1] += 1;
-  if (tid == 64) failed = *a.error;
+  // (nothing here waits for memory ahead of the weights' loads)
+  if (tid == 32 && a.count && blockIdx.x == 0) atomicAdd(a.step + 1, 1ull);
   LoadWeights(sm + kOffSW1, a.W1, kXin);
   LoadWeights(sm + kOffSW2, a.W2, kH);
   LoadWeights(sm + kOffSW2t, a.W2t, kH);
@@ -502,7 +501,6 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
   float* act = reinterpret_cast<float*>(sm + kOffAct);
   const unsigned long long step = a.step[0];
   MmaPhases mma{&bar, a.error};
-  mma.ok = failed == 0;
   const int tiles = a.batch / kTile;
   bool first = true;
   for (int tile = blockIdx.x; tile < tiles && mma.ok; tile += gridDim.x) {
@@ -601,9 +599,6 @@ __global__ void __launch_bounds__(kFusedThreads) FusedStepKernel(FusedArgs a) {
 #pragma unroll
       for (int k = 0; k < mlp::kIn; ++k) out[mlp::kOffW1 + (row - kH) * mlp::kIn + k] = v[k];
     }
-  } else {  // (UpdateKernel does not use sums of a failed step)
-    for (int i = tid; i < kH * kH; i += blockDim.x) out[mlp::kOffW2 + i] = 0.0f;
-    for (int i = tid; i < kH * mlp::kIn; i += blockDim.x) out[mlp::kOffW1 + i] = 0.0f;
   }
   if (tid < 3 * kH + 2) {
     const float t = ((sums[0][tid] + sums[1][tid]) + sums[2][tid]) + sums[3][tid];
